@@ -354,8 +354,8 @@ def main():
         bytes_alg = ntgt * (nc * cb + g.Nb ** 3 * 16)
     t_k = per_step[k] * 1e-3
     # the CUDA-core roofline is taken on the floating-point work the kernels
-    # execute; for the MAC that is less than the pair list's 8 Nc flops per
-    # pair (block-Toeplitz products), which is reported beside it
+    # execute (for the MAC the direct kernel's products, some with absent
+    # blocks); the pair list's 8 Nc flops per pair is reported beside it
     exec_flops = float(stats[9]) / args.steps * nc if k == 1 else flops
     ai = flops / max(bytes_alg, 1)
     if ai > fma * 1e12 / (hbm * 1e9):
@@ -415,7 +415,7 @@ def main():
                 "e2e": {"value": (1 if sharded else world) * cells / (e2e_ms * 1e-3), "unit": "cells/s",
                         "h2d_bytes_per_step": nbytes, "d2h_bytes_per_step": nbytes},
                 "gpu_launches": int(launches),
-                "mac_autotune": {"variants": "0, 1: direct sibling-group kernel (64 x 768, 32 x 512 FP32); "
+                "mac_autotune": {"variants": "0, 1: direct sibling-group kernel (two groups, half a group per warp); "
                                              "2: block-Toeplitz kernel (TMA-staged coefficients); "
                                              "3: tensor-core kernel (tcgen05 TF32, 3-product split, "
                                              "M = 128 groups, N = 16, K = 8 per MMA)",

@@ -158,6 +158,16 @@ struct TpTasks  // tensor-product transfer tasks of one tree level
 // sibling groups per group-MAC tile; the kernel's thread rows x groups per
 // row cover exactly this many
 constexpr int kGroupTileCap = 32;
+// bundles of two sibling groups per tile of the direct MAC
+constexpr int kMacTile = 96;
+// bundles of a table up to which its tile is split over four warps per bundle
+// (the CTA has 20 warps in FP32, 12 in FP64): the tiles of the coarse levels'
+// tables, 1 to 4 bundles, then take 5 instead of 15 us of an SM. At 16 to 24
+// bundles the split costs a third (vortex ring, 1.36 against 1.09 ms).
+constexpr int kMacSplit = 5;
+// candidate x target rows (of 16) from which a half parent runs all of them:
+// 32 products without a branch cost about as much as 24 with
+constexpr int kMacDense = 12;
 // sibling groups per work item of the block-Toeplitz MAC (a tile has up to 3)
 constexpr int kToeplitzPart = 14;
 
@@ -188,6 +198,14 @@ struct FmmPlan
     DevBuf<int> tile_combo;      // per tile: coefficient table of the block-Toeplitz MAC (its level difference)
     DevBuf<int> tile_parts;      // block-Toeplitz work: tile << 2 | part for the non-empty parts of 14 groups
     int n_parts = 0;
+    // direct MAC: tiles (first bundle, end, LGF table, pair mode | 4 if split) of bundles of
+    // two groups; per bundle its groups (mac_grp, second -1: none) and its half
+    // parents [mac_ptr[b], mac_ptr[b + 1]): LGF row of the first offset and the
+    // candidate x target row bits of both groups (mac_head, 2 each), source
+    // rows of both groups (mac_rows, 8 each)
+    int n_mac_tiles = 0;
+    DevBuf<int> mac_tile, mac_ptr, mac_grp, mac_rows;
+    DevBuf<unsigned> mac_head;
     // tensor-core MAC: tiles of up to 128 consecutive groups of one LGF table
     // and pair mode (tc_gptr, tc_tab, tc_mode, tc_pm = union of the groups'
     // parent masks), and per group its 216 candidate source rows (grp_jr)

@@ -320,153 +320,224 @@ __global__ void __launch_bounds__(128) mac_kernel(const cx<R>* __restrict__ G, c
 // neighbours; coarser targets see the non-adjacent ones. The 8 siblings of a
 // parent therefore share one candidate source set (216 = 27 x 8 candidates
 // k = (n, c')), and the offset of (child c, candidate (n, c')) is
-// u = c - c' - 2n in [-3,3]^3 (343 LGF spectra per tile).
-// For one neighbour parent n the 64 (c, c') pairs use only the 27 offsets
-// u = d - 2n, d = c - c' in [-1,1]^3; the kernel walks n and, per dz = cz - c'z,
-// keeps the 9 spectra of that z-offset (shared by the slabs (c'z, cz) = (0, 0)
-// and (1, 1) at dz = 0) in registers for 16 or 32 complex MACs.
-// Adjacency filtering (coarse targets take only non-adjacent sources, the
-// integrating factor only adjacent ones) depends on u alone, so it is applied
-// once when the tile's spectra are staged: excluded offsets become zero rows.
-// Tiles that take all or the non-adjacent pairs then run every pair (an
-// excluded pair adds exactly zero); tiles of adjacent pairs only (the
-// integrating factor, 27 of 216) skip the others.
-// One CTA = (tile of up to 32 sibling groups, chunk of F frequencies); each warp
-// takes one group at 32 consecutive frequencies, so a source load is one
-// contiguous 256-byte (FP32) or 512-byte (FP64) row segment. The tile's
-// spectra and the groups' candidate rows (precomputed with the plan, tile_jr)
-// are copied asynchronously into shared memory; source spectra are read
-// through L1/L2. Candidates that do not exist read a zero spectrum row (zrow),
-// and parents without any candidate are skipped via the group's 27-bit mask
-// (grp_pm).
-template<class R, int F, bool ADJ_ONLY>
-__device__ __forceinline__ void group_mac_parent(const cx<R>* gn, const cx<R> (&sv)[8], cx<R> (&acc)[8], int nx,
-                                                 int ny, int nz)
+// u = c - c' - 2n in [-3,3]^3. For one neighbour parent n the 64 (c, c') pairs
+// use only the 27 offsets u = d - 2n, d = c - c' in [-1,1]^3.
+//
+// One warp = NG = 2 sibling groups of one LGF table (a bundle) at 32
+// consecutive frequencies. It walks the bundle's half parents (n, c'z): the 18
+// LGF values of one go from shared memory into registers once and serve both
+// groups, whose 16 accumulators stay in registers for the whole walk; the
+// source values are read straight from their rows (256-byte row segments in
+// FP32), one group ahead of their use. The CTA stages the table's 343 rows at
+// its 32 frequencies in shared memory and its warps take the tile's bundles
+// from a counter.
+// A half parent with all 4 candidates, seen from a group with all 4 target
+// rows (pairs along x), runs its 32 products without a branch; elsewhere
+// absent candidates, target rows without a target and rows beyond the adjacent
+// ones (neighbour-only plans) are skipped. Offsets that a plan excludes
+// altogether (adjacent ones of coarse targets, the others of neighbour-only
+// plans) are zero rows of the staged table.
+template<class R, int CY, int CZ, int Q>
+__device__ __forceinline__ void mac_row(const cx<R> (&gv)[9], const cx<R>& s, cx<R>* acc)
 {
-#pragma unroll
-    for (int dz = -1; dz <= 1; ++dz)
+    // targets c = (0, CY, CZ) and (1, CY, CZ) of source child Q + 4 c'z;
+    // gv[(dx + 1) + 3 (dy + 1)] with d = c - c', of the plane dz = CZ - c'z
+    constexpr int d0 = (0 - (Q & 1) + 1) + 3 * (CY - (Q >> 1) + 1);
+    cmac<R>(acc[2 * CY + 4 * CZ], gv[d0], s);
+    cmac<R>(acc[2 * CY + 4 * CZ + 1], gv[d0 + 1], s);
+}
+
+template<class R, int CZ, int Q>
+__device__ __forceinline__ void mac_source(const cx<R> (&gv)[9], const cx<R>& s, cx<R>* acc)
+{
+    mac_row<R, 0, CZ, Q>(gv, s, acc);
+    mac_row<R, 1, CZ, Q>(gv, s, acc);
+}
+
+// the products of one half parent with the target rows cz = CZ of one group;
+// mask: bit 4 q + cy + 2 cz of each candidate and target row to take (all 16
+// set also where the few absent candidates read the zero row)
+template<class R, int CZ>
+__device__ __forceinline__ void mac_half(const cx<R> (&gv)[9], const cx<R> (&s)[4], cx<R>* acc, unsigned mask)
+{
+    if (mask == 0xFFFFu)
     {
-        if (ADJ_ONLY && abs(dz - 2 * nz) > 1) continue;
-        cx<R> gv[9];
-#pragma unroll
-        for (int dy = -1; dy <= 1; ++dy)
-#pragma unroll
-            for (int dx = -1; dx <= 1; ++dx)
-                gv[(dy + 1) * 3 + dx + 1] = gn[(dx + 7 * dy + 49 * dz) * F];
-#pragma unroll
-        for (int cpz = 0; cpz < 2; ++cpz)
-        {
-            const int cz = cpz + dz;
-            if (cz < 0 || cz > 1) continue;
-#pragma unroll
-            for (int q = 0; q < 4; ++q)  // c' = 4 cpz + q
-#pragma unroll
-                for (int r = 0; r < 4; ++r)  // c = 4 cz + r
-                {
-                    const int dx = (r & 1) - (q & 1), dy = (r >> 1) - (q >> 1);
-                    if (ADJ_ONLY && (abs(dx - 2 * nx) > 1 || abs(dy - 2 * ny) > 1)) continue;
-                    cmac<R>(acc[4 * cz + r], gv[(dy + 1) * 3 + dx + 1], sv[4 * cpz + q]);
-                }
-        }
+        mac_source<R, CZ, 0>(gv, s[0], acc);
+        mac_source<R, CZ, 1>(gv, s[1], acc);
+        mac_source<R, CZ, 2>(gv, s[2], acc);
+        mac_source<R, CZ, 3>(gv, s[3], acc);
+    }
+    else if (mask & (0x3333u << (2 * CZ)))
+    {
+        constexpr unsigned b = 1u << (2 * CZ);
+        if (mask & b) mac_row<R, 0, CZ, 0>(gv, s[0], acc);
+        if (mask & (b << 1)) mac_row<R, 1, CZ, 0>(gv, s[0], acc);
+        if (mask & (b << 4)) mac_row<R, 0, CZ, 1>(gv, s[1], acc);
+        if (mask & (b << 5)) mac_row<R, 1, CZ, 1>(gv, s[1], acc);
+        if (mask & (b << 8)) mac_row<R, 0, CZ, 2>(gv, s[2], acc);
+        if (mask & (b << 9)) mac_row<R, 1, CZ, 2>(gv, s[2], acc);
+        if (mask & (b << 12)) mac_row<R, 0, CZ, 3>(gv, s[3], acc);
+        if (mask & (b << 13)) mac_row<R, 1, CZ, 3>(gv, s[3], acc);
     }
 }
 
-template<class R, int F, int NT, int MINB, int NB>
-__global__ void __launch_bounds__(NT, MINB) group_mac_kernel(
-    const cx<R>* __restrict__ G, const cx<R>* __restrict__ S, int zrow,
-    const int* __restrict__ tile_gptr, const int* __restrict__ tile_jr,
-    const int* __restrict__ tile_tab, const int* __restrict__ tile_coarse, const int* __restrict__ spec_u,
-    const unsigned* __restrict__ grp_pm,
-    const int* __restrict__ grp_tgt, cx<R>* __restrict__ ACC)
+template<class R, int NB>
+__device__ __forceinline__ void mac_load(cx<R> (&s)[4], const cx<R>* Sf, const uint4& r)
 {
-    constexpr int RW = NT / F;      // thread rows, one group each per pass
-    constexpr int P = 2 * NB - 1;
-    constexpr long long NC = (long long)(P / 2 + 1) * P * P;  // spectrum row length
-    constexpr int per = 16 / sizeof(cx<R>);
-    constexpr int parts = F / per;  // 16-byte pieces of a staged row
-    static_assert(F % 32 == 0 && NT % F == 0, "a warp covers one row");
+    constexpr unsigned NC = (unsigned)NB * (2 * NB - 1) * (2 * NB - 1);
+    s[0] = __ldg(Sf + (unsigned long long)r.x * NC);
+    s[1] = __ldg(Sf + (unsigned long long)r.y * NC);
+    s[2] = __ldg(Sf + (unsigned long long)r.z * NC);
+    s[3] = __ldg(Sf + (unsigned long long)r.w * NC);
+}
+
+// Bound by instruction issue (FP32: 72% of the issue slots, three quarters of
+// them FFMAs; FP64: the DFMA pipe and the LGF rows' shared-memory reads), with
+// DRAM at a tenth. Against one group per warp, 64 frequencies per CTA and tiles
+// of 32 groups, each of one problem of a batch: the MAC of a batch of 256
+// problems 6.06 -> 1.88 ms (one staged table for 192 groups of any problem
+// instead of one for the few groups of each), amr_3level FP32 7.53 -> 7.08 ms,
+// vortex ring FP32 1.12 -> 1.04 ms, amr_2level FP64 3.45 -> 3.41 ms. Not kept: all 27 LGF values of a
+// parent in registers without shared memory (10.0 ms on amr_3level: its loads
+// are not hidden at 16 warps), LGF rows read through L1 by small warps (25 ms).
+// In a split tile (bit 2 of its mode) a warp takes one group of a bundle and one
+// half (cz) of its targets: tiles whose bundles are no more than a quarter of
+// the CTA's warps. ALL: every tile is split, and the kernel keeps the registers
+// of that path only (FP32: two CTAs per SM), for plans with few groups (8
+// groups of a uniform 64^3 solve: 52 against 73 us).
+template<class R, int NB, int NT, int MINB, bool ALL>
+__global__ void __launch_bounds__(NT, MINB) bundle_mac_kernel(
+    const cx<R>* __restrict__ G, const cx<R>* __restrict__ S, const int4* __restrict__ tiles,
+    const int* __restrict__ spec_u, const int* __restrict__ bundle_ptr, const int2* __restrict__ bundle_grp,
+    const uint2* __restrict__ head, const uint4* __restrict__ rows, const int* __restrict__ tgt,
+    cx<R>* __restrict__ ACC)
+{
+    constexpr int P = 2 * NB - 1, F = 32;
+    constexpr long long NC = (long long)NB * P * P;
+    constexpr int per = 16 / sizeof(cx<R>), parts = F / per;  // 16-byte pieces of a staged row
     extern __shared__ __align__(16) unsigned char smraw[];
-    cx<R>* Gs = reinterpret_cast<cx<R>*>(smraw);                      // [343][F]
-    int* Jr = reinterpret_cast<int*>(Gs + 343 * F);                  // [tile groups][216] source rows
-    const int tile = blockIdx.x;
+    cx<R>* Gs = reinterpret_cast<cx<R>*>(smraw);  // [343][F]
+    int* Sl = reinterpret_cast<int*>(Gs + 343 * F);
+    int* next = Sl + 343;
+    const int4 tile = tiles[blockIdx.x];  // first bundle, end, table, mode: 0 all, 1 non-adjacent, 2 adjacent
+    const int mode = tile.w & 3;
+    const bool split = ALL || (tile.w & 4);
     const long long f0 = (long long)blockIdx.y * F;
-    const int lane = threadIdx.x % F, row = threadIdx.x / F;
-    const int mode = tile_coarse[tile];  // 0 all, 1 non-adjacent only, 2 adjacent only
-    const int* su = spec_u + 343 * tile_tab[tile];
-    const int g0 = tile_gptr[tile], g1 = tile_gptr[tile + 1];
     const cx<R> zero = mk<R>(0, 0);
-    const bool full = f0 + F <= NC;
-    {
-        // the tile's candidate rows, one 16-byte copy per 4 entries
-        const int* jsrc = tile_jr + (size_t)tile * kGroupTileCap * 216;
-        for (int i = threadIdx.x; i < kGroupTileCap * 216 / 4; i += blockDim.x)
-            __pipeline_memcpy_async(Jr + 4 * i, jsrc + 4 * i, 16);
-    }
-    // spectrum slot of each offset row (-1: excluded by the tile's mode),
-    // evaluated once per row
-    int* Sl = Jr + kGroupTileCap * 216;
-    for (int r = threadIdx.x; r < 343; r += blockDim.x)
+    for (int r = threadIdx.x; r < 343; r += NT)
     {
         const int ux = r % 7 - 3, uy = (r / 7) % 7 - 3, uz = r / 49 - 3;
         const bool adj = ux >= -1 && ux <= 1 && uy >= -1 && uy <= 1 && uz >= -1 && uz <= 1;
-        Sl[r] = (mode == 1 && adj) || (mode == 2 && !adj) ? -1 : su[r];
+        Sl[r] = (mode == 1 && adj) || (mode == 2 && !adj) ? -1 : spec_u[343 * tile.z + r];
     }
+    if (threadIdx.x == 0) *next = split ? 4 * tile.x : tile.x;
     __syncthreads();
-    for (int q = threadIdx.x; q < 343 * parts; q += blockDim.x)
+    const bool full = f0 + F <= NC;
+    for (int q = threadIdx.x; q < 343 * parts; q += NT)
     {
-        const int r = q / parts, part = q % parts;
-        const int slot = Sl[r];
+        const int r = q / parts, part = q % parts, slot = Sl[r];
         cx<R>* dst = Gs + r * F + part * per;
-        const cx<R>* src = slot >= 0 ? G + (size_t)slot * NC + f0 + part * per : nullptr;
-        if (src && full) __pipeline_memcpy_async(dst, src, 16);
+        const cx<R>* src = G + (size_t)max(slot, 0) * NC + f0 + part * per;
+        if (slot >= 0 && full) __pipeline_memcpy_async(dst, src, 16);
         else
-            for (int e = 0; e < per; ++e)
-                dst[e] = (src && f0 + part * per + e < NC) ? src[e] : zero;
+            for (int e = 0; e < per; ++e) dst[e] = (slot >= 0 && f0 + part * per + e < NC) ? src[e] : zero;
     }
     __pipeline_commit();
     __pipeline_wait_prior(0);
     __syncthreads();
+    const int lane = threadIdx.x & 31;
     const long long f = f0 + lane;
-    const long long fc = f < NC ? f : NC - 1;  // clamped column for the tail chunk
-    const cx<R>* Sf = S + fc;
-    for (int g = g0 + row; g < g1; g += RW)
+    const cx<R>* Sf = S + (f < NC ? f : NC - 1);  // clamped column for the tail
+    for (;;)
     {
-        const int* jr = Jr + (g - g0) * 216;
-        const unsigned pm = grp_pm[g];
-        cx<R> acc[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) acc[c] = zero;
-        // neighbour parents n = (nx, ny, nz): the x-offset unrolled, so that the
-        // LGF row of u = -2n (d = (dx, dy, dz) adds dx + 7 dy + 49 dz) sits at
-        // a compile-time offset from the (ny, nz) base
-        for (int nzy = 0; nzy < 9; ++nzy)
+        int item = 0;
+        if (lane == 0) item = atomicAdd(next, 1);
+        item = __shfl_sync(0xffffffffu, item, 0);
+        const int b = split ? item >> 2 : item;
+        if (b >= tile.y) return;
+        const int2 bg = bundle_grp[b];
+        const int e0 = bundle_ptr[b], e1 = bundle_ptr[b + 1];
+        const uint2* hp = head + e0;
+        if (split)
         {
-            const int ny = nzy % 3 - 1, nz = nzy / 3 - 1;
-            const cx<R>* gzy = Gs + (7 * (3 - 2 * ny) + 49 * (3 - 2 * nz)) * F + lane;
+            const int i = (item >> 1) & 1, cz = item & 1, g = i ? bg.y : bg.x;
+            if (g < 0) continue;
+            cx<R> acc[4];
 #pragma unroll
-            for (int nxi = 0; nxi < 3; ++nxi)
+            for (int c = 0; c < 4; ++c) acc[c] = zero;
+            // source values one half parent ahead, their rows two (the lists end
+            // with spare entries)
+            const uint4* rp = rows + 2 * (size_t)e0 + i;
+            cx<R> s[4], sn[4];
+            mac_load<R, NB>(s, Sf, rp[0]);
+            uint4 rn = rp[2];
+            uint2 h = *hp;
+            for (int e = e0; e < e1; ++e)
             {
-                const int n = 3 * nzy + nxi, nx = nxi - 1;
-                if (!((pm >> n) & 1u)) continue;
-                const int4 ja = *reinterpret_cast<const int4*>(jr + 8 * n);
-                const int4 jb = *reinterpret_cast<const int4*>(jr + 8 * n + 4);
-                const int jj[8] = {ja.x, ja.y, ja.z, ja.w, jb.x, jb.y, jb.z, jb.w};
-                cx<R> sv[8];
+                mac_load<R, NB>(sn, Sf, rn);
+                rn = rp[4];
+                rp += 2;
+                const uint2 hn = *++hp;
+                // the target row bits of this cz, as those of cz = 0
+                unsigned m = i ? h.y >> 16 : h.y & 0xFFFFu;
+                if (m != 0xFFFFu) m = (m >> (2 * cz)) & 0x3333u;
+                if (m)
+                {
+                    cx<R> gv[9];
+                    const cx<R>* g9 = Gs + (h.x + 49u * cz) * F + lane;
 #pragma unroll
-                for (int q = 0; q < 8; ++q) sv[q] = __ldg(Sf + (size_t)jj[q] * NC);
-                const cx<R>* gn = gzy + (3 - 2 * nx) * F;
-                if (mode == 2) group_mac_parent<R, F, true>(gn, sv, acc, nx, ny, nz);
-                else group_mac_parent<R, F, false>(gn, sv, acc, nx, ny, nz);
+                    for (int d = 0; d < 9; ++d) gv[d] = g9[((d % 3) + 7 * (d / 3)) * F];
+                    mac_half<R, 0>(gv, s, acc, m == 0x3333u ? 0xFFFFu : m);
+                }
+#pragma unroll
+                for (int q = 0; q < 4; ++q) s[q] = sn[q];
+                h = hn;
             }
+            if (f < NC)
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                {
+                    const int t = tgt[8 * (size_t)g + 4 * cz + c];
+                    if (t >= 0) ACC[(size_t)t * NC + f] = acc[c];
+                }
         }
-        if (f < NC)
+        else if constexpr (!ALL)
         {
+            cx<R> acc0[8], acc1[8];
 #pragma unroll
-            for (int c = 0; c < 8; ++c)
+            for (int c = 0; c < 8; ++c) acc0[c] = acc1[c] = zero;
+            // the lists end with spare entries, so the reads ahead stay inside
+            const uint4* rp = rows + 2 * (size_t)e0;
+            uint4 ra = rp[0], rb = rp[1];
+            uint2 h = *hp;
+            for (int e = e0; e < e1; ++e)
             {
-                const int t = grp_tgt[(size_t)g * 8 + c];
-                if (t >= 0) ACC[(size_t)t * NC + f] = acc[c];
+                cx<R> s0[4], s1[4], gv[9];
+                mac_load<R, NB>(s0, Sf, ra);
+                mac_load<R, NB>(s1, Sf, rb);
+                const cx<R>* g = Gs + h.x * F + lane;
+                const unsigned m0 = h.y & 0xFFFFu, m1 = h.y >> 16;
+                rp += 2;
+                ra = rp[0];
+                rb = rp[1];
+                h = *++hp;
+#pragma unroll
+                for (int d = 0; d < 9; ++d) gv[d] = g[((d % 3) + 7 * (d / 3)) * F];
+                mac_half<R, 0>(gv, s0, acc0, m0);
+                mac_half<R, 0>(gv, s1, acc1, m1);
+#pragma unroll
+                for (int d = 0; d < 9; ++d) gv[d] = g[((d % 3) + 7 * (d / 3) + 49) * F];
+                mac_half<R, 1>(gv, s0, acc0, m0);
+                mac_half<R, 1>(gv, s1, acc1, m1);
             }
+            if (f < NC)
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                {
+                    const int t0 = tgt[8 * (size_t)bg.x + c], t1 = bg.y >= 0 ? tgt[8 * (size_t)bg.y + c] : -1;
+                    if (t0 >= 0) ACC[(size_t)t0 * NC + f] = acc0[c];
+                    if (t1 >= 0) ACC[(size_t)t1 * NC + f] = acc1[c];
+                }
         }
     }
 }
@@ -618,38 +689,35 @@ struct Conv
 
     static constexpr bool kF32 = std::is_same<R, float>::value;
 
-    // S holds p.n_src source spectra followed by one zero row. Two tile
-    // shapes per precision (frequencies per CTA GF, threads GNT), chosen per
-    // plan by the MAC autotuner: variant 0 = (64, 768) FP32 / (32, 512)
-    // FP64, variant 1 = (32, 512) / (32, 256)
-    template<int GF, int GNT>
+    template<int NT, int MINB, bool ALL>
     static void group_mac_shape(Ctx& c, const FmmPlan& p, const void* S, void* acc)
     {
-        const size_t smem = (size_t)343 * GF * sizeof(cx<R>) + (size_t)(kGroupTileCap * 216 + 344) * sizeof(int);
-        auto kfn = group_mac_kernel<R, GF, GNT, 1, NB>;
+        const size_t smem = (size_t)343 * 32 * sizeof(cx<R>) + 344 * sizeof(int);
+        auto kfn = bundle_mac_kernel<R, NB, NT, MINB, ALL>;
         IBLGF_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        dim3 grid(p.n_tiles, (unsigned)((c.NC + GF - 1) / GF));
-        kfn<<<grid, GNT, smem, c.stream>>>((const cx<R>*)c.d_spec.p, (const cx<R>*)S, p.n_src,
-                                            p.tile_gptr.p, p.tile_jr.p, p.tile_tab.p,
-                                            p.tile_coarse.p, p.spec_u.p, p.grp_pm.p, p.grp_tgt.p,
-                                            (cx<R>*)acc);
+        kfn<<<dim3(p.n_mac_tiles, (unsigned)((c.NC + 31) / 32)), NT, smem, c.stream>>>(
+            (const cx<R>*)c.d_spec.p, (const cx<R>*)S, (const int4*)p.mac_tile.p, p.spec_u.p, p.mac_ptr.p,
+            (const int2*)p.mac_grp.p, (const uint2*)p.mac_head.p, (const uint4*)p.mac_rows.p, p.grp_tgt.p,
+            (cx<R>*)acc);
         c.launches += 1;
     }
 
+    // the direct sibling-group MAC: variant 0 = two groups per warp, 1 = half a
+    // group per warp
     static void group_mac(Ctx& c, const FmmPlan& p, const void* S, void* acc, int variant)
     {
-        if (!p.n_tiles) return;
+        if (!p.n_mac_tiles) return;
         if (c.NC != (long long)NB * (2 * NB - 1) * (2 * NB - 1))
             throw Error(IBLGF_EINTERNAL, "spectrum row length differs from the kernel's");
         if (variant == 1)
         {
-            if constexpr (kF32) group_mac_shape<32, 512>(c, p, S, acc);
-            else group_mac_shape<32, 256>(c, p, S, acc);
+            if constexpr (kF32) group_mac_shape<512, 2, true>(c, p, S, acc);
+            else group_mac_shape<512, 1, true>(c, p, S, acc);
         }
         else
         {
-            if constexpr (kF32) group_mac_shape<64, 768>(c, p, S, acc);
-            else group_mac_shape<32, 512>(c, p, S, acc);
+            if constexpr (kF32) group_mac_shape<640, 1, false>(c, p, S, acc);
+            else group_mac_shape<384, 1, false>(c, p, S, acc);
         }
     }
 
@@ -757,8 +825,8 @@ void launch_forward_sources(Ctx& c, const double* fmm_s, const int* d_src_oct, i
 }
 
 // one run of the sibling-group MAC in the given variant: 0, 1 the direct
-// kernel in its two tile shapes, 2 the block-Toeplitz kernel, 3 the
-// tensor-core kernel
+// kernel with two groups or one group per warp, 2 the block-Toeplitz kernel,
+// 3 the tensor-core kernel
 void group_mac_variant(Ctx& c, const FmmPlan& p, const void* src_spec, void* acc, int variant)
 {
     if (variant == 2 && toeplitz_mac(c, p, src_spec, acc)) return;

@@ -915,6 +915,87 @@ HostPlan build_host_plan(const Ctx& c, int level, int idx, int ge, bool direct_o
     return p;
 }
 
+namespace
+{
+// Tiles and bundles of the direct MAC: the groups by (LGF table, pair mode) in
+// plan order (parent keys ascending), two to a bundle; equal tables of a
+// batch's problems share their tiles. A tile holds up to kMacTile bundles (the
+// staged table serves them all).
+void build_mac_bundles(Ctx& c, FmmPlan& p, const HostPlan& h, const std::vector<int>& gjr)
+{
+    if (!p.n_tiles) return;
+    std::map<std::array<int, 4>, int> first_of;                // table by the key of its first offset
+    std::map<std::pair<int, int>, std::vector<int>> by_table;  // (table, mode) -> groups
+    for (int t = 0; t < p.n_tiles; ++t)
+    {
+        const int tab = first_of.emplace(h.tab_keys[343 * (size_t)h.ttab[t]], h.ttab[t]).first->second;
+        for (int g = h.tgptr[t]; g < h.tgptr[t + 1]; ++g) by_table[{tab, h.tcoarse[t]}].push_back(g);
+    }
+    std::vector<int> tile, ptr{0}, grp, rows;
+    std::vector<unsigned> head;
+    for (auto& kv : by_table)
+    {
+        const int mode = kv.first.second;
+        std::vector<int>& gs = kv.second;
+        std::stable_sort(gs.begin(), gs.end(), [&](int a, int b) {
+            return __builtin_popcount(h.gpm[a]) > __builtin_popcount(h.gpm[b]);
+        });
+        const int nb = ((int)gs.size() + 1) / 2, nt = (nb + kMacTile - 1) / kMacTile, b0 = (int)ptr.size() - 1;
+        for (int i = 0; i < nt; ++i)
+            tile.insert(tile.end(), {b0 + (int)((long long)nb * i / nt), b0 + (int)((long long)nb * (i + 1) / nt),
+                                     kv.first.first, mode | (nb <= kMacSplit ? 4 : 0)});
+        for (int b = 0; b < nb; ++b)
+        {
+            const int g[2] = {gs[2 * b], 2 * b + 1 < (int)gs.size() ? gs[2 * b + 1] : -1};
+            int row_bits[2] = {0, 0};
+            for (int i = 0; i < 2 && g[i] >= 0; ++i)
+                for (int r = 0; r < 4; ++r)
+                    if (h.gtgt[8 * (size_t)g[i] + 2 * r] >= 0 || h.gtgt[8 * (size_t)g[i] + 2 * r + 1] >= 0)
+                        row_bits[i] |= 1 << r;
+            grp.insert(grp.end(), {g[0], g[1]});
+            for (int n = 0; n < 27; ++n)
+                for (int cz = 0; cz < 2; ++cz)
+                {
+                    const int nx = n % 3 - 1, ny = (n / 3) % 3 - 1, nz = n / 9 - 1;
+                    int src[8];
+                    unsigned mask[2] = {0, 0};
+                    for (int i = 0; i < 2; ++i)
+                        for (int q = 0; q < 4; ++q)
+                        {
+                            src[4 * i + q] = g[i] >= 0 ? gjr[(size_t)g[i] * 216 + 8 * n + 4 * cz + q] : p.n_src;
+                            if (src[4 * i + q] == p.n_src) continue;
+                            for (int r = 0; r < 4; ++r)
+                                if (row_bits[i] >> r & 1 &&
+                                    (mode != 2 || (std::abs((r & 1) - (q >> 1) - 2 * ny) <= 1 &&
+                                                   std::abs((r >> 1) - cz - 2 * nz) <= 1)))
+                                    mask[i] |= 1u << (4 * q + r);
+                        }
+                    if (!(mask[0] | mask[1])) continue;
+                    for (unsigned& m : mask)
+                    {
+                        if (mode != 2 && __builtin_popcount(m) >= kMacDense) m = 0xFFFFu;
+                        p.mac_flops += 8 * 2 * __builtin_popcount(m);
+                    }
+                    // offset d = (-1, -1, -c'z) of this half: u = d - 2n
+                    head.insert(head.end(), {(unsigned)((2 - 2 * nx) + 7 * (2 - 2 * ny) + 49 * (3 - cz - 2 * nz)),
+                                             mask[0] | mask[1] << 16});
+                    rows.insert(rows.end(), src, src + 8);
+                }
+            ptr.push_back((int)head.size() / 2);
+        }
+    }
+    rows.insert(rows.end(), 24, p.n_src);  // the kernel reads up to two half parents ahead
+    head.insert(head.end(), 2, 0u);
+    p.n_mac_tiles = (int)tile.size() / 4;
+    p.mac_tile.upload(tile, c.stream);
+    p.mac_ptr.upload(ptr, c.stream);
+    p.mac_grp.upload(grp, c.stream);
+    p.mac_head.upload(head, c.stream);
+    p.mac_rows.upload(rows, c.stream);
+    IBLGF_CUDA(cudaStreamSynchronize(c.stream));  // the host arrays go out of scope
+}
+}  // namespace
+
 std::unique_ptr<FmmPlan> upload_plan(Ctx& c, const HostPlan& h)
 {
     auto plan = std::make_unique<FmmPlan>();
@@ -998,6 +1079,8 @@ std::unique_ptr<FmmPlan> upload_plan(Ctx& c, const HostPlan& h)
                 std::copy_n(jr.begin() + ((size_t)t * kGroupTileCap + (g - h.tgptr[t])) * 216, 216,
                             gjr.begin() + (size_t)g * 216);
         if (p.n_tiles) p.grp_jr.upload(gjr, c.stream);
+        p.mac_flops = (long long)h.psrc.size() * 8;  // per frequency: 8 per complex multiply-add
+        build_mac_bundles(c, p, h, gjr);
         std::vector<int> tg, tt, tm;
         std::vector<unsigned> tp;
         build_tc_tiles(h.tgptr, h.ttab, h.tcoarse, h.gpm, tg, tt, tm, tp);
@@ -1018,15 +1101,6 @@ std::unique_ptr<FmmPlan> upload_plan(Ctx& c, const HostPlan& h)
     p.n_exec = h.n_exec;
     p.adj_only = !h.tcoarse.empty();
     for (int m : h.tcoarse) p.adj_only = p.adj_only && m == 2;
-    // MAC work per frequency: 8 flops per complex multiply-add of the direct
-    // kernels; the block-Toeplitz kernel per (group, present parent) 27
-    // complex multiply-adds and 19 complex additions, and per group the 38
-    // additions of the final combination
-    p.mac_flops = (long long)h.psrc.size() * 8;
-    if (p.adj_only || !toeplitz)
-        p.mac_flops += (h.n_exec - (long long)h.psrc.size()) * 8;
-    else
-        for (unsigned pm : h.gpm) p.mac_flops += (long long)__builtin_popcount(pm) * (27 * 8 + 19 * 2) + 38 * 2;
     p.n_tgt = (int)h.tgt_list.size();
     p.n_pairs = h.n_pairs;
     p.n_spec_unique = h.n_spec_unique;

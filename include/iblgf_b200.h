@@ -387,16 +387,16 @@ int iblgf_stats(iblgf_ctx* ctx, long long* out8);
  * (target, source) spectral products the sibling-group MAC covers: a group
  * covers all 64 (child, candidate) products of every neighbour parent that
  * has a candidate, so [8] >= [3]; and [9] the floating-point operations the
- * MAC kernels execute per spectrum frequency (the block-Toeplitz group
- * kernel forms the 64 products of a parent with 27 complex multiplies).
+ * direct MAC kernels execute per spectrum frequency (they skip absent
+ * candidates and targets where that pays).
  * IBLGF_EINVAL for n outside [1, 10]. */
 int iblgf_stats_n(iblgf_ctx* ctx, long long* out, int n);
 
 /* Sibling-group MAC autotuning (no reference counterpart). On the first
  * sweep of each plan the library times every applicable variant of the
- * group MAC on that sweep's data (0: direct kernel, 64 frequencies x 768
- * threads in FP32 / 32 x 512 in FP64; 1: direct kernel, 32 x 512 / 32 x 256;
- * 2: block-Toeplitz kernel with TMA-staged coefficients, FP32 only; 3:
+ * group MAC on that sweep's data (0: direct kernel, two sibling groups per
+ * warp; 1: direct kernel, half a group per warp, for plans with few groups; 2:
+ * block-Toeplitz kernel with TMA-staged coefficients, FP32 only; 3:
  * tensor-core kernel, tcgen05 TF32 MMAs with a 3-product split and FP32
  * accumulation in tensor memory, FP32 only) and keeps the fastest.
  * iblgf_mac_variant pins a variant for later plans and sweeps (-1:

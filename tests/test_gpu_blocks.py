@@ -1,0 +1,38 @@
+"""Block kernels over the block extents and the edges of their work splits,
+against the oracle."""
+import numpy as np
+import pytest
+
+import iblgf_b200 as B
+import oracle_lib as O
+
+pytestmark = pytest.mark.gpu
+
+
+def rel_linf(a, b):
+    return float(np.abs(a - b).max() / max(np.abs(b).max(), 1e-300))
+
+
+def uneven(e, precision, **kw):
+    """3 x 2 x 1 base blocks (groups with 1, 2 and 4 of their 8 blocks, an odd number of groups), the block at the
+    origin refined once."""
+    args = ((-4 * e,) * 3, (8 * e,) * 3, e, 0.5, [((-2 * e, -e, 0), (3 * e, 2 * e, e))])
+    pred = lambda base, ext, rl, diff: rl == 0 and tuple(base) == (0, 0, 0)  # noqa: E731
+    return (O.Domain(*args, n_levels=1, predicate=pred),
+            B.Solver(*args, n_levels=1, predicate=pred, precision=precision, **kw))
+
+
+@pytest.mark.parametrize("variant", [0, 1])
+@pytest.mark.parametrize("precision,tol", [(B.FP64, 1e-12), (B.FP32, 1e-5)])
+@pytest.mark.parametrize("e", [4, 6, 8, 10, 14, 16])
+def test_solve_uneven_octree(e, precision, tol, variant):
+    """apply_lgf with both shapes of the direct MAC, twice on the same context (the second from scratch fields that
+    the first has filled); tolerances: the FP64 and FP32 parity bars."""
+    o, g = uneven(e, precision)
+    g.mac_variant(variant)
+    src = np.random.default_rng(e).standard_normal((o.n, o.Nb, o.Nb, o.Nb))
+    ref = o.apply_lgf(src)
+    fs, ft = g.field(src), g.field()
+    for _ in range(2):
+        g.apply_lgf(fs, ft)
+        assert rel_linf(g.download(ft), ref) < tol
