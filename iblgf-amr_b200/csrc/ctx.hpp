@@ -342,6 +342,7 @@ struct Ctx
     // fields
     std::vector<std::unique_ptr<Field>> fields;
     int f_source_tmp = -1, f_target_tmp = -1, f_correction_tmp = -1, f_fmm_s = -1, f_fmm_t = -1;
+    int f_if_tmp[2] = {-1, -1};  // source copies of a vector integrating factor's components y, z (on first use)
 
     // LGF table (device), twiddles, transfer matrices
     DevBuf<double> d_lgf_table;
@@ -509,14 +510,29 @@ void ib_warmstart_info(Ctx& c, double* info);
 void ws_check(Ctx& c, int S, int N, const float* params, const float* x, const float* tgt, float* y, float* grads,
               float* loss);
 int ge_table(Ctx& c, double alpha);
-// rp: relative position per axis of the field's mesh object (cell {1,1,1} when null)
-void apply_if(Ctx& c, int src, int tgt, double alpha_base, int fmm_type, const int* rp = nullptr);
+void apply_if(Ctx& c, int src, int tgt, double alpha_base, int fmm_type);
+// n component fields (1 .. 3) at once; rp: relative position per component and
+// axis of the field's mesh object (cell {1,1,1})
+void apply_if_vf(Ctx& c, int n, const int* src, const int* tgt, double alpha_base, int fmm_type, const int (*rp)[3]);
 
+// Targets and neighbour sources of all integrating-factor sweeps of a level
+// together (iblgf_poisson_apply_if): every octant of the level with the sources
+// that any of its sweeps gives it. usable: no source is given twice.
+struct IfLevel
+{
+    int n = 0, sweeps = 0;
+    bool usable = false;
+    long long n_src = 0, n_tgt = 0, n_pairs = 0;
+    DevBuf<int> tgt, src;
+};
 // device block lists of the Poisson level loop and of the level-wise operators
 struct PoissonLists
 {
     DevBuf<int> all, leaves;
     std::vector<DevBuf<int>> level_all, level_leaves;
+    DevBuf<int> leaf;                    // per octant: 1 for leaves
+    // per (level, IB2xIB or not), built on first use
+    std::map<std::pair<int, bool>, std::unique_ptr<IfLevel>> if_levels;
     std::vector<TpTasks> coarsify;       // per level ls (dst parents at ls)
     std::vector<TpTasks> cc_intrp;       // per level l: children of level-l octants
     std::vector<TpTasks> corr_intrp;     // per level l: correction children
@@ -574,10 +590,13 @@ bool toeplitz_mac(Ctx& c, const FmmPlan& p, const void* src_spec, void* acc);
 // the coefficient table of level difference ld from the 343 spectrum slots
 // of its offsets (created once per context)
 int combo_table(Ctx& c, int ld, const std::vector<int>& slots);
-// direct separable sweep of a neighbour-only plan with integrating-factor
-// table ge (adds into ft); false if the plan or the table does not allow it
+// direct separable sweep with integrating-factor table ge (which ge_direct_ok
+// must allow) of n component fields: target octants tgt, their 27 source octants
+// each (src, -1: none), whose interiors are read; adds into or assigns to the
+// targets' blocks
 bool ge_direct_ok(const Ctx& c, int ge);
-bool launch_ge_direct(Ctx& c, const FmmPlan& p, const double* fs, double* ft, int ge, double scale);
+void launch_ge_direct(Ctx& c, const int* tgt, const int* src, int n_tgt, const double* const* from, double* const* to,
+                      int n, int ge, double scale, bool assign);
 // tensor-core sibling-group MAC (FP32 path); false if not applicable
 bool tc_mac_ok(const Ctx& c, const FmmPlan& p);
 bool tc_mac(Ctx& c, const FmmPlan& p, const void* src_spec, void* acc);
@@ -625,7 +644,14 @@ void launch_tp(Ctx& c, const TpTasks& t, const double* src, double* dst, int mat
 // per-axis matrix pairs (mat_base[3]): face / edge components of the cell-centred transfers
 void launch_tp_axes(Ctx& c, const TpTasks& t, const double* src, double* dst, const int* mat_base, int mode,
                     bool fp32 = false);
+// the component fields of one vector field (n = 1 .. 3) in one launch, each
+// with its matrix pairs per axis (at most two different ones)
+void launch_tp_vf(Ctx& c, const TpTasks& t, const double* const* src, double* const* dst, int n,
+                  const int (*mat_base)[3], int mode, bool fp32 = false);
 void launch_halo(Ctx& c, double* f, const int* list, int n);
+void launch_halo_vf(Ctx& c, double* const* f, int m, const int* list, int n);
+// dst = src on the blocks whose flag is set, 0 on the others, n component fields
+void launch_masked_copy_vf(Ctx& c, const double* const* src, double* const* dst, int n, const int* flag);
 void launch_source_correction(Ctx& c, const double* target_tmp, double* corr, const int* list, int n,
                               double inv_dx2);
 void launch_op(Ctx& c, int op, const double* const* in, int n_in, double* const* out, int n_out, const int* list,

@@ -336,7 +336,8 @@ void apply_schur(Ctx& c, IbState& s, const int* src, const int* tgt)
 {
     OpLists& ol = op_lists(c);
     const int l = c.tree.depth - 1;
-    for (int k = 0; k < 3; ++k) launch_halo(c, c.field(src[k]), ol.list[l].p, (int)ol.list[l].n);
+    double* ph[3] = {c.field(src[0]), c.field(src[1]), c.field(src[2])};
+    launch_halo_vf(c, ph, 3, ol.list[l].p, (int)ol.list[l].n);
     const double* pin[3] = {c.field(src[0]), c.field(src[1]), c.field(src[2])};
     double* pc[1] = {c.field(s.cell_aux2)};
     launch_op(c, 2, pin, 3, pc, 1, ol.list[l].p, ol.dx[l].p, (int)ol.list[l].n, 1.0);
@@ -348,11 +349,8 @@ void apply_schur(Ctx& c, IbState& s, const int* src, const int* tgt)
     const double* pg[1] = {c.field(s.cell_aux2)};
     double* pt[3] = {c.field(tgt[0]), c.field(tgt[1]), c.field(tgt[2])};
     launch_op(c, 1, pg, 1, pt, 3, ol.list[l].p, ol.dx[l].p, (int)ol.list[l].n, 1.0);
-    for (int k = 0; k < 3; ++k)
-    {
-        launch_halo(c, pt[k], ol.list[l].p, (int)ol.list[l].n);
-        launch_face_planes(c, pt[k], s.ibc_list.p, s.ibc_faces.p, s.n_ibc, 2);
-    }
+    launch_halo_vf(c, pt, 3, ol.list[l].p, (int)ol.list[l].n);
+    for (int k = 0; k < 3; ++k) launch_face_planes(c, pt[k], s.ibc_list.p, s.ibc_faces.p, s.n_ibc, 2);
 }
 
 // LinSysSolver::ET_H_S_E (linsys.hpp:260-297): device forces in, device
@@ -361,13 +359,8 @@ void et_h_s_e(Ctx& c, IbState& s, const double* fin, double* fout, double alpha)
 {
     for (int k = 0; k < 3; ++k) launch_fill_zero(c, c.field(s.face_aux[k]), c.field_elems());
     smearing(c, s, fin, s.face_aux2);
-    if (std::fabs(alpha) > 1e-14)
-        for (int k = 0; k < 3; ++k)
-        {
-            int rp[3] = {1, 1, 1};
-            rp[k] = 0;  // face component k
-            apply_if(c, s.face_aux2[k], s.face_aux2[k], alpha, IBLGF_IB2xIB, rp);
-        }
+    static const int face[3][3] = {{0, 1, 1}, {1, 0, 1}, {1, 1, 0}};  // relative positions of face components
+    if (std::fabs(alpha) > 1e-14) apply_if_vf(c, 3, s.face_aux2, s.face_aux2, alpha, IBLGF_IB2xIB, face);
     apply_schur(c, s, s.face_aux2, s.face_aux);
     for (int k = 0; k < 3; ++k) launch_axpby(c, c.field(s.face_aux2[k]), c.field(s.face_aux[k]), -1.0, 1);
     projection(c, s, s.face_aux2, fout);
@@ -738,7 +731,8 @@ void ns_ib_stage(Ctx& c, int stage, double alpha, double threshold, int max_iter
     const int l = c.tree.depth - 1;
     launch_fill_zero(c, c.field(s.cell_aux2), c.field_elems());
     smearing(c, s, s.cg_f.p, s.face_aux2);
-    for (int k = 0; k < 3; ++k) launch_halo(c, c.field(s.face_aux2[k]), ol.list[l].p, (int)ol.list[l].n);
+    double* ph[3] = {c.field(s.face_aux2[0]), c.field(s.face_aux2[1]), c.field(s.face_aux2[2])};
+    launch_halo_vf(c, ph, 3, ol.list[l].p, (int)ol.list[l].n);
     const double* pin[3] = {c.field(s.face_aux2[0]), c.field(s.face_aux2[1]), c.field(s.face_aux2[2])};
     double* pc[1] = {c.field(s.cell_aux2)};
     launch_op(c, 2, pin, 3, pc, 1, ol.list[l].p, ol.dx[l].p, (int)ol.list[l].n, 1.0);

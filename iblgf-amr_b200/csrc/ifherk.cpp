@@ -393,34 +393,46 @@ class Step
         for (int k = 0; k < f.n; ++k) t[k] = F(f.id[k]);
         launch_axpby_vf(c, t, nullptr, f.n, a_, 2);
     }
+    // field pointers and transfer matrices of the components
+    void comps(const VF& f, double* (&p)[3]) const
+    {
+        for (int k = 0; k < f.n; ++k) p[k] = c.field(f.id[k]);
+    }
+    void mats(const VF& f, int one, int zero, int (&m)[3][3]) const
+    {
+        for (int k = 0; k < f.n; ++k)
+        {
+            int rp[3];
+            relpos(f.mesh, k, rp);
+            for (int a_ = 0; a_ < 3; ++a_) m[k][a_] = rp[a_] ? one : zero;
+        }
+    }
     void exchange(const VF& f, int l)
     {
-        for (int k = 0; k < f.n; ++k) launch_halo(c, F(f.id[k]), ol.list[l].p, (int)ol.list[l].n);
+        double* p[3];
+        comps(f, p);
+        launch_halo_vf(c, p, f.n, ol.list[l].p, (int)ol.list[l].n);
     }
     // source_coarsify (poisson.hpp:1136-1194) into the field itself
     void up(const VF& f)
     {
-        for (int k = 0; k < f.n; ++k)
-        {
-            int rp[3], m[3];
-            relpos(f.mesh, k, rp);
-            for (int a_ = 0; a_ < 3; ++a_) m[a_] = rp[a_] ? 4 : 8;
-            for (int ls = depth - 2; ls >= bl; --ls) launch_tp_axes(c, pl.coarsify[ls], F(f.id[k]), F(f.id[k]), m, 0);
-        }
+        double* p[3];
+        int m[3][3];
+        comps(f, p);
+        mats(f, 4, 8, m);
+        for (int ls = depth - 2; ls >= bl; --ls) launch_tp_vf(c, pl.coarsify[ls], p, p, f.n, m, 0);
     }
     // intrp_to_correction_buffer (poisson.hpp:1015-1069), correction children only
     void down_to_correction(const VF& f)
     {
-        for (int k = 0; k < f.n; ++k)
+        double* p[3];
+        int m[3][3];
+        comps(f, p);
+        mats(f, 2, 6, m);
+        for (int l = depth - 2; l >= bl; --l)
         {
-            int rp[3], m[3];
-            relpos(f.mesh, k, rp);
-            for (int a_ = 0; a_ < 3; ++a_) m[a_] = rp[a_] ? 2 : 6;
-            for (int l = depth - 2; l >= bl; --l)
-            {
-                launch_halo(c, F(f.id[k]), ol.list[l].p, (int)ol.list[l].n);
-                launch_tp_axes(c, pl.corr_intrp[l], F(f.id[k]), F(f.id[k]), m, 2);
-            }
+            launch_halo_vf(c, p, f.n, ol.list[l].p, (int)ol.list[l].n);
+            launch_tp_vf(c, pl.corr_intrp[l], p, p, f.n, m, 2);
         }
     }
     void up_and_down(const VF& f)
@@ -490,14 +502,11 @@ class Step
             exchange(tgt, l);
         }
     }
-    void apply_if(const VF& src, const VF& tgt, double alpha_base)
+    void apply_if(const VF& src, const VF& tgt, double alpha_base, int type = IBLGF_AMR2AMR)
     {
-        for (int k = 0; k < src.n; ++k)
-        {
-            int rp[3];
-            relpos(src.mesh, k, rp);
-            iblgf_b200::apply_if(c, src.id[k], tgt.id[k], alpha_base, IBLGF_AMR2AMR, rp);
-        }
+        int rp[3][3];
+        for (int k = 0; k < src.n; ++k) relpos(src.mesh, k, rp[k]);
+        iblgf_b200::apply_if_vf(c, src.n, src.id, tgt.id, alpha_base, type, rp);
     }
     void lin_sys(double alpha_k)
     {
@@ -513,13 +522,7 @@ class Step
             copy(s.r_i, fa2, 1.0);
             gradient(s.d_i, s.face_aux);
             add(s.face_aux, fa2, -1.0);
-            if (std::fabs(alpha_k) > 1e-14)
-                for (int k = 0; k < 3; ++k)
-                {
-                    int rp[3];
-                    relpos(kFace, k, rp);
-                    iblgf_b200::apply_if(c, fa2.id[k], fa2.id[k], alpha_k, IBLGF_IB2xIB, rp);
-                }
+            if (std::fabs(alpha_k) > 1e-14) apply_if(fa2, fa2, alpha_k, IBLGF_IB2xIB);
             ns_ib_stage(c, stage, alpha_k, opt.cg_threshold, opt.cg_max_iter, s.d_i.id[0], s.face_aux.id,
                         [&]() { gradient(s.d_i, s.face_aux); }, write_prev);
             add(s.face_aux, s.r_i, -1.0);

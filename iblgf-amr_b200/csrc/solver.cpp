@@ -423,7 +423,10 @@ void build_ib_masks(Ctx& c, std::vector<int>& ib)
         for (int o : c.level_octs[lv]) mv.set(o, (ib[o] & 1) != 0, true);
         upward_pass(c, lv, mv);
     }
-    // plans built from the previous masks are stale
+    // plans and lists built from the previous masks are stale
+    if (auto* pl = c.ext_get<PoissonLists>(Ctx::kExtPLists))
+        for (auto it = pl->if_levels.begin(); it != pl->if_levels.end();)
+            it = it->first.second ? pl->if_levels.erase(it) : std::next(it);
     for (auto it = c.plans.begin(); it != c.plans.end();)
     {
         const int idx = std::get<0>(it->first);
@@ -1312,6 +1315,19 @@ void run_sweep(Ctx& c, FmmPlan& p, int src, int tgt, double dx_level, double add
     double* ft = c.field(c.f_fmm_t);
     Timer tm(c);
     tm.mark(0);
+    // integrating-factor sweeps whose kernel is short: direct separable sums
+    // instead of transforms (same result to FP64 rounding), from the source
+    // field into the target field unless these are one or the sweep is sharded
+    const bool direct = ge >= 0 && c.ge_direct_enabled && p.n_ge && ge_direct_ok(c, ge);
+    if (direct && src != tgt && c.owner.empty())
+    {
+        const double* from = c.field(src);
+        double* to = c.field(tgt);
+        for (int i = 1; i < 4; ++i) tm.mark(i);
+        launch_ge_direct(c, p.ge_tgt.p, p.ge_src.p, p.n_ge, &from, &to, 1, ge, add_with_scale, false);
+        tm.mark(4);
+        return;
+    }
     launch_zero_blocks(c, fs, p.zero_s.p, (int)p.zero_s.n);
     launch_zero_blocks(c, ft, p.zero_t.p, (int)p.zero_t.n);
     launch_copy_interior(c, c.field(src), fs, p.copy_s.p, (int)p.copy_s.n);
@@ -1322,9 +1338,6 @@ void run_sweep(Ctx& c, FmmPlan& p, int src, int tgt, double dx_level, double add
     for (auto& t : p.antrp) launch_tp(c, t, fs, fs, 0, 0, fp32);
     tm.mark(1);
     const size_t cb = c.cplx_bytes();
-    // integrating-factor sweeps whose kernel is negligible beyond 8 cells:
-    // direct separable sums instead of transforms (same result to FP64 rounding)
-    const bool direct = ge >= 0 && c.ge_direct_enabled && p.n_ge && ge_direct_ok(c, ge);
     if (!p.empty() && !direct)
     {
         // the source spectra and one zero row after them (absent MAC candidates read it)
@@ -1337,7 +1350,11 @@ void run_sweep(Ctx& c, FmmPlan& p, int src, int tgt, double dx_level, double add
     tm.mark(2);
     if (!p.empty() && !direct) launch_mac(c, p, c.d_src_spec.p, c.d_acc.p);
     tm.mark(3);
-    if (!p.empty() && direct) launch_ge_direct(c, p, fs, ft, ge, 1.0);
+    if (direct)
+    {
+        const double* from = fs;
+        launch_ge_direct(c, p.ge_tgt.p, p.ge_src.p, p.n_ge, &from, &ft, 1, ge, 1.0, false);
+    }
     else if (!p.empty())
     {
         // compute_influence_field (fmm.hpp:1021-1026): dx^2 for LGF_GL, 1 for LGF_GE
@@ -1371,6 +1388,9 @@ PoissonLists& poisson_lists(Ctx& c)
         all.push_back(i);
         if (c.flags[i] & 1) leaves.push_back(i);
     }
+    std::vector<int> leaf(c.n_oct);
+    for (int i = 0; i < c.n_oct; ++i) leaf[i] = c.flags[i] & 1;
+    pl->leaf.upload(leaf, c.stream);
     pl->all.upload(all, c.stream);
     pl->leaves.upload(leaves, c.stream);
     const int L = kMaxLevel + 1;
@@ -1563,54 +1583,171 @@ int ge_table(Ctx& c, double alpha)
     return idx;
 }
 
-// PoissonSolver::apply_lgf_IF / apply_if (poisson.hpp:428-494), AMR2AMR
-void apply_if(Ctx& c, int src, int tgt, double alpha_base, int fmm_type, const int* rp)
+namespace
+{
+// the sweeps apply_if makes at a level: the IB2xIB mask's, or the AMR2AMR
+// masks of non_leaf_as_source false and (unless subtract_non_leaf) true
+IfLevel& if_level(Ctx& c, PoissonLists& pl, int l, bool ib)
+{
+    auto& slot = pl.if_levels[{l, ib}];
+    if (slot) return *slot;
+    auto lev = std::make_unique<IfLevel>();
+    std::vector<int> idx;
+    const int rl = l - c.tree.base_level;
+    if (ib) idx.push_back(mask_idx_gen(IBLGF_IB2xIB, rl, 0));
+    else idx.push_back(mask_idx_gen(IBLGF_AMR2AMR, rl, 0));
+    if (!ib && !c.subtract_non_leaf) idx.push_back(mask_idx_gen(IBLGF_AMR2AMR, rl, 1));
+    if (ib && c.subtract_non_leaf) idx.clear();
+    const int e = c.cfg.block_extent;
+    std::vector<int> tgt = c.level_octs[l], src(27 * c.level_octs[l].size(), -1);
+    lev->usable = true;
+    lev->sweeps = (int)idx.size();
+    for (int k : idx)
+    {
+        const auto& m = c.masks[k];
+        for (size_t t = 0; t < tgt.size(); ++t)
+        {
+            const int o = tgt[t];
+            if (m[2 * o]) ++lev->n_src;
+            if (!m[2 * o + 1]) continue;
+            bool any = false;
+            for (int i = 0; i < 27; ++i)
+            {
+                const int n = c.nbr[27 * (size_t)o + i];
+                if (n < 0 || !m[2 * n]) continue;
+                int at = 0;
+                for (int a = 0, w = 1; a < 3; ++a, w *= 3)
+                {
+                    const int d = c.bbase[3 * n + a] - c.bbase[3 * o + a];
+                    if (d != 0 && d != e && d != -e) lev->usable = false;
+                    at += (d / e + 1) * w;
+                }
+                if (!lev->usable || src[27 * t + at] >= 0)
+                {
+                    lev->usable = false;
+                    break;
+                }
+                src[27 * t + at] = n;
+                ++lev->n_pairs;
+                any = true;
+            }
+            lev->n_tgt += any ? 1 : 0;
+        }
+    }
+    lev->n = (int)tgt.size();
+    lev->tgt.upload(tgt, c.stream);
+    lev->src.upload(src, c.stream);
+    IBLGF_CUDA(cudaStreamSynchronize(c.stream));
+    slot = std::move(lev);
+    return *slot;
+}
+
+// all sweeps of level l from the copies st into tgt, assigned on every block of
+// the level; false where the direct sums do not apply
+bool if_level_direct(Ctx& c, PoissonLists& pl, int l, bool ib, int n, const int* st, const int* tgt, int ge)
+{
+    if (!c.ge_direct_enabled || !c.owner.empty() || !ge_direct_ok(c, ge)) return false;
+    IfLevel& lev = if_level(c, pl, l, ib);
+    if (!lev.usable) return false;
+    const double* from[3];
+    double* to[3];
+    for (int k = 0; k < n; ++k)
+    {
+        from[k] = c.field(st[k]);
+        to[k] = c.field(tgt[k]);
+    }
+    c.stats[0] += (long long)n * lev.sweeps;
+    c.stats[1] += n * lev.n_src;
+    c.stats[2] += n * lev.n_tgt;
+    c.stats[3] += n * lev.n_pairs;
+    launch_ge_direct(c, lev.tgt.p, lev.src.p, lev.n, from, to, n, ge, 1.0, true);
+    return true;
+}
+}  // namespace
+
+// PoissonSolver::apply_lgf_IF / apply_if (poisson.hpp:428-494). The sources
+// are copied first, so a target may be its source. Where the kernel is short
+// (ge_direct_ok) the sweeps of a level are one launch over its blocks and the
+// component fields, written straight to the targets; otherwise each sweep runs
+// through target_tmp.
+void apply_if_vf(Ctx& c, int n, const int* src, const int* tgt, double alpha_base, int fmm_type, const int (*rp)[3])
 {
     need_single(c);
-    static const int cell[3] = {1, 1, 1};
-    if (!rp) rp = cell;
-    // cell-centred transfer matrices per axis: relative position 1 -> [4,5]
-    // coarsify / [2,3] interpolate, relative position 0 -> [8,9] / [6,7]
-    const int coarse_m[3] = {rp[0] ? 4 : 8, rp[1] ? 4 : 8, rp[2] ? 4 : 8};
-    const int intrp_m[3] = {rp[0] ? 2 : 6, rp[1] ? 2 : 6, rp[2] ? 2 : 6};
     if (!c.finalized) throw Error(IBLGF_EINVAL, "domain not finalized");
     if (fmm_type != IBLGF_AMR2AMR && fmm_type != IBLGF_IB2xIB)
         throw Error(IBLGF_EINVAL, "apply_if supports AMR2AMR and IB2xIB");
+    if (n < 1 || n > 3) throw Error(IBLGF_EINVAL, "one to three component fields");
+    // cell-centred transfer matrices per axis: relative position 1 -> [4,5]
+    // coarsify / [2,3] interpolate, relative position 0 -> [8,9] / [6,7]
+    int coarse_m[3][3], intrp_m[3][3];
+    for (int k = 0; k < n; ++k)
+        for (int a = 0; a < 3; ++a)
+        {
+            coarse_m[k][a] = rp[k][a] ? 4 : 8;
+            intrp_m[k][a] = rp[k][a] ? 2 : 6;
+        }
     PoissonLists& pl = poisson_lists(c);
     OpLists& ol = op_lists(c);
-    double* st = c.field(c.f_source_tmp);
+    int st[3] = {c.f_source_tmp, -1, -1};
+    for (int k = 1; k < n; ++k)
+    {
+        if (c.f_if_tmp[k - 1] < 0) c.f_if_tmp[k - 1] = field_create(c);
+        st[k] = c.f_if_tmp[k - 1];
+    }
+    const double* ps[3];
+    double* pst[3];
+    const double* cst[3];
+    for (int k = 0; k < n; ++k)
+    {
+        ps[k] = c.field(src[k]);
+        cst[k] = pst[k] = c.field(st[k]);
+    }
     double* tt = c.field(c.f_target_tmp);
-    const size_t bytes = c.field_elems() * sizeof(double);
-    launch_fill_zero(c, st, bytes / sizeof(double));
-    launch_fill_zero(c, tt, bytes / sizeof(double));
     const int bl = c.tree.base_level, depth = c.tree.depth;
     if (fmm_type == IBLGF_IB2xIB)
     {
         // poisson.hpp:447-448, 465-494: finest level only, interior copy, the
         // non-leaf-as-source sweep with the IB2xIB mask, level copied out
         const int l = depth - 1;
-        launch_copy_interior(c, c.field(src), st, pl.level_all[l].p, (int)pl.level_all[l].n);
         const int ge = ge_table(c, alpha_base * std::pow(4.0, l - bl));
-        if (!c.subtract_non_leaf) fmm_apply(c, c.f_source_tmp, c.f_target_tmp, l, true, 1.0, IBLGF_IB2xIB, ge);
-        launch_axpy_blocks(c, tt, c.field(tgt), pl.level_all[l].p, (int)pl.level_all[l].n, 1.0, true);
+        for (int k = 0; k < n; ++k)
+            launch_copy_interior(c, ps[k], pst[k], pl.level_all[l].p, (int)pl.level_all[l].n);
+        if (if_level_direct(c, pl, l, true, n, st, tgt, ge)) return;
+        for (int k = 0; k < n; ++k)
+        {
+            launch_zero_blocks(c, tt, pl.level_all[l].p, (int)pl.level_all[l].n);
+            if (!c.subtract_non_leaf) fmm_apply(c, st[k], c.f_target_tmp, l, true, 1.0, IBLGF_IB2xIB, ge);
+            launch_axpy_blocks(c, tt, c.field(tgt[k]), pl.level_all[l].p, (int)pl.level_all[l].n, 1.0, true);
+        }
         return;
     }
-    launch_axpy_blocks(c, c.field(src), st, pl.leaves.p, (int)pl.leaves.n, 1.0, true);
-    for (int ls = depth - 2; ls >= bl; --ls) launch_tp_axes(c, pl.coarsify[ls], st, st, coarse_m, 0);
+    launch_masked_copy_vf(c, ps, pst, n, pl.leaf.p);
+    for (int ls = depth - 2; ls >= bl; --ls) launch_tp_vf(c, pl.coarsify[ls], cst, pst, n, coarse_m, 0);
     // intrp_to_correction_buffer (poisson.hpp:1015-1069)
     for (int l = depth - 2; l >= bl; --l)
     {
-        launch_halo(c, st, ol.list[l].p, (int)ol.list[l].n);
-        launch_tp_axes(c, pl.corr_intrp[l], st, st, intrp_m, 2);
+        launch_halo_vf(c, pst, n, ol.list[l].p, (int)ol.list[l].n);
+        launch_tp_vf(c, pl.corr_intrp[l], cst, pst, n, intrp_m, 2);
     }
     for (int l = bl; l < depth; ++l)
     {
         // LGF_GE::change_level_impl: alpha = alpha_base * 4^(l - base)
         const int ge = ge_table(c, alpha_base * std::pow(4.0, l - bl));
-        fmm_apply(c, c.f_source_tmp, c.f_target_tmp, l, false, 1.0, IBLGF_AMR2AMR, ge);
-        if (!c.subtract_non_leaf) fmm_apply(c, c.f_source_tmp, c.f_target_tmp, l, true, 1.0, IBLGF_AMR2AMR, ge);
-        launch_axpy_blocks(c, tt, c.field(tgt), pl.level_all[l].p, (int)pl.level_all[l].n, 1.0, true);
+        if (if_level_direct(c, pl, l, false, n, st, tgt, ge)) continue;
+        for (int k = 0; k < n; ++k)
+        {
+            launch_zero_blocks(c, tt, pl.level_all[l].p, (int)pl.level_all[l].n);
+            fmm_apply(c, st[k], c.f_target_tmp, l, false, 1.0, IBLGF_AMR2AMR, ge);
+            if (!c.subtract_non_leaf) fmm_apply(c, st[k], c.f_target_tmp, l, true, 1.0, IBLGF_AMR2AMR, ge);
+            launch_axpy_blocks(c, tt, c.field(tgt[k]), pl.level_all[l].p, (int)pl.level_all[l].n, 1.0, true);
+        }
     }
+}
+
+void apply_if(Ctx& c, int src, int tgt, double alpha_base, int fmm_type)
+{
+    static const int cell[1][3] = {{1, 1, 1}};
+    apply_if_vf(c, 1, &src, &tgt, alpha_base, fmm_type, cell);
 }
 
 void poisson_release(Ctx& c)

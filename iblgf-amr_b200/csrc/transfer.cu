@@ -23,17 +23,27 @@ namespace iblgf_b200
 {
 namespace
 {
-// The Nb x Nb matrices of a transfer per axis and child bit, passed by
-// value: they sit in the constant bank, and with the passes fully unrolled
-// every matrix entry is an FMA operand at a fixed offset (no shared-memory
-// loads). Face and edge components use different matrices per axis.
+// The Nb x Nb matrices of a transfer per set and child bit, passed by
+// value: they sit in the constant bank, and with the dense passes fully
+// unrolled every matrix entry is an FMA operand at a fixed offset (no
+// shared-memory loads). Face and edge components use one of two sets per axis
+// (their relative positions 0 and 1); set[c][a] is that of component c and
+// axis a. Dense transfers have one set.
 // lo: for the banded passes (W > 0), first column of row m's band of width W
 // in summation order (the row's nonzeros all lie in [lo, lo + W))
 template<int NB, class T>
 struct TpMats
 {
-    T m[3][2][NB * NB];
-    unsigned char lo[3][2][NB];
+    T m[2][2][NB * NB];
+    unsigned char lo[2][2][NB];
+    unsigned char set[3][3];
+};
+
+// the component fields of one transfer (blockIdx.y = component)
+struct TpFields
+{
+    const double* src[3];
+    double* dst[3];
 };
 
 template<int NB>
@@ -54,9 +64,9 @@ constexpr int tp_threads()
 // sum unchanged, so the result equals the full row's
 // T: arithmetic and shared-memory type of the passes (the accumulators acc,
 // which start from and end in the FP64 target block, stay FP64)
-template<int NB, int A, int K, bool TR, bool LAST, int W, class T>
+template<int NB, int K, bool TR, bool LAST, int W, class T>
 __device__ __forceinline__ void tp_pass(const T* __restrict__ in, T* __restrict__ out,
-                                        const TpMats<NB, T>& mt, int p, double* acc)
+                                        const TpMats<NB, T>& mt, int set, int p, double* acc)
 {
     if constexpr (W == 0)
     {
@@ -68,7 +78,7 @@ __device__ __forceinline__ void tp_pass(const T* __restrict__ in, T* __restrict_
         {
             T s = 0;
 #pragma unroll
-            for (int n = 0; n < NB; ++n) s = fma(TR ? mt.m[A][K][n * NB + m] : mt.m[A][K][m * NB + n], v[n], s);
+            for (int n = 0; n < NB; ++n) s = fma(TR ? mt.m[0][K][n * NB + m] : mt.m[0][K][m * NB + n], v[n], s);
             if (LAST) acc[m] += s;
             else out[m * NB * NB + p] = s;
         }
@@ -76,16 +86,17 @@ __device__ __forceinline__ void tp_pass(const T* __restrict__ in, T* __restrict_
     else
     {
         const T* row = in + p * NB;
+        const T* mat = mt.m[set][K];
 #pragma unroll
         for (int m = 0; m < NB; ++m)
         {
-            const int lo = mt.lo[A][K][m];
+            const int lo = mt.lo[set][K][m];
             T s = 0;
 #pragma unroll
             for (int j = 0; j < W; ++j)
             {
                 const int n = lo + j;
-                s = fma(TR ? mt.m[A][K][n * NB + m] : mt.m[A][K][m * NB + n], row[n], s);
+                s = fma(TR ? mat[n * NB + m] : mat[m * NB + n], row[n], s);
             }
             if (LAST) acc[m] += s;
             else out[m * NB * NB + p] = s;
@@ -93,11 +104,12 @@ __device__ __forceinline__ void tp_pass(const T* __restrict__ in, T* __restrict_
     }
 }
 
-template<int NB, int A, bool TR, bool LAST, int W, class T>
-__device__ __forceinline__ void tp_pass_bit(int bit, const T* in, T* out, const TpMats<NB, T>& mt, int p, double* acc)
+template<int NB, bool TR, bool LAST, int W, class T>
+__device__ __forceinline__ void tp_pass_bit(int bit, const T* in, T* out, const TpMats<NB, T>& mt, int set, int p,
+                                            double* acc)
 {
-    if (bit) tp_pass<NB, A, 1, TR, LAST, W, T>(in, out, mt, p, acc);
-    else tp_pass<NB, A, 0, TR, LAST, W, T>(in, out, mt, p, acc);
+    if (bit) tp_pass<NB, 1, TR, LAST, W, T>(in, out, mt, set, p, acc);
+    else tp_pass<NB, 0, TR, LAST, W, T>(in, out, mt, set, p, acc);
 }
 
 // mode 0: dst[group] += sum_tasks A(src)        (anterpolation / coarsify)
@@ -108,10 +120,12 @@ __device__ __forceinline__ void tp_pass_bit(int bit, const T* in, T* out, const 
 template<int NB, bool TR, int W, class T>
 __global__ void __launch_bounds__(tp_threads<NB>(), 2) tp_kernel(
     const int* __restrict__ gptr, const int* __restrict__ gdst, const int* __restrict__ tsrc,
-    const int* __restrict__ tcid, const double* __restrict__ src, double* __restrict__ dst,
-    const __grid_constant__ TpMats<NB, T> mt, int mode)
+    const int* __restrict__ tcid, const __grid_constant__ TpFields f, const __grid_constant__ TpMats<NB, T> mt, int mode)
 {
     constexpr int N3 = NB * NB * NB;
+    const double* src = f.src[blockIdx.y];
+    double* dst = f.dst[blockIdx.y];
+    const unsigned char* set = mt.set[blockIdx.y];
     extern __shared__ __align__(16) unsigned char tp_smem[];
     T* a = reinterpret_cast<T*>(tp_smem);
     T* b = a + N3;
@@ -134,11 +148,11 @@ __global__ void __launch_bounds__(tp_threads<NB>(), 2) tp_kernel(
             a[2 * i + 1] = (T)v.y;
         }
         __syncthreads();
-        if (active) tp_pass_bit<NB, 0, TR, false, W, T>(cid & 1, a, b, mt, p, acc);
+        if (active) tp_pass_bit<NB, TR, false, W, T>(cid & 1, a, b, mt, set[0], p, acc);
         __syncthreads();
-        if (active) tp_pass_bit<NB, 1, TR, false, W, T>((cid >> 1) & 1, b, a, mt, p, acc);
+        if (active) tp_pass_bit<NB, TR, false, W, T>((cid >> 1) & 1, b, a, mt, set[1], p, acc);
         __syncthreads();
-        if (active) tp_pass_bit<NB, 2, TR, true, W, T>((cid >> 2) & 1, a, (T*)nullptr, mt, p, acc);
+        if (active) tp_pass_bit<NB, TR, true, W, T>((cid >> 2) & 1, a, (T*)nullptr, mt, set[2], p, acc);
         __syncthreads();
     }
     if (!active) return;
@@ -146,77 +160,97 @@ __global__ void __launch_bounds__(tp_threads<NB>(), 2) tp_kernel(
     for (int m = 0; m < NB; ++m) d[m * NB * NB] = acc[m];
 }
 
-// Width-2 band, sending-side form (mode 0, coarsening): thread p = (x', y')
-// owns the receiving z-pencil, as in the last pass of tp_kernel, and forms
-// the three passes' values it needs straight from the sending block in
-// registers, in the passes' order (x band, then y band, then z band, the
-// band entries in summation order): the same FMAs as tp_kernel<NB, false, 2>
-// without the shared-memory staging and its barriers. Sending blocks whose x
-// or y band is zero for the thread (they feed other octants of the
-// receiving block) are skipped: their sums would add exact zeros.
+// Width-2 band (mode 0, coarsening): each receiving node takes 2 x 2 x 2 nodes
+// of the one sending block that covers it (per axis, the child bit whose row of
+// this node is not zero; buffer nodes receive nothing). One thread per
+// receiving node, so the 8 loads of a node and those of a thread's kBandNodes
+// nodes are in flight together; the sums run in the order of the separable
+// passes (x band, then y, then z, entries in summation order).
+// Measured at Nb = 18 on the vortex ring's coarsening (40 to 248 receiving
+// blocks): 55 us per component with one thread per receiving z pencil, whose
+// sending blocks and planes followed one another.
+constexpr int kBandNodes = 4;
+
 template<int NB, class T>
-__global__ void __launch_bounds__(tp_threads<NB>(), 2) tp_band2_kernel(
-    const int* __restrict__ gptr, const int* __restrict__ gdst, const int* __restrict__ tsrc,
-    const int* __restrict__ tcid, const double* __restrict__ src, double* __restrict__ dst,
-    const __grid_constant__ TpMats<NB, T> mt)
+__global__ void __launch_bounds__(256) tp_band2_kernel(const int* __restrict__ gptr, const int* __restrict__ gdst,
+                                                       const int* __restrict__ tsrc, const int* __restrict__ tcid,
+                                                       const __grid_constant__ TpFields f, const __grid_constant__ TpMats<NB, T> mt)
 {
-    constexpr int N3 = NB * NB * NB;
+    constexpr int N3 = NB * NB * NB, E = NB - 2, E3 = E * E * E;
+    __shared__ int child[8];           // sending block per child id, -1: none
+    __shared__ unsigned char bit[3][NB], lo[3][NB];
+    __shared__ T w0[3][NB], w1[3][NB];
+    const double* __restrict__ src = f.src[blockIdx.y];
     const int g = blockIdx.x;
-    const int p = threadIdx.x;
-    if (p >= NB * NB) return;
-    const int xo = p % NB, yo = p / NB;
-    double* d = dst + (size_t)gdst[g] * N3 + p;
-    double acc[NB];
-#pragma unroll
-    for (int m = 0; m < NB; ++m) acc[m] = d[m * NB * NB];
-    for (int t = gptr[g]; t < gptr[g + 1]; ++t)
+    if (threadIdx.x < 8) child[threadIdx.x] = -1;
+    for (int i = threadIdx.x; i < 3 * NB; i += blockDim.x)
     {
-        const int cid = tcid[t];
-        const int kx = cid & 1, ky = (cid >> 1) & 1, kz = (cid >> 2) & 1;
-        const int lx = mt.lo[0][kx][xo], ly = mt.lo[1][ky][yo];
-        const T wx0 = mt.m[0][kx][xo * NB + lx], wx1 = mt.m[0][kx][xo * NB + lx + 1];
-        const T wy0 = mt.m[1][ky][yo * NB + ly], wy1 = mt.m[1][ky][yo * NB + ly + 1];
-        if ((wx0 == (T)0 && wx1 == (T)0) || (wy0 == (T)0 && wy1 == (T)0)) continue;
-        const double* blk = src + (size_t)tsrc[t] * N3;
-        T cz[NB];
-#pragma unroll
-        for (int nz = 0; nz < NB; ++nz)
+        // the child bit whose row of node m is not zero, and its band
+        const int a = i / NB, m = i % NB, s = mt.set[blockIdx.y][a];
+        int k = 0, l = mt.lo[s][0][m];
+        T u = mt.m[s][0][m * NB + l], v = mt.m[s][0][m * NB + l + 1];
+        if (u == (T)0 && v == (T)0)
         {
-            const double* r0 = blk + (size_t)(nz * NB + ly) * NB + lx;
-            const double* r1 = r0 + NB;
-            T b0 = 0, b1 = 0;
-            b0 = fma(wx0, (T)__ldg(r0), b0);
-            b0 = fma(wx1, (T)__ldg(r0 + 1), b0);
-            b1 = fma(wx0, (T)__ldg(r1), b1);
-            b1 = fma(wx1, (T)__ldg(r1 + 1), b1);
-            T c = 0;
-            c = fma(wy0, b0, c);
-            c = fma(wy1, b1, c);
-            cz[nz] = c;
+            k = 1;
+            l = mt.lo[s][1][m];
+            u = mt.m[s][1][m * NB + l];
+            v = mt.m[s][1][m * NB + l + 1];
         }
+        bit[a][m] = (unsigned char)k;
+        lo[a][m] = (unsigned char)l;
+        w0[a][m] = u;
+        w1[a][m] = v;
+    }
+    __syncthreads();
+    for (int t = gptr[g] + threadIdx.x; t < gptr[g + 1]; t += blockDim.x) child[tcid[t]] = tsrc[t];
+    __syncthreads();
+    double* __restrict__ d = f.dst[blockIdx.y] + (size_t)gdst[g] * N3;
+    const int i0 = blockIdx.z * (256 * kBandNodes) + threadIdx.x;
+    double v[kBandNodes][8], old[kBandNodes];
+    int at[kBandNodes];
 #pragma unroll
-        for (int m = 0; m < NB; ++m)
-        {
-            const int lz = mt.lo[2][kz][m];
-            T s = 0;
-            s = fma(mt.m[2][kz][m * NB + lz], cz[lz], s);
-            s = fma(mt.m[2][kz][m * NB + lz + 1], cz[lz + 1], s);
-            acc[m] += s;
-        }
+    for (int k = 0; k < kBandNodes; ++k)
+    {
+        const int i = i0 + 256 * k;
+        at[k] = -1;
+        if (i >= E3) continue;
+        const int x = 1 + i % E, y = 1 + (i / E) % E, z = 1 + i / (E * E);
+        const int b = child[bit[0][x] + 2 * bit[1][y] + 4 * bit[2][z]];
+        if (b < 0) continue;
+        at[k] = (z * NB + y) * NB + x;
+        const double* p = src + (size_t)b * N3 + (lo[2][z] * NB + lo[1][y]) * NB + lo[0][x];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[k][j] = p[(j >> 2) * NB * NB + ((j >> 1) & 1) * NB + (j & 1)];
+        old[k] = d[at[k]];
     }
 #pragma unroll
-    for (int m = 0; m < NB; ++m) d[m * NB * NB] = acc[m];
+    for (int k = 0; k < kBandNodes; ++k)
+    {
+        if (at[k] < 0) continue;
+        const int x = at[k] % NB, y = (at[k] / NB) % NB, z = at[k] / (NB * NB);
+        const T x0 = w0[0][x], x1 = w1[0][x], y0 = w0[1][y], y1 = w1[1][y];
+        T c[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+        {
+            const T b0 = fma(x1, (T)v[k][4 * j + 1], fma(x0, (T)v[k][4 * j], (T)0));
+            const T b1 = fma(x1, (T)v[k][4 * j + 3], fma(x0, (T)v[k][4 * j + 2], (T)0));
+            c[j] = fma(y1, b1, fma(y0, b0, (T)0));
+        }
+        d[at[k]] = old[k] + fma(w1[2][z], c[1], fma(w0[2][z], c[0], (T)0));
+    }
 }
 
 // threads walk the buffer shell only: the two z = 0, NB-1 planes, then per
 // inner z plane its ring (rows y = 0, NB-1, columns x = 0, NB-1)
 template<int NB>
-__global__ void halo_kernel(double* __restrict__ f, const int* __restrict__ list, const int* __restrict__ nbr,
+__global__ void halo_kernel(const __grid_constant__ TpFields fs, const int* __restrict__ list, const int* __restrict__ nbr,
                             const int* __restrict__ bbase, int e)
 {
     constexpr int N3 = NB * NB * NB;
     constexpr int P2 = NB * NB, RING = 4 * NB - 4, SHELL = 2 * P2 + (NB - 2) * RING;
     const int o = list[blockIdx.x];
+    double* f = fs.dst[blockIdx.y];
     double* blk = f + (size_t)o * N3;
     for (int t = threadIdx.x; t < SHELL; t += blockDim.x)
     {
@@ -330,57 +364,67 @@ void nb_dispatch(int Nb, F&& f)
 
 void launch_tp(Ctx& c, const TpTasks& t, const double* src, double* dst, int mat_base, int mode, bool fp32)
 {
-    const int bases[3] = {mat_base, mat_base, mat_base};
-    launch_tp_axes(c, t, src, dst, bases, mode, fp32);
+    const int bases[1][3] = {{mat_base, mat_base, mat_base}};
+    launch_tp_vf(c, t, &src, &dst, 1, bases, mode, fp32);
 }
 
 namespace
 {
 template<int NB, class T>
-void launch_tp_typed(Ctx& c, const TpTasks& t, const double* src, double* dst, const int* mat_base, int mode)
+void launch_tp_typed(Ctx& c, const TpTasks& t, const TpFields& f, int n, const int (*mat_base)[3], int mode)
 {
     static_assert((NB * NB * NB) % 2 == 0, "blocks are copied as double2");
-    TpMats<NB, T> mt;
+    TpMats<NB, T> mt{};
     const bool tr = mode != 0;
     int width = 0;  // widest band of any row, in summation order
-    for (int a = 0; a < 3; ++a)
-    {
-        const size_t off = (size_t)mat_base[a] * NB * NB;
-        if (c.h_mats.size() < off + 2 * NB * NB) throw Error(IBLGF_EINTERNAL, "transfer matrices missing");
-        for (int k = 0; k < 2; ++k)
-            for (int i = 0; i < NB * NB; ++i) mt.m[a][k][i] = (T)c.h_mats[off + (size_t)k * NB * NB + i];
-        for (int k = 0; k < 2; ++k)
-            for (int m = 0; m < NB; ++m)
-            {
-                int lo = NB, hi = 0;
-                for (int n = 0; n < NB; ++n)
-                    if ((tr ? mt.m[a][k][n * NB + m] : mt.m[a][k][m * NB + n]) != (T)0)
-                    {
-                        lo = std::min(lo, n);
-                        hi = n + 1;
-                    }
-                mt.lo[a][k][m] = (unsigned char)(lo < hi ? lo : 0);
-                width = std::max(width, lo < hi ? hi - lo : 0);
-            }
-    }
-    const int W = width <= 2 ? 2 : (width <= 5 ? 5 : 0);
-    if (W)
+    int base[2] = {-1, -1};
+    for (int q = 0; q < n; ++q)
         for (int a = 0; a < 3; ++a)
+        {
+            int s = 0;
+            while (s < 2 && base[s] >= 0 && base[s] != mat_base[q][a]) ++s;
+            if (s == 2) throw Error(IBLGF_EINTERNAL, "a transfer takes two matrix sets at most");
+            mt.set[q][a] = (unsigned char)s;
+            if (base[s] >= 0) continue;
+            base[s] = mat_base[q][a];
+            const size_t off = (size_t)base[s] * NB * NB;
+            if (c.h_mats.size() < off + 2 * NB * NB) throw Error(IBLGF_EINTERNAL, "transfer matrices missing");
             for (int k = 0; k < 2; ++k)
-                for (int m = 0; m < NB; ++m) mt.lo[a][k][m] = (unsigned char)std::min<int>(mt.lo[a][k][m], NB - W);
+                for (int i = 0; i < NB * NB; ++i) mt.m[s][k][i] = (T)c.h_mats[off + (size_t)k * NB * NB + i];
+            for (int k = 0; k < 2; ++k)
+                for (int m = 0; m < NB; ++m)
+                {
+                    int lo = NB, hi = 0;
+                    for (int i = 0; i < NB; ++i)
+                        if ((tr ? mt.m[s][k][i * NB + m] : mt.m[s][k][m * NB + i]) != (T)0)
+                        {
+                            lo = std::min(lo, i);
+                            hi = i + 1;
+                        }
+                    mt.lo[s][k][m] = (unsigned char)(lo < hi ? lo : 0);
+                    width = std::max(width, lo < hi ? hi - lo : 0);
+                }
+        }
+    const int W = width <= 2 ? 2 : (width <= 5 ? 5 : 0);
+    if (!W && base[1] >= 0) throw Error(IBLGF_EINTERNAL, "dense transfers have one matrix set");
+    if (W)
+        for (int s = 0; s < 2; ++s)
+            for (int k = 0; k < 2; ++k)
+                for (int m = 0; m < NB; ++m) mt.lo[s][k][m] = (unsigned char)std::min<int>(mt.lo[s][k][m], NB - W);
     const size_t smem = 2 * (size_t)NB * NB * NB * sizeof(T);
     auto launch = [&](auto kfn) {
         IBLGF_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kfn<<<t.n_groups, tp_threads<NB>(), smem, c.stream>>>(t.group_ptr.p, t.group_dst.p, t.task_src.p,
-                                                              t.task_cid.p, src, dst, mt, mode);
+        kfn<<<dim3(t.n_groups, n), tp_threads<NB>(), smem, c.stream>>>(t.group_ptr.p, t.group_dst.p, t.task_src.p,
+                                                                       t.task_cid.p, f, mt, mode);
     };
     if (mode == 0)
     {
         if (W == 2)
         {
+            constexpr int per = 256 * kBandNodes, e3 = (NB - 2) * (NB - 2) * (NB - 2);
             auto kfn = tp_band2_kernel<NB, T>;
-            kfn<<<t.n_groups, tp_threads<NB>(), 0, c.stream>>>(t.group_ptr.p, t.group_dst.p, t.task_src.p,
-                                                              t.task_cid.p, src, dst, mt);
+            kfn<<<dim3(t.n_groups, n, (e3 + per - 1) / per), 256, 0, c.stream>>>(
+                t.group_ptr.p, t.group_dst.p, t.task_src.p, t.task_cid.p, f, mt);
         }
         else if (W == 5) launch(tp_kernel<NB, false, 5, T>);
         else launch(tp_kernel<NB, false, 0, T>);
@@ -396,28 +440,45 @@ void launch_tp_typed(Ctx& c, const TpTasks& t, const double* src, double* dst, c
 
 // fp32: the passes in FP32 (matrices rounded to FP32), the sums into the
 // FP64 receiving blocks in FP64
-void launch_tp_axes(Ctx& c, const TpTasks& t, const double* src, double* dst, const int* mat_base, int mode, bool fp32)
+void launch_tp_vf(Ctx& c, const TpTasks& t, const double* const* src, double* const* dst, int n,
+                  const int (*mat_base)[3], int mode, bool fp32)
 {
-    if (!t.n_groups) return;
+    if (!t.n_groups || n < 1) return;
+    TpFields f{};
+    for (int k = 0; k < n; ++k)
+    {
+        f.src[k] = src[k];
+        f.dst[k] = dst[k];
+    }
     nb_dispatch(c.Nb, [&](auto nbc) {
         constexpr int NB = decltype(nbc)::value;
-        if (fp32) launch_tp_typed<NB, float>(c, t, src, dst, mat_base, mode);
-        else launch_tp_typed<NB, double>(c, t, src, dst, mat_base, mode);
+        if (fp32) launch_tp_typed<NB, float>(c, t, f, n, mat_base, mode);
+        else launch_tp_typed<NB, double>(c, t, f, n, mat_base, mode);
     });
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }
 
-void launch_halo(Ctx& c, double* f, const int* list, int n)
+void launch_tp_axes(Ctx& c, const TpTasks& t, const double* src, double* dst, const int* mat_base, int mode, bool fp32)
 {
-    if (!n) return;
+    const int bases[1][3] = {{mat_base[0], mat_base[1], mat_base[2]}};
+    launch_tp_vf(c, t, &src, &dst, 1, bases, mode, fp32);
+}
+
+void launch_halo_vf(Ctx& c, double* const* f, int m, const int* list, int n)
+{
+    if (!n || m < 1) return;
+    TpFields p{};
+    for (int k = 0; k < m; ++k) p.dst[k] = f[k];
     nb_dispatch(c.Nb, [&](auto nbc) {
         constexpr int NB = decltype(nbc)::value;
-        halo_kernel<NB><<<n, 256, 0, c.stream>>>(f, list, c.d_nbr.p, c.d_bbase.p, c.cfg.block_extent);
+        halo_kernel<NB><<<dim3(n, m), 256, 0, c.stream>>>(p, list, c.d_nbr.p, c.d_bbase.p, c.cfg.block_extent);
     });
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }
+
+void launch_halo(Ctx& c, double* f, const int* list, int n) { launch_halo_vf(c, &f, 1, list, n); }
 
 void launch_source_correction(Ctx& c, const double* target_tmp, double* corr, const int* list, int n,
                               double inv_dx2)
@@ -486,6 +547,39 @@ void launch_fill_zero(Ctx& c, double* p, size_t n)
     if (!n) return;
     const size_t blocks = std::min<size_t>((n / 2 + 255) / 256, 148 * 8);
     fill_zero_kernel<<<(unsigned)std::max<size_t>(blocks, 1), 256, 0, c.stream>>>(p, n);
+    c.launches += 1;
+    IBLGF_CUDA(cudaGetLastError());
+}
+
+namespace
+{
+// one CTA per (block, component)
+__global__ void masked_copy_kernel(const __grid_constant__ TpFields f, const int* __restrict__ flag, int half)
+{
+    const size_t off = (size_t)blockIdx.x * half;
+    double2* __restrict__ d = reinterpret_cast<double2*>(f.dst[blockIdx.y]) + off;
+    if (flag[blockIdx.x])
+    {
+        const double2* __restrict__ s = reinterpret_cast<const double2*>(f.src[blockIdx.y]) + off;
+#pragma unroll 4
+        for (int i = threadIdx.x; i < half; i += blockDim.x) d[i] = s[i];
+    }
+    else
+        for (int i = threadIdx.x; i < half; i += blockDim.x) d[i] = make_double2(0.0, 0.0);
+}
+}  // namespace
+
+void launch_masked_copy_vf(Ctx& c, const double* const* src, double* const* dst, int n, const int* flag)
+{
+    if (!c.n_oct || n < 1) return;
+    TpFields f{};
+    for (int k = 0; k < n; ++k)
+    {
+        f.src[k] = src[k];
+        f.dst[k] = dst[k];
+    }
+    // Nb is even, so blocks are whole 16-byte pieces
+    masked_copy_kernel<<<dim3(c.n_oct, n), 256, 0, c.stream>>>(f, flag, (int)(c.block_elems() / 2));
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }

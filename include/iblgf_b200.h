@@ -407,10 +407,11 @@ int iblgf_stats_n(iblgf_ctx* ctx, long long* out, int n);
 int iblgf_mac_variant(iblgf_ctx* ctx, int variant);
 /* Integrating-factor sweeps (neighbour-only, LGF_GE; fmm.hpp:754-770) whose
  * 1-D factor e^{-2a} I_m(2a) is below 2^-56 of its centre value for every
- * m > R, R in {4, 6, 8} (the smallest that holds), run as direct separable
- * sums over the 27 neighbour blocks instead of block FFT convolutions: the
- * same sums up to terms below FP64 rounding (default on). iblgf_ge_direct(ctx, 0) selects the transform path for all
- * of them. */
+ * m > R, R in {4, 6, 8, 12, 16} (the smallest that holds, or that reaches
+ * across the neighbours), run as direct separable sums over the 27 neighbour
+ * blocks instead of block FFT convolutions: the same sums up to terms below
+ * FP64 rounding (default on). iblgf_ge_direct(ctx, 0) selects the transform
+ * path for all of them. */
 int iblgf_ge_direct(iblgf_ctx* ctx, int enable);
 int iblgf_mac_tuning(iblgf_ctx* ctx, double* out, int max_rows, int* n_rows);
 /* Measures the device's FMA throughput (TFLOP/s, 2 flops per FMA) for

@@ -36,3 +36,21 @@ def test_solve_uneven_octree(e, precision, tol, variant):
     for _ in range(2):
         g.apply_lgf(fs, ft)
         assert rel_linf(g.download(ft), ref) < tol
+
+
+# e^{-2a} I_m(2a) falls below 2^-56 of its centre beyond m = 4, 6, 8, 12, 16 for these a
+@pytest.mark.parametrize("alpha", [4e-4, 8e-3, 4e-2, 0.25, 0.6])
+@pytest.mark.parametrize("e", [4, 10, 16])
+def test_integrating_factor_radii(e, alpha):
+    """Separable sums and block convolutions against the oracle, into another field and into the source itself."""
+    o, g = uneven(e, B.FP64)
+    src = np.random.default_rng(e).standard_normal((o.n, o.Nb, o.Nb, o.Nb))
+    ref = o.apply_if(src, alpha)
+    for direct in (True, False):
+        g.ge_direct(direct)
+        fs, ft = g.field(src), g.field()
+        g.apply_if(fs, ft, alpha)
+        assert rel_linf(g.download(ft), ref) < 1e-12
+        g.apply_if(fs, fs, alpha)
+        sel = np.asarray(o.levels) >= o.base_level  # the coarser blocks keep their values
+        assert rel_linf(g.download(fs)[sel], ref[sel]) < 1e-12
