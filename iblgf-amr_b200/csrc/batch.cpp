@@ -34,9 +34,8 @@ struct BatchState
 {
     int rmax = 0;                    // largest number of mesh levels over the problems
     std::vector<int> depth_rel;      // mesh levels per problem
-    DevBuf<int> leaves;
     // per relative level r
-    std::vector<DevBuf<int>> level_leaves, corr_all, corr_next, corr_children;
+    std::vector<DevBuf<int>> level_leaves, corr_all, corr_children;
     std::vector<TpTasks> coarsify, cc_intrp, corr_intrp;
     std::map<std::pair<int, int>, std::unique_ptr<FmmPlan>> plans;  // (r, non_leaf_as_source)
 };
@@ -143,20 +142,16 @@ BatchState& batch_state(Ctx& c)
     const int R = b->rmax;
     b->level_leaves.resize(R);
     b->corr_all.resize(R);
-    b->corr_next.resize(R);
     b->corr_children.resize(R);
     b->coarsify.resize(R);
     b->cc_intrp.resize(R);
     b->corr_intrp.resize(R);
-    std::vector<int> leaves;
-    std::vector<std::vector<int>> lleaves(R), call(R), cnext(R), cchild(R);
+    std::vector<std::vector<int>> lleaves(R), call(R), cchild(R);
     std::vector<HostTasks> hco(R), hcc(R), hci(R);
     for (int i = 0; i < np; ++i)
     {
         const Ctx& s = *c.sub[i];
         const int off = c.sub_off[i], bl = s.tree.base_level, dr = b->depth_rel[i];
-        for (int o = 0; o < s.n_oct; ++o)
-            if (s.flags[o] & 1) leaves.push_back(o + off);
         for (int r = 0; r < dr; ++r)
         {
             const int l = bl + r;
@@ -198,17 +193,14 @@ BatchState& batch_state(Ctx& c)
                 host_tasks(t, kdst, kt);
                 append_tasks(hci[r], t, off);
                 for (int o : s.level_octs[l]) call[r].push_back(o + off);
-                for (int o : s.level_octs[l + 1]) cnext[r].push_back(o + off);
                 append_off(cchild[r], ch, off);
             }
         }
     }
-    b->leaves.upload(leaves, c.stream);
     for (int r = 0; r < R; ++r)
     {
         b->level_leaves[r].upload(lleaves[r], c.stream);
         b->corr_all[r].upload(call[r], c.stream);
-        b->corr_next[r].upload(cnext[r], c.stream);
         b->corr_children[r].upload(cchild[r], c.stream);
         upload_host_tasks(c, b->coarsify[r], hco[r]);
         upload_host_tasks(c, b->cc_intrp[r], hcc[r]);
@@ -294,6 +286,7 @@ void batch_finalize(Ctx& c)
     }
     c.d_nbr.upload(nbr, c.stream);
     c.d_bbase.upload(c.bbase, c.stream);
+    upload_flags(c);
     c.f_source_tmp = field_create(c);
     c.f_target_tmp = field_create(c);
     c.f_correction_tmp = field_create(c);
@@ -312,11 +305,7 @@ void batch_apply_lgf(Ctx& c, int src, int tgt)
     double* st = c.field(c.f_source_tmp);
     double* tt = c.field(c.f_target_tmp);
     double* ct = c.field(c.f_correction_tmp);
-    const size_t bytes = c.field_elems() * sizeof(double);
-    launch_fill_zero(c, st, bytes / sizeof(double));
-    launch_fill_zero(c, tt, bytes / sizeof(double));
-    launch_fill_zero(c, ct, bytes / sizeof(double));
-    launch_axpy_blocks(c, c.field(src), st, b.leaves.p, (int)b.leaves.n, 1.0, true);
+    launch_solve_begin(c, c.field(src), st, tt, ct, c.subtract_non_leaf || !c.use_correction);
     for (int r = b.rmax - 2; r >= 0; --r) launch_tp(c, b.coarsify[r], st, st, 4, 0);
     for (int r = 0; r < b.rmax; ++r)
     {
@@ -332,8 +321,7 @@ void batch_apply_lgf(Ctx& c, int src, int tgt)
         launch_halo(c, st, b.corr_all[r].p, (int)b.corr_all[r].n);
         launch_tp(c, b.corr_intrp[r], st, ct, 2, 2);
         const double dx = dx_level / 2.0;
-        launch_source_correction(c, tt, ct, b.corr_children[r].p, (int)b.corr_children[r].n, 1.0 / (dx * dx));
-        launch_axpy_blocks(c, ct, st, b.corr_next[r].p, (int)b.corr_next[r].n, 1.0, false);
+        launch_source_correction(c, tt, ct, st, b.corr_children[r].p, (int)b.corr_children[r].n, 1.0 / (dx * dx));
     }
 }
 

@@ -174,7 +174,11 @@ constexpr int kToeplitzPart = 14;
 struct FmmPlan
 {
     int level = 0, mask_idx = 0;
-    DevBuf<int> zero_s, zero_t, copy_s, add_t;
+    // start of the sweep, block << 2 | op: source blocks zeroed (0) or, at the
+    // sweep level, taken from the source field (1), target blocks that no
+    // inverse transform assigns zeroed (2)
+    DevBuf<int> begin;
+    DevBuf<int> add_t;
     std::vector<TpTasks> antrp;  // levels level-1 .. 0
     std::vector<TpTasks> intrp;  // levels 1 .. level-1
     int n_src = 0, n_tgt = 0;
@@ -323,6 +327,11 @@ struct Ctx
 
     // device octant data
     DevBuf<int> d_bbase, d_nbr;
+    DevBuf<int> d_flags;  // per octant: bit 0 leaf, bit 1 correction, bit 2 at or above the base level
+    // correction_tmp is zero everywhere: set by the solves that clean it, reset
+    // whenever its memory is handed out
+    bool correction_zero = false;
+    bool capturing_step = false;  // ns_step records a time step (its solves run in the recorded order only)
     // leaf blocks in canonical order and the device staging of their
     // interiors (leaf-interior field transfers); rebuilt with the domain
     DevBuf<int> d_leaf_blocks;
@@ -432,7 +441,11 @@ struct Ctx
     size_t block_elems() const { return (size_t)Nb * Nb * Nb; }
     size_t field_elems() const { return (size_t)n_oct * block_elems(); }
     size_t cplx_bytes() const { return cfg.precision == IBLGF_FP32 ? 8 : 16; }
-    double* field(int id) { return fields.at(id)->d.p; }
+    double* field(int id)
+    {
+        if (id == f_correction_tmp) correction_zero = false;
+        return fields.at(id)->d.p;
+    }
 };
 
 // -------------------------------------------------------------- library
@@ -530,7 +543,6 @@ struct PoissonLists
 {
     DevBuf<int> all, leaves;
     std::vector<DevBuf<int>> level_all, level_leaves;
-    DevBuf<int> leaf;                    // per octant: 1 for leaves
     // per (level, IB2xIB or not), built on first use
     std::map<std::pair<int, bool>, std::unique_ptr<IfLevel>> if_levels;
     std::vector<TpTasks> coarsify;       // per level ls (dst parents at ls)
@@ -563,6 +575,7 @@ void ib_on_adapt(Ctx& c);
 std::vector<int> ib_octant_flags(Ctx& c);
 // octree rebuild after the host tree changed (lists, masks; no fields)
 void domain_rebuild(Ctx& c);
+void upload_flags(Ctx& c);
 // Ifherk::adapt + Domain::adapt for one process: attempts (key, level change),
 // then every field remapped to the new octants, the listed fields
 // interpolated into the children of the interpolation parents
@@ -608,11 +621,12 @@ void build_tc_tiles(const std::vector<int>& tgptr, const std::vector<int>& ttab,
 // waits for the context stream and throws IBLGF_ETIMEOUT if a kernel's
 // bounded wait ran out since the last check
 void check_status(Ctx& c);
-void launch_inverse_add(Ctx& c, const FmmPlan& p, const void* acc, double* fmm_t, double scale);
+// inverse transforms assigned to the plan's target blocks
+void launch_inverse_targets(Ctx& c, const FmmPlan& p, const void* acc, double* fmm_t, double scale);
 // prime-factor inverse (inverse.cu); false when the block size has no
 // prime-factor split (the direct inverse runs instead)
 bool inverse_pfa(Ctx& c, const void* acc, const int* d_tgt_oct, int n, double scale, double* target,
-                 bool fp32_passes);
+                 bool fp32_passes, bool assign);
 void init_pfa_constants(int device);
 // sharding (solver.cpp): the reference server's load-balanced partition and
 // this context's share of it
@@ -650,10 +664,18 @@ void launch_tp_vf(Ctx& c, const TpTasks& t, const double* const* src, double* co
                   const int (*mat_base)[3], int mode, bool fp32 = false);
 void launch_halo(Ctx& c, double* f, const int* list, int n);
 void launch_halo_vf(Ctx& c, double* const* f, int m, const int* list, int n);
-// dst = src on the blocks whose flag is set, 0 on the others, n component fields
-void launch_masked_copy_vf(Ctx& c, const double* const* src, double* const* dst, int n, const int* flag);
-void launch_source_correction(Ctx& c, const double* target_tmp, double* corr, const int* list, int n,
-                              double inv_dx2);
+// dst = src on leaf blocks, 0 on the others, n component fields
+void launch_leaf_copy_vf(Ctx& c, const double* const* src, double* const* dst, int n);
+void launch_zero_blocks_vf(Ctx& c, double* const* f, int m, const int* list, int n);
+void launch_copy_interior_vf(Ctx& c, const double* const* src, double* const* dst, int m, const int* list, int n);
+// start of an FMM sweep (FmmPlan::begin entries) and of a solve (st = leaves of
+// src, else 0; tt = ct = 0 at and above the base level, everywhere if zero)
+void launch_sweep_begin(Ctx& c, const int* entries, int n, const double* src, double* fs, double* ft);
+void launch_solve_begin(Ctx& c, const double* src, double* st, double* tt, double* ct, bool zero);
+// correction_tmp of the listed child blocks from target_tmp (and, on correction
+// blocks, its interpolated values), added into source_tmp
+void launch_source_correction(Ctx& c, const double* target_tmp, double* corr, double* source_tmp, const int* list,
+                              int n, double inv_dx2);
 void launch_op(Ctx& c, int op, const double* const* in, int n_in, double* const* out, int n_out, const int* list,
                const double* dx, int n, double scale);
 void buffer_exchange(Ctx& c, int field, int level);

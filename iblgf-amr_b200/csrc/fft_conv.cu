@@ -558,7 +558,7 @@ __global__ void __launch_bounds__(NT, MINB) bundle_mac_kernel(
 template<class RA, int NB>
 __global__ void __launch_bounds__(NB * NB, 2) inv_fused_kernel(const cx<RA>* __restrict__ ACC,
                                                                const int* __restrict__ tgt_oct, double scale,
-                                                               double* __restrict__ target)
+                                                               double* __restrict__ target, int assign)
 {
     constexpr int P = 2 * NB - 1, NP = P * NB, ZH = NB / 2, S = NB + 1;
     static_assert(NB % 2 == 0, "the block splits into two halves of output planes");
@@ -624,7 +624,7 @@ __global__ void __launch_bounds__(NB * NB, 2) inv_fused_kernel(const cx<RA>* __r
     const double y0 = yrow[0].x;
     double* out = target + (size_t)tgt_oct[t] * NB * NB * NB + ((size_t)(h * ZH + zl2) * NB + yo) * NB + xh * ZH;
 #pragma unroll
-    for (int i = 0; i < ZH; ++i) out[i] += scale * (y0 + 2.0 * sx[i]);
+    for (int i = 0; i < ZH; ++i) out[i] = assign ? scale * (y0 + 2.0 * sx[i]) : out[i] + scale * (y0 + 2.0 * sx[i]);
 }
 
 template<class R, int NB>
@@ -643,12 +643,13 @@ struct Conv
         kfn<<<n, NB * NB, smem, c.stream>>>(field, d_item_oct, W);
     }
 
-    static void launch_inverse(Ctx& c, const cx<R>* acc, const int* d_tgt_oct, int n, double scale, double* target)
+    static void launch_inverse(Ctx& c, const cx<R>* acc, const int* d_tgt_oct, int n, double scale, double* target,
+                               bool assign)
     {
         const int smem = (P * NB + NB / 2 * NP) * (int)sizeof(double2);
         auto kfn = inv_fused_kernel<R, NB>;
         IBLGF_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        kfn<<<dim3(n, 2), NB * NB, smem, c.stream>>>(acc, d_tgt_oct, scale, target);
+        kfn<<<dim3(n, 2), NB * NB, smem, c.stream>>>(acc, d_tgt_oct, scale, target, assign ? 1 : 0);
     }
 
     static void forward_field(Ctx& c, const double* field, const int* d_item_oct, int n, void* spec)
@@ -721,11 +722,12 @@ struct Conv
         }
     }
 
-    static void inverse(Ctx& c, const void* acc, const int* d_tgt_oct, int n_tgt, double scale, double* target)
+    static void inverse(Ctx& c, const void* acc, const int* d_tgt_oct, int n_tgt, double scale, double* target,
+                        bool assign)
     {
         if (!n_tgt) return;
-        if (inverse_pfa(c, acc, d_tgt_oct, n_tgt, scale, target, inverse_fp32_passes(c))) return;
-        launch_inverse(c, (const cx<R>*)acc, d_tgt_oct, n_tgt, scale, target);
+        if (inverse_pfa(c, acc, d_tgt_oct, n_tgt, scale, target, inverse_fp32_passes(c), assign)) return;
+        launch_inverse(c, (const cx<R>*)acc, d_tgt_oct, n_tgt, scale, target, assign);
         c.launches += 1;
     }
 };
@@ -902,11 +904,11 @@ void launch_mac(Ctx& c, const FmmPlan& p, const void* src_spec, void* acc)
     IBLGF_CUDA(cudaGetLastError());
 }
 
-void launch_inverse_add(Ctx& c, const FmmPlan& p, const void* acc, double* fmm_t, double scale)
+void launch_inverse_targets(Ctx& c, const FmmPlan& p, const void* acc, double* fmm_t, double scale)
 {
     dispatch(c, [&](auto cv) {
         using CV = decltype(cv);
-        CV::inverse(c, acc, p.tgt_oct.p, p.n_tgt, scale, fmm_t);
+        CV::inverse(c, acc, p.tgt_oct.p, p.n_tgt, scale, fmm_t, true);
     });
     IBLGF_CUDA(cudaGetLastError());
 }
@@ -929,7 +931,7 @@ void launch_conv_block(Ctx& c, const double* src, const double* kernel, double* 
         CV::forward_lgf(c, nullptr, kernel, nullptr, 1, gspec.p);
         CV::forward_field(c, src, d_zero.p, 1, sspec.p);
         CV::mac(c, gspec.p, sspec.p, d_ptr.p, d_zero.p, d_zero.p, 1, acc.p);
-        CV::inverse(c, acc.p, d_zero.p, 1, s, out);
+        CV::inverse(c, acc.p, d_zero.p, 1, s, out, false);
     });
     IBLGF_CUDA(cudaGetLastError());
     IBLGF_CUDA(cudaStreamSynchronize(c.stream));
@@ -1050,7 +1052,7 @@ void launch_conv_block_noalloc(Ctx& c, const double* src, const double* kernel, 
             (const cx<R>*)W, nullptr, (cx<R>*)sspec);
         mac_kernel<R><<<dim3((unsigned)((c.NC + 127) / 128), 1), 128, 0, c.stream>>>(
             (const cx<R>*)gspec, (const cx<R>*)sspec, d_ptr, d_zero, d_zero, c.NC, (cx<R>*)acc);
-        CV::launch_inverse(c, (const cx<R>*)acc, d_zero, 1, s, out);
+        CV::launch_inverse(c, (const cx<R>*)acc, d_zero, 1, s, out, false);
         c.launches += 6;
     });
     IBLGF_CUDA(cudaGetLastError());

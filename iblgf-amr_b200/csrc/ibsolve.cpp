@@ -322,12 +322,21 @@ std::vector<double> download(Ctx& c, const double* d, size_t n)
     return h;
 }
 
+// zero the finest-level blocks of three component fields: the force solve
+// reads no others
+void zero_finest(Ctx& c, const int* f)
+{
+    OpLists& ol = op_lists(c);
+    const int l = c.tree.depth - 1;
+    double* p[3] = {c.field(f[0]), c.field(f[1]), c.field(f[2])};
+    launch_zero_blocks_vf(c, p, 3, ol.list[l].p, (int)ol.list[l].n);
+}
+
 // Operator::ib_smearing of the device forces f (3 n)
 void smearing(Ctx& c, IbState& s, const double* f, const int* u, bool cleaning = true)
 {
     double* pu[3] = {c.field(u[0]), c.field(u[1]), c.field(u[2])};
-    if (cleaning)
-        for (int k = 0; k < 3; ++k) launch_fill_zero(c, pu[k], c.field_elems());
+    if (cleaning) zero_finest(c, u);
     launch_ib_smearing(c, pu, s.node_at.p, s.nptr.p, s.npt.p, s.nent.p, s.w.p, s.n_nodes, f);
 }
 
@@ -357,12 +366,16 @@ void apply_schur(Ctx& c, IbState& s, const int* src, const int* tgt)
 // projection out
 void et_h_s_e(Ctx& c, IbState& s, const double* fin, double* fout, double alpha)
 {
-    for (int k = 0; k < 3; ++k) launch_fill_zero(c, c.field(s.face_aux[k]), c.field_elems());
+    zero_finest(c, s.face_aux);
     smearing(c, s, fin, s.face_aux2);
     static const int face[3][3] = {{0, 1, 1}, {1, 0, 1}, {1, 1, 0}};  // relative positions of face components
     if (std::fabs(alpha) > 1e-14) apply_if_vf(c, 3, s.face_aux2, s.face_aux2, alpha, IBLGF_IB2xIB, face);
     apply_schur(c, s, s.face_aux2, s.face_aux);
-    for (int k = 0; k < 3; ++k) launch_axpby(c, c.field(s.face_aux2[k]), c.field(s.face_aux[k]), -1.0, 1);
+    OpLists& ol = op_lists(c);
+    const int l = c.tree.depth - 1;
+    for (int k = 0; k < 3; ++k)
+        launch_axpy_blocks(c, c.field(s.face_aux[k]), c.field(s.face_aux2[k]), ol.list[l].p, (int)ol.list[l].n, -1.0,
+                           false);
     projection(c, s, s.face_aux2, fout);
 }
 }  // namespace
@@ -612,7 +625,7 @@ void cg_solve(Ctx& c, IbState& s, const int* u, double alpha, double threshold, 
 {
     const int m = 3 * s.n;
     projection(c, s, u, s.cg_uc.p);
-    for (int k = 0; k < 3; ++k) launch_fill_zero(c, c.field(s.face_aux2[k]), c.field_elems());
+    zero_finest(c, s.face_aux2);
     et_h_s_e(c, s, s.cg_f.p, s.cg_Ap.p, alpha);
     launch_cg_init(c, s.cg_uc.p, s.cg_Ap.p, s.cg_r.p, s.cg_p.p, m, s.cg_ctl.p, max_iter);
     launch_cg_dot(c, s.cg_r.p, s.cg_r.p, nullptr, nullptr, m, s.cg_sc.p, nullptr, nullptr);

@@ -602,6 +602,9 @@ void ns_step(Ctx& c, const int* u, int p, double dt, double Re, double* T, int n
             cudaGraph_t g = nullptr;
             IBLGF_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeRelaxed));
             bool ok = true;
+            // a step's first solve cleans correction_tmp by itself, so the
+            // recorded order holds whatever ran before a replay
+            c.capturing_step = true;
             try
             {
                 st.time_step(uf, pf, false);
@@ -610,6 +613,7 @@ void ns_step(Ctx& c, const int* u, int p, double dt, double Re, double* T, int n
             {
                 ok = false;
             }
+            c.capturing_step = false;
             const cudaError_t e = cudaStreamEndCapture(c.stream, &g);
             if (!ok || e != cudaSuccess || !g || cudaGraphInstantiate(&s.graph, g, 0) != cudaSuccess)
             {
@@ -617,6 +621,7 @@ void ns_step(Ctx& c, const int* u, int p, double dt, double Re, double* T, int n
                 if (g) cudaGraphDestroy(g);
                 s.graph = nullptr;
                 s.graph_failed = true;
+                c.correction_zero = false;
                 c.launches = l0;
                 st.time_step(uf, pf, false);  // nothing of the failed capture ran
             }

@@ -13,7 +13,7 @@
 //      outputs (a partial sum)
 // then each CTA adds its half of the planes, own partial plus the peer's
 // read through distributed shared memory (always rank 0's partial first, so
-// the result does not depend on timing), into the target.
+// the result does not depend on timing), into the target, or assigns it.
 // The z and y passes use the prime-factor (Good-Thomas) algorithm for
 // P = N1 N2 with coprime N1, N2 (35 = 5 x 7, 15 = 3 x 5): with input
 // n = (N2 n1 + N1 n2) mod P and output k, e^{2 pi i n k / P} =
@@ -152,7 +152,7 @@ struct InvSmem
 template<class RZ, class RA, int NB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NB* NB)
     inv_pfa_kernel(const cx<RA>* __restrict__ ACC, const int* __restrict__ tgt_oct, double scale,
-                   double* __restrict__ target)
+                   double* __restrict__ target, int assign)
 {
     constexpr int P = 2 * NB - 1, KH = NB / 2, NP = P * NB;
     using SM = InvSmem<RZ, NB>;
@@ -218,19 +218,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NB* NB)
         const double* p1 = h == 1 ? part : cluster.map_shared_rank(part, 1);
         double* out = target + (size_t)tgt_oct[t] * NB * NB * NB;
         const int base = h * (NB / 2) * NB * NB;
-        for (int i = threadIdx.x; i < (NB / 2) * NB * NB; i += blockDim.x)
-            out[base + i] += scale * (p0[base + i] + p1[base + i]);
+        if (assign)
+            for (int i = threadIdx.x; i < (NB / 2) * NB * NB; i += blockDim.x)
+                out[base + i] = scale * (p0[base + i] + p1[base + i]);
+        else
+            for (int i = threadIdx.x; i < (NB / 2) * NB * NB; i += blockDim.x)
+                out[base + i] += scale * (p0[base + i] + p1[base + i]);
     }
     cluster.sync();  // the peer has read this CTA's partials
 }
 
 template<class RZ, class RA, int NB>
-void launch_inv_pfa(Ctx& c, const void* acc, const int* d_tgt_oct, int n, double scale, double* target)
+void launch_inv_pfa(Ctx& c, const void* acc, const int* d_tgt_oct, int n, double scale, double* target, bool assign)
 {
     using SM = InvSmem<RZ, NB>;
     auto kfn = inv_pfa_kernel<RZ, RA, NB>;
     IBLGF_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM::total));
-    kfn<<<2 * n, NB * NB, SM::total, c.stream>>>((const cx<RA>*)acc, d_tgt_oct, scale, target);
+    kfn<<<2 * n, NB * NB, SM::total, c.stream>>>((const cx<RA>*)acc, d_tgt_oct, scale, target, assign ? 1 : 0);
     c.launches += 1;
 }
 }  // namespace
@@ -264,21 +268,21 @@ void init_pfa_constants(int device)
 // true if the prime-factor inverse handles this block size; the FP32 path
 // runs its z and y passes in FP32 when fp32_passes is set
 bool inverse_pfa(Ctx& c, const void* acc, const int* d_tgt_oct, int n, double scale, double* target,
-                 bool fp32_passes)
+                 bool fp32_passes, bool assign)
 {
     if (!n) return true;
     const bool f32 = c.cfg.precision == IBLGF_FP32;
     switch (c.Nb)
     {
         case 18:
-            if (!f32) launch_inv_pfa<double, double, 18>(c, acc, d_tgt_oct, n, scale, target);
-            else if (fp32_passes) launch_inv_pfa<float, float, 18>(c, acc, d_tgt_oct, n, scale, target);
-            else launch_inv_pfa<double, float, 18>(c, acc, d_tgt_oct, n, scale, target);
+            if (!f32) launch_inv_pfa<double, double, 18>(c, acc, d_tgt_oct, n, scale, target, assign);
+            else if (fp32_passes) launch_inv_pfa<float, float, 18>(c, acc, d_tgt_oct, n, scale, target, assign);
+            else launch_inv_pfa<double, float, 18>(c, acc, d_tgt_oct, n, scale, target, assign);
             return true;
         case 8:
-            if (!f32) launch_inv_pfa<double, double, 8>(c, acc, d_tgt_oct, n, scale, target);
-            else if (fp32_passes) launch_inv_pfa<float, float, 8>(c, acc, d_tgt_oct, n, scale, target);
-            else launch_inv_pfa<double, float, 8>(c, acc, d_tgt_oct, n, scale, target);
+            if (!f32) launch_inv_pfa<double, double, 8>(c, acc, d_tgt_oct, n, scale, target, assign);
+            else if (fp32_passes) launch_inv_pfa<float, float, 8>(c, acc, d_tgt_oct, n, scale, target, assign);
+            else launch_inv_pfa<double, float, 8>(c, acc, d_tgt_oct, n, scale, target, assign);
             return true;
         default: return false;
     }

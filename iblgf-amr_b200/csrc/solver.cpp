@@ -474,6 +474,20 @@ void domain_finalize(Ctx& c)
     c.f_fmm_t = field_create(c);
 }
 
+// the octants' flags on the device; bit 2: no parent level among the mesh levels
+void upload_flags(Ctx& c)
+{
+    std::vector<int> f(c.flags);
+    if (c.batch)
+        for (size_t i = 0; i < c.sub.size(); ++i)
+            for (int o = 0; o < c.sub[i]->n_oct; ++o)
+                f[c.sub_off[i] + o] |= c.sub[i]->levels[o] <= c.sub[i]->tree.base_level ? 4 : 0;
+    else
+        for (int o = 0; o < c.n_oct; ++o) f[o] |= c.levels[o] <= c.tree.base_level ? 4 : 0;
+    c.d_flags.upload(f, c.stream);
+    IBLGF_CUDA(cudaStreamSynchronize(c.stream));  // the host array goes out of scope
+}
+
 void domain_rebuild(Ctx& c)
 {
     HostTree& t = c.tree;
@@ -526,6 +540,7 @@ void domain_rebuild(Ctx& c)
     IBLGF_CUDA(cudaMemcpyAsync(c.infl.data(), d_infl.p, c.infl.size() * 4, cudaMemcpyDeviceToHost, c.stream));
     IBLGF_CUDA(cudaMemcpyAsync(c.n_infl.data(), d_ninfl.p, n * 4, cudaMemcpyDeviceToHost, c.stream));
     c.d_bbase.upload(c.bbase, c.stream);
+    upload_flags(c);
     IBLGF_CUDA(cudaStreamSynchronize(c.stream));
     build_masks(c);
     c.finalized = true;
@@ -1005,9 +1020,17 @@ std::unique_ptr<FmmPlan> upload_plan(Ctx& c, const HostPlan& h)
     FmmPlan& p = *plan;
     p.level = h.level;
     p.mask_idx = h.mask_idx;
-    p.zero_s.upload(h.zs, c.stream);
-    p.zero_t.upload(h.zt, c.stream);
-    p.copy_s.upload(h.cs, c.stream);
+    {
+        std::vector<char> from_src(c.n_oct, 0), assigned(c.n_oct, 0);
+        for (int o : h.cs) from_src[o] = 1;
+        for (int o : h.tgt_list) assigned[o] = 1;
+        std::vector<int> begin;
+        for (int o : h.zs) begin.push_back(o << 2 | (from_src[o] ? 1 : 0));
+        for (int o : h.zt)
+            if (!assigned[o] || h.ge >= 0) begin.push_back(o << 2 | 2);
+        p.begin.upload(begin, c.stream);
+        IBLGF_CUDA(cudaStreamSynchronize(c.stream));  // the host array goes out of scope
+    }
     p.add_t.upload(h.at, c.stream);
     for (auto& t : h.antrp)
     {
@@ -1328,9 +1351,7 @@ void run_sweep(Ctx& c, FmmPlan& p, int src, int tgt, double dx_level, double add
         tm.mark(4);
         return;
     }
-    launch_zero_blocks(c, fs, p.zero_s.p, (int)p.zero_s.n);
-    launch_zero_blocks(c, ft, p.zero_t.p, (int)p.zero_t.n);
-    launch_copy_interior(c, c.field(src), fs, p.copy_s.p, (int)p.copy_s.n);
+    launch_sweep_begin(c, p.begin.p, (int)p.begin.n, c.field(src), fs, ft);
     // the FMM's Lagrange anterpolation of the sources (fmm_nli.hpp) runs its
     // passes in FP32 on the FP32 path (the coarse sources feed FP32
     // transforms); the interpolation of the targets stays FP64
@@ -1359,7 +1380,7 @@ void run_sweep(Ctx& c, FmmPlan& p, int src, int tgt, double dx_level, double add
     {
         // compute_influence_field (fmm.hpp:1021-1026): dx^2 for LGF_GL, 1 for LGF_GE
         const double scale = (ge >= 0 ? 1.0 : dx_level * dx_level) / ((double)c.P * c.P * c.P);
-        launch_inverse_add(c, p, c.d_acc.p, ft, scale);
+        launch_inverse_targets(c, p, c.d_acc.p, ft, scale);
     }
     for (auto& t : p.intrp) launch_tp(c, t, ft, ft, 0, 1);
     if (!c.owner.empty() && p.add_t.n)
@@ -1388,9 +1409,6 @@ PoissonLists& poisson_lists(Ctx& c)
         all.push_back(i);
         if (c.flags[i] & 1) leaves.push_back(i);
     }
-    std::vector<int> leaf(c.n_oct);
-    for (int i = 0; i < c.n_oct; ++i) leaf[i] = c.flags[i] & 1;
-    pl->leaf.upload(leaf, c.stream);
     pl->all.upload(all, c.stream);
     pl->leaves.upload(leaves, c.stream);
     const int L = kMaxLevel + 1;
@@ -1710,8 +1728,7 @@ void apply_if_vf(Ctx& c, int n, const int* src, const int* tgt, double alpha_bas
         // non-leaf-as-source sweep with the IB2xIB mask, level copied out
         const int l = depth - 1;
         const int ge = ge_table(c, alpha_base * std::pow(4.0, l - bl));
-        for (int k = 0; k < n; ++k)
-            launch_copy_interior(c, ps[k], pst[k], pl.level_all[l].p, (int)pl.level_all[l].n);
+        launch_copy_interior_vf(c, ps, pst, n, pl.level_all[l].p, (int)pl.level_all[l].n);
         if (if_level_direct(c, pl, l, true, n, st, tgt, ge)) return;
         for (int k = 0; k < n; ++k)
         {
@@ -1721,7 +1738,7 @@ void apply_if_vf(Ctx& c, int n, const int* src, const int* tgt, double alpha_bas
         }
         return;
     }
-    launch_masked_copy_vf(c, ps, pst, n, pl.leaf.p);
+    launch_leaf_copy_vf(c, ps, pst, n);
     for (int ls = depth - 2; ls >= bl; --ls) launch_tp_vf(c, pl.coarsify[ls], cst, pst, n, coarse_m, 0);
     // intrp_to_correction_buffer (poisson.hpp:1015-1069)
     for (int l = depth - 2; l >= bl; --l)
@@ -1764,17 +1781,27 @@ void poisson_apply_lgf(Ctx& c, int src, int tgt, int fmm_type)
     PoissonLists& pl = poisson_lists(c);
     double* st = c.field(c.f_source_tmp);
     double* tt = c.field(c.f_target_tmp);
-    double* ct = c.field(c.f_correction_tmp);
-    const size_t bytes = c.field_elems() * sizeof(double);
-    launch_fill_zero(c, st, bytes / sizeof(double));
-    launch_fill_zero(c, tt, bytes / sizeof(double));
-    launch_fill_zero(c, ct, bytes / sizeof(double));
+    double* ct = c.fields[c.f_correction_tmp]->d.p;
+    const size_t elems = c.field_elems();
+    // the solves without a source correction leave correction_tmp zero; one
+    // recorded in a graph by the caller may be replayed after any other solve,
+    // so it cleans the field itself
+    if (fmm_type != IBLGF_AMR2AMR)
+    {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        if (!c.capturing_step) IBLGF_CUDA(cudaStreamIsCapturing(c.stream, &cs));
+        const bool caller = cs != cudaStreamCaptureStatusNone;
+        if (!c.correction_zero || caller) launch_fill_zero(c, ct, elems);
+        c.correction_zero = !caller;
+    }
     if (fmm_type == IBLGF_IB2AMR)
     {
         // finest-level interior copy, coarsified (cell mesh), one sweep per
         // level with the IB2AMR mask, leaves assigned, no source correction
         // (poisson.hpp:617-618, 632-634, 702-745)
         const int bl = c.tree.base_level, depth = c.tree.depth;
+        launch_fill_zero(c, st, elems);
+        launch_fill_zero(c, tt, elems);
         launch_copy_interior(c, c.field(src), st, pl.level_all[depth - 1].p, (int)pl.level_all[depth - 1].n);
         for (int ls = depth - 2; ls >= bl; --ls) launch_tp(c, pl.coarsify[ls], st, st, 4, 0);
         for (int l = bl; l < depth && !c.subtract_non_leaf; ++l)
@@ -1786,31 +1813,35 @@ void poisson_apply_lgf(Ctx& c, int src, int tgt, int fmm_type)
     }
     if (fmm_type == IBLGF_xIB2IB || fmm_type == IBLGF_IB2xIB)
     {
-        // finest level only: copy_level (interior), one sweep with the IB
-        // mask, leaves of that level assigned (poisson.hpp:615-616, 702-745)
+        // finest level only: one sweep with the IB mask from the source's
+        // interiors, leaves of that level assigned (poisson.hpp:615-616, 702-745)
         const int l = c.tree.depth - 1;
-        launch_copy_interior(c, c.field(src), st, pl.level_all[l].p, (int)pl.level_all[l].n);
         if (!c.subtract_non_leaf)
         {
-            fmm_apply(c, c.f_source_tmp, c.f_target_tmp, l, false, 1.0, fmm_type);
+            launch_zero_blocks(c, tt, pl.level_all[l].p, (int)pl.level_all[l].n);
+            fmm_apply(c, src, c.f_target_tmp, l, false, 1.0, fmm_type);
             launch_axpy_blocks(c, tt, c.field(tgt), pl.level_leaves[l].p, (int)pl.level_leaves[l].n, 1.0, true);
         }
         return;
     }
     if (fmm_type == IBLGF_STREAM)
     {
-        // base level only: copy_level (interior), one sweep with the stream
-        // mask, leaves copied out (poisson.hpp:612-614, 749-781)
+        // base level only: one sweep with the stream mask from the source's
+        // interiors, leaves copied out (poisson.hpp:612-614, 749-781)
         const int bl = c.tree.base_level;
-        launch_copy_interior(c, c.field(src), st, pl.level_all[bl].p, (int)pl.level_all[bl].n);
         if (!c.subtract_non_leaf)
         {
-            fmm_apply(c, c.f_source_tmp, c.f_target_tmp, bl, false, 1.0, IBLGF_STREAM);
+            launch_zero_blocks(c, tt, pl.level_all[bl].p, (int)pl.level_all[bl].n);
+            fmm_apply(c, src, c.f_target_tmp, bl, false, 1.0, IBLGF_STREAM);
             launch_axpy_blocks(c, tt, c.field(tgt), pl.level_leaves[bl].p, (int)pl.level_leaves[bl].n, 1.0, true);
         }
         return;
     }
-    launch_axpy_blocks(c, c.field(src), st, pl.leaves.p, (int)pl.leaves.n, 1.0, true);
+    // below the base level target_tmp is assigned by the interpolation and
+    // correction_tmp by the correction, so only the blocks at and above it are
+    // zeroed, unless a switch leaves these out
+    launch_solve_begin(c, c.field(src), st, tt, ct, c.subtract_non_leaf || !c.use_correction);
+    c.correction_zero = false;
     const int bl = c.tree.base_level, depth = c.tree.depth;
     for (int ls = depth - 2; ls >= bl; --ls) launch_tp(c, pl.coarsify[ls], st, st, 4, 0);
     for (int l = bl; l < depth; ++l)
@@ -1826,8 +1857,7 @@ void poisson_apply_lgf(Ctx& c, int src, int tgt, int fmm_type)
         launch_halo(c, st, pl.level_all[l].p, (int)pl.level_all[l].n);
         launch_tp(c, pl.corr_intrp[l], st, ct, 2, 2);
         const double dx = c.cfg.dx_base / std::pow(2.0, l - bl) / 2.0;
-        launch_source_correction(c, tt, ct, pl.children[l].p, (int)pl.children[l].n, 1.0 / (dx * dx));
-        launch_axpy_blocks(c, ct, st, pl.level_all[l + 1].p, (int)pl.level_all[l + 1].n, 1.0, false);
+        launch_source_correction(c, tt, ct, st, pl.children[l].p, (int)pl.children[l].n, 1.0 / (dx * dx));
     }
 }
 

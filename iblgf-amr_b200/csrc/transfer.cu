@@ -292,57 +292,176 @@ __global__ void halo_kernel(const __grid_constant__ TpFields fs, const int* __re
     }
 }
 
+// Block copies and sums are split over blockIdx.y in pieces of kPiece 16-byte
+// pairs, kPairs per thread with all loads in flight before the first store: a
+// block per CTA with one load after another took 15 us for 64 blocks of 18^3
+// (uniform 64^3 solve), 3 us as a piece per CTA.
+constexpr int kPairs = 4;
+constexpr int kPiece = 256 * kPairs;
+constexpr int pieces(int n3) { return (n3 / 2 + kPiece - 1) / kPiece; }
+
+// add_source_correction on the listed (child) blocks: ct = c0 - laplace(tt) r
+// on the interior, c0 = ct where the block is a correction block (flag bit 1:
+// interpolated from its parent), 0 elsewhere; then st += ct
 template<int NB>
-__global__ void correction_kernel(const double* __restrict__ tt, double* __restrict__ corr,
-                                  const int* __restrict__ list, double r)
+__global__ void __launch_bounds__(256) correction_kernel(const double* __restrict__ tt, double* __restrict__ corr,
+                                                         double* __restrict__ st, const int* __restrict__ list,
+                                                         const int* __restrict__ flags, double r)
 {
     constexpr int N3 = NB * NB * NB;
     const int o = list[blockIdx.x];
-    const double* t = tt + (size_t)o * N3;
-    double* c = corr + (size_t)o * N3;
-    for (int i = threadIdx.x; i < N3; i += blockDim.x)
+    const bool have = flags[o] & 2;
+    const double* __restrict__ t = tt + (size_t)o * N3;
+    double* __restrict__ c = corr + (size_t)o * N3;
+    double* __restrict__ s = st + (size_t)o * N3;
+#pragma unroll
+    for (int k = 0; k < 2 * kPairs; ++k)
     {
+        const int i = blockIdx.y * (2 * kPiece) + 256 * k + threadIdx.x;
+        if (i >= N3) break;
         const int x = i % NB, y = (i / NB) % NB, z = i / (NB * NB);
-        if (x == 0 || y == 0 || z == 0 || x == NB - 1 || y == NB - 1 || z == NB - 1) continue;
-        double v = c[i];
-        v += 6.0 * t[i] * r;
-        v -= t[i - NB * NB] * r;
-        v -= t[i + NB * NB] * r;
-        v -= t[i - NB] * r;
-        v -= t[i + NB] * r;
-        v -= t[i + 1] * r;
-        v -= t[i - 1] * r;
+        const bool in = x > 0 && y > 0 && z > 0 && x < NB - 1 && y < NB - 1 && z < NB - 1;
+        double v = have ? c[i] : 0.0;
+        if (in)
+        {
+            v += 6.0 * t[i] * r;
+            v -= t[i - NB * NB] * r;
+            v -= t[i + NB * NB] * r;
+            v -= t[i - NB] * r;
+            v -= t[i + NB] * r;
+            v -= t[i + 1] * r;
+            v -= t[i - 1] * r;
+        }
         c[i] = v;
+        if (in || have) s[i] += v;
     }
 }
 
-__global__ void zero_kernel(double* __restrict__ f, const int* __restrict__ list, int n3)
+// f.dst[component] = 0 on the listed blocks
+__global__ void __launch_bounds__(256) zero_kernel(const __grid_constant__ TpFields f, const int* __restrict__ list,
+                                                   int half)
 {
-    double* b = f + (size_t)list[blockIdx.x] * n3;
-    for (int i = threadIdx.x; i < n3; i += blockDim.x) b[i] = 0.0;
-}
-
-__global__ void copy_interior_kernel(const double* __restrict__ s, double* __restrict__ d,
-                                     const int* __restrict__ list, int NB)
-{
-    const int n3 = NB * NB * NB;
-    const size_t off = (size_t)list[blockIdx.x] * n3;
-    for (int i = threadIdx.x; i < n3; i += blockDim.x)
+    double2* b = reinterpret_cast<double2*>(f.dst[blockIdx.z]) + (size_t)list[blockIdx.x] * half;
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k)
     {
-        const int x = i % NB, y = (i / NB) % NB, z = i / (NB * NB);
-        if (x == 0 || y == 0 || z == 0 || x == NB - 1 || y == NB - 1 || z == NB - 1) continue;
-        d[off + i] = s[off + i];
+        const int i = blockIdx.y * kPiece + 256 * k + threadIdx.x;
+        if (i < half) b[i] = make_double2(0.0, 0.0);
     }
 }
 
-__global__ void axpy_kernel(const double* __restrict__ s, double* __restrict__ d, const int* __restrict__ list,
-                            int n3, double a, int assign)
+// 1 if node i of a block is in its interior
+template<int NB>
+__device__ __forceinline__ bool interior(int i)
 {
-    const size_t off = (size_t)list[blockIdx.x] * n3;
-    for (int i = threadIdx.x; i < n3; i += blockDim.x)
+    const int x = i % NB, y = (i / NB) % NB, z = i / (NB * NB);
+    return x > 0 && y > 0 && z > 0 && x < NB - 1 && y < NB - 1 && z < NB - 1;
+}
+
+// the interiors of the listed blocks of component blockIdx.z
+template<int NB>
+__global__ void __launch_bounds__(256) copy_interior_kernel(const __grid_constant__ TpFields f,
+                                                            const int* __restrict__ list)
+{
+    constexpr int N3 = NB * NB * NB;
+    const size_t off = (size_t)list[blockIdx.x] * N3;
+    const double* __restrict__ s = f.src[blockIdx.z] + off;
+    double* __restrict__ d = f.dst[blockIdx.z] + off;
+    double v[2 * kPairs];
+#pragma unroll
+    for (int k = 0; k < 2 * kPairs; ++k)
     {
-        if (assign) d[off + i] = a * s[off + i];
-        else d[off + i] += s[off + i] * a;
+        const int i = blockIdx.y * (2 * kPiece) + 256 * k + threadIdx.x;
+        v[k] = i < N3 ? s[i] : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < 2 * kPairs; ++k)
+    {
+        const int i = blockIdx.y * (2 * kPiece) + 256 * k + threadIdx.x;
+        if (i < N3 && interior<NB>(i)) d[i] = v[k];
+    }
+}
+
+// start of a sweep: entry = block << 2 | op; op 0: fs = 0, 1: fs = interior of
+// src and 0 around it, 2: ft = 0
+template<int NB>
+__global__ void __launch_bounds__(256) sweep_begin_kernel(const int* __restrict__ entries,
+                                                          const double* __restrict__ src, double* __restrict__ fs,
+                                                          double* __restrict__ ft)
+{
+    constexpr int N3 = NB * NB * NB;
+    const int e = entries[blockIdx.x], op = e & 3;
+    const size_t off = (size_t)(e >> 2) * (N3 / 2);
+    double2* __restrict__ d = reinterpret_cast<double2*>(op == 2 ? ft : fs) + off;
+    double2 v[kPairs];
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k)
+    {
+        const int i = blockIdx.y * kPiece + 256 * k + threadIdx.x;
+        v[k] = make_double2(0.0, 0.0);
+        if (op == 1 && i < N3 / 2)
+        {
+            v[k] = reinterpret_cast<const double2*>(src)[off + i];
+            if (!interior<NB>(2 * i)) v[k].x = 0.0;
+            if (!interior<NB>(2 * i + 1)) v[k].y = 0.0;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k)
+    {
+        const int i = blockIdx.y * kPiece + 256 * k + threadIdx.x;
+        if (i < N3 / 2) d[i] = v[k];
+    }
+}
+
+__global__ void __launch_bounds__(256) axpy_kernel(const double2* __restrict__ s, double2* __restrict__ d,
+                                                   const int* __restrict__ list, int half, double a, int assign)
+{
+    const size_t off = (size_t)list[blockIdx.x] * half;
+    double2 v[kPairs], w[kPairs];
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k)
+    {
+        const int i = blockIdx.y * kPiece + 256 * k + threadIdx.x;
+        if (i < half) v[k] = s[off + i];
+        if (i < half && !assign) w[k] = d[off + i];
+    }
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k)
+    {
+        const int i = blockIdx.y * kPiece + 256 * k + threadIdx.x;
+        if (i >= half) break;
+        if (assign) d[off + i] = make_double2(a * v[k].x, a * v[k].y);
+        else d[off + i] = make_double2(w[k].x + v[k].x * a, w[k].y + v[k].y * a);
+    }
+}
+
+// start of a solve, one block per blockIdx.x: st = src on leaves (flag bit 0), 0
+// elsewhere, and tt = ct = 0 where zero is set or the block's bit 2 is
+__global__ void __launch_bounds__(256) solve_begin_kernel(const __grid_constant__ TpFields f,
+                                                          const int* __restrict__ flags, int half, int zero)
+{
+    const int fl = flags[blockIdx.x];
+    const size_t off = (size_t)blockIdx.x * half;
+    const double2* __restrict__ src = reinterpret_cast<const double2*>(f.src[0]) + off;
+    double2* __restrict__ st = reinterpret_cast<double2*>(f.dst[0]) + off;
+    double2* __restrict__ tt = reinterpret_cast<double2*>(f.dst[1]) + off;
+    double2* __restrict__ ct = reinterpret_cast<double2*>(f.dst[2]) + off;
+    double2 v[kPairs];
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k)
+    {
+        const int i = blockIdx.y * kPiece + 256 * k + threadIdx.x;
+        v[k] = (fl & 1) && i < half ? src[i] : make_double2(0.0, 0.0);
+    }
+    const bool z = zero || (fl & 4);
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k)
+    {
+        const int i = blockIdx.y * kPiece + 256 * k + threadIdx.x;
+        if (i >= half) break;
+        st[i] = v[k];
+        if (z) tt[i] = ct[i] = make_double2(0.0, 0.0);
     }
 }
 
@@ -480,14 +599,40 @@ void launch_halo_vf(Ctx& c, double* const* f, int m, const int* list, int n)
 
 void launch_halo(Ctx& c, double* f, const int* list, int n) { launch_halo_vf(c, &f, 1, list, n); }
 
-void launch_source_correction(Ctx& c, const double* target_tmp, double* corr, const int* list, int n,
-                              double inv_dx2)
+void launch_source_correction(Ctx& c, const double* target_tmp, double* corr, double* source_tmp, const int* list,
+                              int n, double inv_dx2)
 {
     if (!n) return;
     nb_dispatch(c.Nb, [&](auto nbc) {
         constexpr int NB = decltype(nbc)::value;
-        correction_kernel<NB><<<n, 256, 0, c.stream>>>(target_tmp, corr, list, inv_dx2);
+        correction_kernel<NB><<<dim3(n, pieces(NB * NB * NB)), 256, 0, c.stream>>>(target_tmp, corr, source_tmp, list,
+                                                                                  c.d_flags.p, inv_dx2);
     });
+    c.launches += 1;
+    IBLGF_CUDA(cudaGetLastError());
+}
+
+void launch_sweep_begin(Ctx& c, const int* entries, int n, const double* src, double* fs, double* ft)
+{
+    if (!n) return;
+    nb_dispatch(c.Nb, [&](auto nbc) {
+        constexpr int NB = decltype(nbc)::value;
+        sweep_begin_kernel<NB><<<dim3(n, pieces(NB * NB * NB)), 256, 0, c.stream>>>(entries, src, fs, ft);
+    });
+    c.launches += 1;
+    IBLGF_CUDA(cudaGetLastError());
+}
+
+void launch_solve_begin(Ctx& c, const double* src, double* st, double* tt, double* ct, bool zero)
+{
+    if (!c.n_oct) return;
+    TpFields f{};
+    f.src[0] = src;
+    f.dst[0] = st;
+    f.dst[1] = tt;
+    f.dst[2] = ct;
+    const int half = (int)(c.block_elems() / 2);  // Nb is even
+    solve_begin_kernel<<<dim3(c.n_oct, pieces(2 * half)), 256, 0, c.stream>>>(f, c.d_flags.p, half, zero ? 1 : 0);
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }
@@ -553,44 +698,61 @@ void launch_fill_zero(Ctx& c, double* p, size_t n)
 
 namespace
 {
-// one CTA per (block, component)
-__global__ void masked_copy_kernel(const __grid_constant__ TpFields f, const int* __restrict__ flag, int half)
+// component blockIdx.z of one block
+__global__ void __launch_bounds__(256) masked_copy_kernel(const __grid_constant__ TpFields f,
+                                                          const int* __restrict__ flags, int half)
 {
     const size_t off = (size_t)blockIdx.x * half;
-    double2* __restrict__ d = reinterpret_cast<double2*>(f.dst[blockIdx.y]) + off;
-    if (flag[blockIdx.x])
+    const double2* __restrict__ s = reinterpret_cast<const double2*>(f.src[blockIdx.z]) + off;
+    double2* __restrict__ d = reinterpret_cast<double2*>(f.dst[blockIdx.z]) + off;
+    const bool leaf = flags[blockIdx.x] & 1;
+    double2 v[kPairs];
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k)
     {
-        const double2* __restrict__ s = reinterpret_cast<const double2*>(f.src[blockIdx.y]) + off;
-#pragma unroll 4
-        for (int i = threadIdx.x; i < half; i += blockDim.x) d[i] = s[i];
+        const int i = blockIdx.y * kPiece + 256 * k + threadIdx.x;
+        v[k] = leaf && i < half ? s[i] : make_double2(0.0, 0.0);
     }
-    else
-        for (int i = threadIdx.x; i < half; i += blockDim.x) d[i] = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int k = 0; k < kPairs; ++k)
+    {
+        const int i = blockIdx.y * kPiece + 256 * k + threadIdx.x;
+        if (i < half) d[i] = v[k];
+    }
 }
-}  // namespace
 
-void launch_masked_copy_vf(Ctx& c, const double* const* src, double* const* dst, int n, const int* flag)
+TpFields tp_fields(const double* const* src, double* const* dst, int n)
 {
-    if (!c.n_oct || n < 1) return;
     TpFields f{};
     for (int k = 0; k < n; ++k)
     {
-        f.src[k] = src[k];
+        f.src[k] = src ? src[k] : nullptr;
         f.dst[k] = dst[k];
     }
-    // Nb is even, so blocks are whole 16-byte pieces
-    masked_copy_kernel<<<dim3(c.n_oct, n), 256, 0, c.stream>>>(f, flag, (int)(c.block_elems() / 2));
+    return f;
+}
+}  // namespace
+
+void launch_leaf_copy_vf(Ctx& c, const double* const* src, double* const* dst, int n)
+{
+    if (!c.n_oct || n < 1) return;
+    const int half = (int)(c.block_elems() / 2);  // Nb is even, so blocks are whole 16-byte pieces
+    masked_copy_kernel<<<dim3(c.n_oct, pieces(2 * half), n), 256, 0, c.stream>>>(tp_fields(src, dst, n), c.d_flags.p,
+                                                                                 half);
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }
 
-void launch_zero_blocks(Ctx& c, double* f, const int* list, int n)
+void launch_zero_blocks_vf(Ctx& c, double* const* f, int m, const int* list, int n)
 {
-    if (!n) return;
-    zero_kernel<<<n, 256, 0, c.stream>>>(f, list, (int)c.block_elems());
+    if (!n || m < 1) return;
+    const int half = (int)(c.block_elems() / 2);
+    zero_kernel<<<dim3(n, pieces(2 * half), m), 256, 0, c.stream>>>(tp_fields(nullptr, f, m), list, half);
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }
+
+void launch_zero_blocks(Ctx& c, double* f, const int* list, int n) { launch_zero_blocks_vf(c, &f, 1, list, n); }
 
 // one CTA per leaf; host order: leaf i's interior e^3 values, x fastest
 __global__ void leaves_scatter_kernel(const double* __restrict__ stage, double* __restrict__ f,
@@ -789,18 +951,29 @@ void copy_stream_release(Ctx& c)
     c.ev_gathered = c.ev_copied = c.ev_in_copied = c.ev_scattered = nullptr;
 }
 
-void launch_copy_interior(Ctx& c, const double* src, double* dst, const int* list, int n)
+void launch_copy_interior_vf(Ctx& c, const double* const* src, double* const* dst, int m, const int* list, int n)
 {
-    if (!n) return;
-    copy_interior_kernel<<<n, 256, 0, c.stream>>>(src, dst, list, c.Nb);
+    if (!n || m < 1) return;
+    nb_dispatch(c.Nb, [&](auto nbc) {
+        constexpr int NB = decltype(nbc)::value;
+        copy_interior_kernel<NB><<<dim3(n, pieces(NB * NB * NB), m), 256, 0, c.stream>>>(tp_fields(src, dst, m), list);
+    });
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
+}
+
+void launch_copy_interior(Ctx& c, const double* src, double* dst, const int* list, int n)
+{
+    launch_copy_interior_vf(c, &src, &dst, 1, list, n);
 }
 
 void launch_axpy_blocks(Ctx& c, const double* src, double* dst, const int* list, int n, double a, bool assign)
 {
     if (!n) return;
-    axpy_kernel<<<n, 256, 0, c.stream>>>(src, dst, list, (int)c.block_elems(), a, assign ? 1 : 0);
+    const int half = (int)(c.block_elems() / 2);
+    axpy_kernel<<<dim3(n, pieces(2 * half)), 256, 0, c.stream>>>(reinterpret_cast<const double2*>(src),
+                                                                 reinterpret_cast<double2*>(dst), list, half, a,
+                                                                 assign ? 1 : 0);
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }
