@@ -368,6 +368,7 @@ struct Ctx
     int spec_cap = 0, spec_used = 0;
     DevBuf<char> d_spec;
 
+    DevBuf<char> conv_work;  // single-block convolution, on first use
     // per-sweep work buffers (sized on demand)
     DevBuf<char> d_src_spec, d_acc, d_w;
 

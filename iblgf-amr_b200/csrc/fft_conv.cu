@@ -38,8 +38,6 @@ namespace iblgf_b200
 {
 namespace
 {
-enum InMode { kFromLgf = 1, kFromDense = 2 };
-
 template<class R>
 __device__ __forceinline__ void load_tw(cx<R>* s_tw, const R* tw, int P)
 {
@@ -161,57 +159,12 @@ __global__ void __launch_bounds__(NB * NB) fwd_xy_rows_kernel(const double* __re
     }
 }
 
-// fwd_xy: x and y transforms of one z plane of one block.
-//   kFromLgf:   G((b + i) * 2^ld), desc[4*item] = {ld, bx, by, bz}  (NIN = P)
-//   kFromDense: dense[item * P^3]                                  (NIN = P)
-// W: [item][z < NIN][ky < P][kx < NB]
-template<class R, int NB, int NIN, int MODE>
-__global__ void __launch_bounds__(256) fwd_xy_kernel(const double* __restrict__ field,
-                                                     const int* __restrict__ item_oct,
-                                                     const int* __restrict__ desc,
-                                                     const double* __restrict__ table,
-                                                     const R* __restrict__ tw, cx<R>* __restrict__ W,
-                                                     const double* __restrict__ ge, int ge_stride)
+// x and y transforms of one staged z plane s_in[y][x] (NIN rows of NIN) into
+// out[ky][kx]
+template<class R, int NB, int NIN>
+__device__ __forceinline__ void plane_xy(const cx<R>* s_tw, const R* s_in, cx<R>* s_x1, cx<R>* __restrict__ out)
 {
     constexpr int P = 2 * NB - 1;
-    __shared__ cx<R> s_tw[P];
-    __shared__ R s_in[NIN * NIN];
-    __shared__ cx<R> s_x1[NIN * NB];
-    const int item = blockIdx.x;
-    const int z = blockIdx.y;
-    load_tw<R>(s_tw, tw, P);
-    if (MODE == kFromLgf)
-    {
-        // desc[0] >= 0: LGF_GL at stride 2^level_diff (lgf.hpp:222-262);
-        // desc[0] < 0: LGF_GE table -desc[0]-1, E(n) = f[|n1|] f[|n2|] f[|n3|]
-        const int ld = desc[4 * item];
-        const int bx = desc[4 * item + 1], by = desc[4 * item + 2], bz = desc[4 * item + 3];
-        if (ld >= 0)
-        {
-            const int st = 1 << ld;
-            for (int i = threadIdx.x; i < NIN * NIN; i += blockDim.x)
-            {
-                const int x = i % NIN, y = i / NIN;
-                s_in[i] = (R)lgf_get_dev((bx + x) * st, (by + y) * st, (bz + z) * st, table);
-            }
-        }
-        else
-        {
-            const double* f = ge + (size_t)(-ld - 1) * ge_stride;
-            const double fz = f[abs(bz + z)];
-            for (int i = threadIdx.x; i < NIN * NIN; i += blockDim.x)
-            {
-                const int x = i % NIN, y = i / NIN;
-                s_in[i] = (R)(f[abs(bx + x)] * f[abs(by + y)] * fz);
-            }
-        }
-    }
-    else
-    {
-        const double* blk = field + (size_t)item * P * P * P + (size_t)z * P * P;
-        for (int i = threadIdx.x; i < NIN * NIN; i += blockDim.x) s_in[i] = (R)blk[i];
-    }
-    __syncthreads();
     // x: real NIN -> NB half frequencies
     for (int i = threadIdx.x; i < NIN * NB; i += blockDim.x)
     {
@@ -229,7 +182,6 @@ __global__ void __launch_bounds__(256) fwd_xy_kernel(const double* __restrict__ 
     }
     __syncthreads();
     // y: NIN -> P
-    cx<R>* out = W + ((size_t)item * NIN + z) * (P * NB);
     for (int i = threadIdx.x; i < P * NB; i += blockDim.x)
     {
         const int ky = i / NB, kx = i % NB;
@@ -244,6 +196,176 @@ __global__ void __launch_bounds__(256) fwd_xy_kernel(const double* __restrict__ 
         }
         out[i] = s;
     }
+}
+
+// fwd_xy: x and y transforms of one z plane of one LGF block, in FP64:
+//   desc[4*item] = {ld, bx, by, bz}: G((b + i) * 2^ld), ld < 0: table -ld-1 of
+//   the integrating factor
+// W: [item][z < P][ky < P][kx < NB]
+template<int NB>
+__global__ void __launch_bounds__(256) fwd_xy_kernel(const int* __restrict__ desc, const double* __restrict__ table,
+                                                     const double* __restrict__ tw, double2* __restrict__ W,
+                                                     const double* __restrict__ ge, int ge_stride)
+{
+    constexpr int P = 2 * NB - 1, NIN = P;
+    __shared__ double2 s_tw[P];
+    __shared__ double s_in[NIN * NIN];
+    __shared__ double2 s_x1[NIN * NB];
+    const int item = blockIdx.x;
+    const int z = blockIdx.y;
+    load_tw<double>(s_tw, tw, P);
+    // desc[0] >= 0: LGF_GL at stride 2^level_diff (lgf.hpp:222-262);
+    // desc[0] < 0: LGF_GE table -desc[0]-1, E(n) = f[|n1|] f[|n2|] f[|n3|]
+    const int ld = desc[4 * item];
+    const int bx = desc[4 * item + 1], by = desc[4 * item + 2], bz = desc[4 * item + 3];
+    if (ld >= 0)
+    {
+        const int st = 1 << ld;
+        for (int i = threadIdx.x; i < NIN * NIN; i += blockDim.x)
+        {
+            const int x = i % NIN, y = i / NIN;
+            s_in[i] = lgf_get_dev((bx + x) * st, (by + y) * st, (bz + z) * st, table);
+        }
+    }
+    else
+    {
+        const double* f = ge + (size_t)(-ld - 1) * ge_stride;
+        const double fz = f[abs(bz + z)];
+        for (int i = threadIdx.x; i < NIN * NIN; i += blockDim.x)
+        {
+            const int x = i % NIN, y = i / NIN;
+            s_in[i] = f[abs(bx + x)] * f[abs(by + y)] * fz;
+        }
+    }
+    __syncthreads();
+    plane_xy<double, NB, NIN>(s_tw, s_in, s_x1, W + ((size_t)item * NIN + z) * (P * NB));
+}
+
+// Single-block convolution (fft::Convolution, convolution.hpp:141-328): out +=
+// scale * window of source * kernel, in three launches that spread the one
+// block over the chip (one CTA per block left 147 SMs idle: 82 us in six
+// launches at Nb = 18 FP64).
+//   conv_xy   CTA per z plane of the kernel (P, FP64) and of the source (NB)
+//   conv_z    CTA per ky: z transforms of both, their product (kernel spectrum
+//             rounded to R first, as the sweeps keep it) and the inverse z
+//             transform to the NB window planes, in shared memory
+//   conv_out  CTA per window plane: inverse y, c2r along x, added to out
+// The inverse runs in FP64 in both precisions.
+template<class R, int NB>
+__global__ void __launch_bounds__(256) conv_xy_kernel(const double* __restrict__ kernel,
+                                                      const double* __restrict__ source,
+                                                      const double* __restrict__ tw, double2* __restrict__ WK,
+                                                      cx<R>* __restrict__ WS)
+{
+    constexpr int P = 2 * NB - 1;
+    __shared__ double2 s_tw[P];
+    __shared__ double s_in[P * P];
+    __shared__ double2 s_x1[P * NB];
+    const int z = blockIdx.x;
+    if (z < P)
+    {
+        load_tw<double>(s_tw, tw, P);
+        for (int i = threadIdx.x; i < P * P; i += blockDim.x) s_in[i] = kernel[(size_t)z * P * P + i];
+        __syncthreads();
+        plane_xy<double, NB, P>(s_tw, s_in, s_x1, WK + (size_t)z * P * NB);
+    }
+    else
+    {
+        cx<R>* t = reinterpret_cast<cx<R>*>(s_tw);
+        R* in = reinterpret_cast<R*>(s_in);
+        for (int j = threadIdx.x; j < P; j += blockDim.x) t[j] = mk<R>((R)tw[2 * j], (R)tw[2 * j + 1]);
+        for (int i = threadIdx.x; i < NB * NB; i += blockDim.x) in[i] = (R)source[(size_t)(z - P) * NB * NB + i];
+        __syncthreads();
+        plane_xy<R, NB, NB>(t, in, reinterpret_cast<cx<R>*>(s_x1), WS + (size_t)(z - P) * P * NB);
+    }
+}
+
+template<class R, int NB>
+__global__ void __launch_bounds__((2 * NB - 1) * NB) conv_z_kernel(const double2* __restrict__ WK,
+                                                                   const cx<R>* __restrict__ WS,
+                                                                   const double* __restrict__ tw,
+                                                                   double2* __restrict__ V)
+{
+    constexpr int P = 2 * NB - 1, NP = P * NB;
+    __shared__ double2 s_tw[P];
+    __shared__ cx<R> s_twr[P];
+    __shared__ double2 s_k[P * NB];
+    __shared__ cx<R> s_s[NB * NB];
+    __shared__ double2 s_p[P * NB];
+    const int ky = blockIdx.x, kx = threadIdx.x % NB, kz = threadIdx.x / NB;
+    for (int j = threadIdx.x; j < P; j += blockDim.x)
+    {
+        s_tw[j] = make_double2(tw[2 * j], tw[2 * j + 1]);
+        s_twr[j] = mk<R>((R)tw[2 * j], (R)tw[2 * j + 1]);
+    }
+    s_k[threadIdx.x] = WK[(size_t)kz * NP + ky * NB + kx];
+    if (kz < NB) s_s[threadIdx.x] = WS[(size_t)kz * NP + ky * NB + kx];
+    __syncthreads();
+    double2 g = make_double2(0.0, 0.0);
+    cx<R> s = mk<R>(0, 0);
+    int j = 0;
+#pragma unroll 5
+    for (int z = 0; z < P; ++z)
+    {
+        cmac<double>(g, s_k[z * NB + kx], s_tw[j]);
+        if (z < NB) cmac<R>(s, s_s[z * NB + kx], s_twr[j]);
+        j += kz;
+        if (j >= P) j -= P;
+    }
+    cx<R> p = mk<R>(0, 0);
+    cmac<R>(p, mk<R>((R)g.x, (R)g.y), s);
+    s_p[threadIdx.x] = make_double2((double)p.x, (double)p.y);
+    __syncthreads();
+    if (kz >= NB) return;
+    // window plane zo = kz
+    double2 v = make_double2(0.0, 0.0);
+    j = 0;
+#pragma unroll 5
+    for (int k = 0; k < P; ++k)
+    {
+        cmac_conj<double>(v, s_p[k * NB + kx], s_tw[j]);
+        j += kz + NB - 1;
+        if (j >= P) j -= P;
+    }
+    V[((size_t)kz * P + ky) * NB + kx] = v;
+}
+
+template<int NB>
+__global__ void __launch_bounds__(NB* NB) conv_out_kernel(const double2* __restrict__ V,
+                                                          const double* __restrict__ tw, double scale,
+                                                          double* __restrict__ out)
+{
+    constexpr int P = 2 * NB - 1;
+    __shared__ double2 s_tw[P];
+    __shared__ double2 s_v[P * NB];
+    __shared__ double2 s_y[NB * (NB + 1)];
+    const int zo = blockIdx.x, a = threadIdx.x % NB, yo = threadIdx.x / NB;
+    for (int j = threadIdx.x; j < P; j += blockDim.x) s_tw[j] = make_double2(tw[2 * j], tw[2 * j + 1]);
+    for (int i = threadIdx.x; i < P * NB; i += blockDim.x) s_v[i] = V[(size_t)zo * P * NB + i];
+    __syncthreads();
+    double2 v = make_double2(0.0, 0.0);
+    int j = 0;
+#pragma unroll 5
+    for (int k = 0; k < P; ++k)
+    {
+        cmac_conj<double>(v, s_v[k * NB + a], s_tw[j]);
+        j += yo + NB - 1;
+        if (j >= P) j -= P;
+    }
+    s_y[yo * (NB + 1) + a] = v;
+    __syncthreads();
+    // c2r: Re y_0 + 2 sum_{k >= 1} Re(y_k e^{+2 pi i k (xo + NB - 1) / P}), xo = a
+    double sx = 0.0;
+    j = 0;
+#pragma unroll 6
+    for (int k = 1; k < NB; ++k)
+    {
+        j += a + NB - 1;
+        if (j >= P) j -= P;
+        const double2 y = s_y[yo * (NB + 1) + k], t = s_tw[j];
+        sx = fma(y.x, t.x, fma(y.y, t.y, sx));
+    }
+    out[((size_t)zo * NB + yo) * NB + a] += scale * (s_y[yo * (NB + 1)].x + 2.0 * sx);
 }
 
 // fwd_z: per (ky,kx) pencil, NIN -> P; spectrum slot = item_slot[item] (or item)
@@ -661,21 +783,30 @@ struct Conv
         c.launches += 2;
     }
 
-    // LGF blocks (or a dense kernel) are transformed in FP64 and stored in R
-    static void forward_lgf(Ctx& c, const int* d_desc, const double* dense, const int* d_slot, int n,
-                            void* spec)
+    // LGF blocks are transformed in FP64 and stored in R
+    static void forward_lgf(Ctx& c, const int* d_desc, const int* d_slot, int n, void* spec)
     {
         if (!n) return;
         double2* W = (double2*)c.d_w.p;
-        if (dense)
-            fwd_xy_kernel<double, NB, P, kFromDense><<<dim3(n, P), 256, 0, c.stream>>>(
-                dense, nullptr, nullptr, nullptr, c.d_tw64.p, W, nullptr, 0);
-        else
-            fwd_xy_kernel<double, NB, P, kFromLgf><<<dim3(n, P), 256, 0, c.stream>>>(
-                nullptr, nullptr, d_desc, c.d_lgf_table.p, c.d_tw64.p, W, c.d_ge.p, c.ge_stride);
+        fwd_xy_kernel<NB><<<dim3(n, P), 256, 0, c.stream>>>(d_desc, c.d_lgf_table.p, c.d_tw64.p, W, c.d_ge.p,
+                                                            c.ge_stride);
         fwd_z_kernel<double, R, NB, P><<<dim3(n, (NP + 127) / 128), 128, 0, c.stream>>>(W, d_slot,
                                                                                       (cx<R>*)spec);
         c.launches += 2;
+    }
+
+    // bytes of a single-block convolution's work buffer
+    static constexpr size_t conv_bytes = (size_t)(P + 2 * NB) * NP * sizeof(double2);
+
+    static void conv_block(Ctx& c, const double* src, const double* kernel, double* out, double scale, void* work)
+    {
+        double2* WK = (double2*)work;
+        double2* V = WK + (size_t)P * NP;
+        cx<R>* WS = (cx<R>*)(V + (size_t)NB * NP);
+        conv_xy_kernel<R, NB><<<P + NB, 256, 0, c.stream>>>(kernel, src, c.d_tw64.p, WK, WS);
+        conv_z_kernel<R, NB><<<P, P * NB, 0, c.stream>>>(WK, WS, c.d_tw64.p, V);
+        conv_out_kernel<NB><<<NB, NB * NB, 0, c.stream>>>(V, c.d_tw64.p, scale, out);
+        c.launches += 3;
     }
 
     static void mac(Ctx& c, const void* G, const void* S, const int* ptr, const int* src, const int* spec,
@@ -809,7 +940,7 @@ void launch_spectra(Ctx& c, const std::vector<std::array<int, 5>>& new_slots)
         d_slot.upload(slot, c.stream);
         dispatch(c, [&](auto cv) {
             using CV = decltype(cv);
-            CV::forward_lgf(c, d_desc.p, nullptr, d_slot.p, (int)nb, c.d_spec.p);
+            CV::forward_lgf(c, d_desc.p, d_slot.p, (int)nb, c.d_spec.p);
         });
         IBLGF_CUDA(cudaGetLastError());
         IBLGF_CUDA(cudaStreamSynchronize(c.stream));  // d_desc / d_slot go out of scope
@@ -913,36 +1044,24 @@ void launch_inverse_targets(Ctx& c, const FmmPlan& p, const void* acc, double* f
     IBLGF_CUDA(cudaGetLastError());
 }
 
+// the work buffer is kept with the context
 void launch_conv_block(Ctx& c, const double* src, const double* kernel, double* out, double scale)
 {
-    const size_t cb = c.cplx_bytes();
-    DevBuf<char> gspec, sspec, acc;
-    gspec.alloc(c.NC * cb);
-    sspec.alloc(c.NC * cb);
-    acc.alloc(c.NC * cb);
-    ensure(c.d_w, (size_t)c.P * c.P * c.Nb * 16);
-    std::vector<int> zero{0}, ptr{0, 1};  // the FP64 inverse of one block fits: Nb*P*Nb <= P*P*Nb
-    DevBuf<int> d_zero, d_ptr;
-    d_zero.upload(zero, c.stream);
-    d_ptr.upload(ptr, c.stream);
     const double s = scale / ((double)c.P * c.P * c.P);
     dispatch(c, [&](auto cv) {
         using CV = decltype(cv);
-        CV::forward_lgf(c, nullptr, kernel, nullptr, 1, gspec.p);
-        CV::forward_field(c, src, d_zero.p, 1, sspec.p);
-        CV::mac(c, gspec.p, sspec.p, d_ptr.p, d_zero.p, d_zero.p, 1, acc.p);
-        CV::inverse(c, acc.p, d_zero.p, 1, s, out, false);
+        ensure(c.conv_work, CV::conv_bytes);
+        CV::conv_block(c, src, kernel, out, s, c.conv_work.p);
     });
     IBLGF_CUDA(cudaGetLastError());
     IBLGF_CUDA(cudaStreamSynchronize(c.stream));
 }
 
 // ---------------------------------------------------------------------------
-// Single-block convolution without any device allocation. The per-call
-// temporaries of launch_conv_block (LGF, source and product spectra, the
-// transform work array, two index arrays) live instead in one file-scope
-// device array of kNoAllocScratchBytes (2 MiB). At the largest supported
-// block (Nb = 18, FP64) a call needs 1.41 MB of it.
+// Single-block convolution without any device allocation. The work buffer of
+// launch_conv_block lives instead in one file-scope device array of
+// kNoAllocScratchBytes (2 MiB); the largest supported block (Nb = 18) needs
+// 0.72 MB of it.
 //
 // Who needs it: a host application that has already reserved the device
 // memory for its own block pool, or that calls the solve from a section in
@@ -955,10 +1074,9 @@ void launch_conv_block(Ctx& c, const double* src, const double* kernel, double* 
 // Limits: the scratch is one array per device, shared by every context and
 // stream of that device, so calls that overlap in time on different streams
 // race on it; serialise them (one stream, or a host lock). The first call on a
-// device performs the one-time set-up (symbol address, index arrays), so make
-// it before any stream capture begins. No scratch byte needs to start at zero:
-// every byte a kernel reads is written earlier in the same call, and the two
-// index arrays are written once at set-up.
+// device looks up the symbol's address, so make it before any stream capture
+// begins. No scratch byte needs to start at zero: every byte a kernel reads is
+// written earlier in the same call.
 constexpr size_t kNoAllocScratchBytes = size_t(2) << 20;
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
@@ -967,19 +1085,6 @@ namespace
 constexpr int kNoAllocMaxDevices = 64;
 unsigned char* g_noalloc_ptr[kNoAllocMaxDevices] = {};
 std::mutex g_noalloc_mutex;
-
-// index arrays of the one-block pair list: zero = {0}, ptr = {0, 1}
-__global__ void noalloc_index_kernel(int* idx)
-{
-    if (threadIdx.x == 0)
-    {
-        idx[0] = 0;
-        idx[1] = 0;
-        idx[2] = 1;
-    }
-}
-
-size_t round256(size_t b) { return (b + 255) / 256 * 256; }
 
 // Makes the context's device current for the scope of a call and restores
 // the caller's current device on every way out (return or exception).
@@ -1000,7 +1105,7 @@ struct DeviceScope
 
 // the static scratch's device address on the current device (set up once
 // per device); the caller holds a DeviceScope for the context's device
-unsigned char* noalloc_scratch(Ctx& c)
+unsigned char* noalloc_scratch()
 {
     int dev = -1;
     IBLGF_CUDA(cudaGetDevice(&dev));
@@ -1011,9 +1116,6 @@ unsigned char* noalloc_scratch(Ctx& c)
         void* ptr = nullptr;
         IBLGF_CUDA(cudaGetSymbolAddress(&ptr, g_noalloc_scratch));
         if (!ptr) throw Error(IBLGF_ECUDA, "cudaGetSymbolAddress returned a null scratch address");
-        noalloc_index_kernel<<<1, 32, 0, c.stream>>>(static_cast<int*>(ptr));
-        IBLGF_CUDA(cudaGetLastError());
-        IBLGF_CUDA(cudaStreamSynchronize(c.stream));
         g_noalloc_ptr[dev] = static_cast<unsigned char*>(ptr);
     }
     return g_noalloc_ptr[dev];
@@ -1022,38 +1124,13 @@ unsigned char* noalloc_scratch(Ctx& c)
 
 void launch_conv_block_noalloc(Ctx& c, const double* src, const double* kernel, double* out, double scale)
 {
-    // scratch layout: [index ints | LGF spectrum | source spectrum | product | work]
-    const size_t spec = round256((size_t)c.NC * 16);  // sized for FP64 spectra
-    const size_t work = round256((size_t)c.P * c.P * c.Nb * 16);
-    const size_t need = 256 + 3 * spec + work;
-    if (need > kNoAllocScratchBytes)
-        throw Error(IBLGF_EINVAL, "block too large for the static convolution scratch (needs " +
-                                      std::to_string(need) + " bytes, limit " +
-                                      std::to_string(kNoAllocScratchBytes) + ")");
     DeviceScope on_device(c.cfg.device);
-    unsigned char* base = noalloc_scratch(c);
-    const int* d_zero = reinterpret_cast<const int*>(base);
-    const int* d_ptr = d_zero + 1;
-    unsigned char* gspec = base + 256;
-    unsigned char* sspec = gspec + spec;
-    unsigned char* acc = sspec + spec;
-    unsigned char* W = acc + spec;
+    unsigned char* work = noalloc_scratch();
     const double s = scale / ((double)c.P * c.P * c.P);
     dispatch(c, [&](auto cv) {
         using CV = decltype(cv);
-        using R = typename CV::Real;
-        constexpr int NB = CV::Nb, P = CV::P, NP = CV::NP;
-        fwd_xy_kernel<double, NB, P, kFromDense><<<dim3(1, P), 256, 0, c.stream>>>(
-            kernel, nullptr, nullptr, nullptr, c.d_tw64.p, (double2*)W, nullptr, 0);
-        fwd_z_kernel<double, R, NB, P><<<dim3(1, (NP + 127) / 128), 128, 0, c.stream>>>(
-            (const double2*)W, nullptr, (cx<R>*)gspec);
-        CV::launch_fwd_xy_rows(c, src, d_zero, 1, (cx<R>*)W);
-        fwd_z_kernel<R, R, NB, NB><<<dim3(1, (NP + 127) / 128), 128, 0, c.stream>>>(
-            (const cx<R>*)W, nullptr, (cx<R>*)sspec);
-        mac_kernel<R><<<dim3((unsigned)((c.NC + 127) / 128), 1), 128, 0, c.stream>>>(
-            (const cx<R>*)gspec, (const cx<R>*)sspec, d_ptr, d_zero, d_zero, c.NC, (cx<R>*)acc);
-        CV::launch_inverse(c, (const cx<R>*)acc, d_zero, 1, s, out, false);
-        c.launches += 6;
+        static_assert(CV::conv_bytes <= kNoAllocScratchBytes, "every supported block fits the static scratch");
+        CV::conv_block(c, src, kernel, out, s, work);
     });
     IBLGF_CUDA(cudaGetLastError());
 }

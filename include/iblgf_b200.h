@@ -354,14 +354,14 @@ int iblgf_batch_apply_lgf(iblgf_ctx* ctx, int src, int tgt);
 int iblgf_conv_block(iblgf_ctx* ctx, const double* src, const double* kernel, double* out,
                      double scale);
 /* Same result as iblgf_conv_block, but the call allocates no device memory:
- * its temporaries live in a 2 MiB static device array (1.41 MB used at
- * Nb = 18); a block needing more is rejected with IBLGF_EINVAL. For hosts
+ * its temporaries live in a 2 MiB static device array (0.72 MB used at
+ * Nb = 18, the largest block). For hosts
  * that must not allocate at call time (device memory already reserved for
  * their own pool, or no device-wide synchronisation from cudaFree allowed).
  * Enqueues on the context stream and returns without synchronising. The
  * scratch is shared by all contexts on a device: calls overlapping in time on
- * different streams race. The first call on a device runs a one-time set-up;
- * make it before any stream capture. No reference counterpart: the
+ * different streams race. The first call on a device looks up the array's
+ * address; make it before any stream capture. No reference counterpart: the
  * reference's fft::Convolution owns FFTW buffers allocated at construction. */
 int iblgf_conv_block_noalloc(iblgf_ctx* ctx, const double* src, const double* kernel, double* out,
                              double scale);

@@ -54,3 +54,23 @@ def test_integrating_factor_radii(e, alpha):
         g.apply_if(fs, fs, alpha)
         sel = np.asarray(o.levels) >= o.base_level  # the coarser blocks keep their values
         assert rel_linf(g.download(fs)[sel], ref[sel]) < 1e-12
+
+
+@pytest.mark.parametrize("precision,tol", [(B.FP64, 1e-12), (B.FP32, 1e-5)])
+@pytest.mark.parametrize("e", [4, 6, 8, 10, 14, 16])
+def test_conv_block_extents(e, precision, tol):
+    """The single-block convolution adds to its output; twice, so that the kept work buffer is used again."""
+    torch = pytest.importorskip("torch")
+    N = e + 2
+    P = 2 * N - 1
+    g = B.Solver((-2 * e,) * 3, (4 * e,) * 3, e, 1.0, [((-e,) * 3, (2 * e,) * 3)], precision=precision)
+    rng = np.random.default_rng(e)
+    for _ in range(2):
+        src, ker = rng.standard_normal((N, N, N)), rng.standard_normal((P, P, P))
+        base = rng.standard_normal(N ** 3)
+        out = torch.tensor(base, device="cuda")
+        ts, tk = (torch.tensor(a.ravel(order="F"), device="cuda") for a in (src, ker))
+        torch.cuda.synchronize()
+        g.conv_block(ts.data_ptr(), tk.data_ptr(), out.data_ptr(), 0.5)
+        ref = O.block_conv(src, ker, 0.5).ravel(order="F")
+        assert rel_linf(out.cpu().numpy() - base, ref) < tol
