@@ -677,8 +677,10 @@ void launch_solve_begin(Ctx& c, const double* src, double* st, double* tt, doubl
 // blocks, its interpolated values), added into source_tmp
 void launch_source_correction(Ctx& c, const double* target_tmp, double* corr, double* source_tmp, const int* list,
                               int n, double inv_dx2);
+// shift: constants added to the three velocity components that the nonlinear
+// term reads (null: none); scale: of curl_transpose and of the nonlinear term
 void launch_op(Ctx& c, int op, const double* const* in, int n_in, double* const* out, int n_out, const int* list,
-               const double* dx, int n, double scale);
+               const double* dx, int n, double scale, const double* shift = nullptr);
 void buffer_exchange(Ctx& c, int field, int level);
 void apply_op(Ctx& c, int op, const int* in, int n_in, const int* out, int n_out, int level, double scale);
 void launch_conv_block(Ctx& c, const double* src, const double* kernel, double* out, double scale);

@@ -27,7 +27,10 @@ void launch_clean(Ctx& c, double* f, const int* d_leaf, bool non_leaf_only, int 
 void launch_axpby(Ctx& c, double* to, const double* from, double a, int mode);
 void launch_clean_vf(Ctx& c, double* const* f, int n, const int* d_leaf, bool non_leaf_only, int width = 1);
 void launch_axpby_vf(Ctx& c, double* const* to, const double* const* from, int n, double a, int mode);
-void launch_smooth(Ctx& c, double* f, const int* list, const int* ptr, const int* dirs, int n, int reps);
+void launch_lincomb_vf(Ctx& c, double* const* to, const double* const* x, const double* const* y, int n, double a,
+                       int mode);
+void launch_smooth_vf(Ctx& c, double* const* f, int m, const int* list, const int* ptr, const int* dirs, int n,
+                      int reps);
 
 namespace
 {
@@ -245,26 +248,21 @@ class Step
         else
             up_and_down(u);
         copy(u, s.q_i, 1.0);
-        // stage 1
-        clean(s.g_i, false);
+        // stage 1. A copy followed by an add into it, and a clean of a field
+        // that the next call writes as a whole, are one pass here.
         clean(s.d_i, false);
         clean(s.cell_aux, false);
-        clean(s.face_aux, false);
         nonlinear(u, s.g_i, coeff_a(1, 1) * (-dt));
-        copy(s.q_i, s.r_i, 1.0);
-        add(s.g_i, s.r_i, 1.0);
+        lincomb(s.q_i, s.g_i, s.r_i, 1.0, 0);
         stage = 1;
         lin_sys(alpha[0]);
         // stage 2
-        clean(s.r_i, false);
         clean(s.d_i, false);
         clean(s.cell_aux, false);
-        add(s.g_i, s.face_aux, -1.0);
-        copy(s.face_aux, s.w_1, -1.0 / dt / coeff_a(1, 1));
+        lincomb(s.face_aux, s.g_i, s.w_1, -1.0 / dt / coeff_a(1, 1), 1);
         apply_if(s.q_i, s.q_i, alpha[0]);
         apply_if(s.w_1, s.w_1, alpha[0]);
-        add(s.q_i, s.r_i, 1.0);
-        add(s.w_1, s.r_i, dt * coeff_a(2, 1));
+        lincomb(s.q_i, s.w_1, s.r_i, dt * coeff_a(2, 1), 0);
         up_and_down(s.u_i);
         nonlinear(s.u_i, s.g_i, coeff_a(2, 2) * (-dt));
         add(s.g_i, s.r_i, 1.0);
@@ -273,11 +271,8 @@ class Step
         // stage 3
         clean(s.d_i, false);
         clean(s.cell_aux, false);
-        clean(s.w_2, false);
-        add(s.g_i, s.face_aux, -1.0);
-        copy(s.face_aux, s.w_2, -1.0 / dt / coeff_a(2, 2));
-        copy(s.q_i, s.r_i, 1.0);
-        add(s.w_1, s.r_i, dt * coeff_a(3, 1));
+        lincomb(s.face_aux, s.g_i, s.w_2, -1.0 / dt / coeff_a(2, 2), 1);
+        lincomb(s.q_i, s.w_1, s.r_i, dt * coeff_a(3, 1), 0);
         add(s.w_2, s.r_i, dt * coeff_a(3, 2));
         apply_if(s.r_i, s.r_i, alpha[1]);
         up_and_down(s.u_i);
@@ -387,11 +382,14 @@ class Step
         for (int k = 0; k < from.n; ++k) t[k] = F(to.id[k]), fr[k] = F(from.id[k]);
         launch_axpby_vf(c, t, fr, from.n, a_, 1);
     }
-    void scale(const VF& f, double a_)
+    // mode 0: to = x + a y, 1: to = a (x - y)
+    void lincomb(const VF& x, const VF& y, const VF& to, double a_, int mode)
     {
-        double* t[3];
-        for (int k = 0; k < f.n; ++k) t[k] = F(f.id[k]);
-        launch_axpby_vf(c, t, nullptr, f.n, a_, 2);
+        double *t[3], *px[3], *py[3];
+        comps(to, t);
+        comps(x, px);
+        comps(y, py);
+        launch_lincomb_vf(c, t, px, py, to.n, a_, mode);
     }
     // field pointers and transfer matrices of the components
     void comps(const VF& f, double* (&p)[3]) const
@@ -441,7 +439,8 @@ class Step
         up(f);
         down_to_correction(f);
     }
-    void op(int o, std::initializer_list<const VF*> in, const VF& out, int l, double sc)
+    void op(int o, std::initializer_list<const VF*> in, const VF& out, int l, double sc,
+            const double* shift = nullptr)
     {
         const double* pin[6] = {};
         double* pout[3] = {};
@@ -449,39 +448,38 @@ class Step
         for (const VF* v : in)
             for (int k = 0; k < v->n; ++k) pin[n_in++] = F(v->id[k]);
         for (int k = 0; k < out.n; ++k) pout[k] = F(out.id[k]);
-        launch_op(c, o, pin, n_in, pout, out.n, ol.list[l].p, ol.dx[l].p, (int)ol.list[l].n, sc);
+        launch_op(c, o, pin, n_in, pout, out.n, ol.list[l].p, ol.dx[l].p, (int)ol.list[l].n, sc,
+                  shift);
     }
     void clean_leaf_correction_boundary(const VF& f, int l, bool leaf_only_boundary)
     {
-        if (leaf_only_boundary)
-            for (int k = 0; k < f.n; ++k) launch_zero_blocks(c, F(f.id[k]), s.corr[l].p, (int)s.corr[l].n);
+        double* p[3];
+        comps(f, p);
+        if (leaf_only_boundary) launch_zero_blocks_vf(c, p, f.n, s.corr[l].p, (int)s.corr[l].n);
         if (l != bl) return;
         const int v = leaf_only_boundary ? 1 : 0;
         // smooth2zero scales every component; the reference calls it once per component
-        for (int k = 0; k < f.n; ++k)
-            launch_smooth(c, F(f.id[k]), s.sm_list[v].p, s.sm_ptr[v].p, s.sm_dirs[v].p, s.sm_n[v], f.n);
+        launch_smooth_vf(c, p, f.n, s.sm_list[v].p, s.sm_ptr[v].p, s.sm_dirs[v].p, s.sm_n[v], f.n);
     }
+    // the convecting velocity src - frame velocity is formed where the operator
+    // reads it, and its result scaled where it is written
     void nonlinear(const VF& src, const VF& tgt, double sc)
     {
         clean(s.edge_aux, false);
         clean(tgt, false);
-        clean(s.face_aux, false);
         for (int l = bl; l < depth; ++l)
         {
             exchange(src, l);
             op(3, {&src}, s.edge_aux, l, 1.0);
         }
-        copy(src, s.face_aux, 1.0);
         // add_field_expression(frame_vel, -1): a constant frame velocity
-        for (int k = 0; k < 3; ++k)
-            if (opt.frame_vel[k] != 0.0) launch_axpby(c, F(s.face_aux.id[k]), nullptr, -opt.frame_vel[k], 3);
+        const double shift[3] = {-opt.frame_vel[0], -opt.frame_vel[1], -opt.frame_vel[2]};
         for (int l = bl; l < depth; ++l)
         {
             exchange(s.edge_aux, l);
             clean_leaf_correction_boundary(s.edge_aux, l, false);
-            op(5, {&s.face_aux, &s.edge_aux}, tgt, l, 1.0);
+            op(5, {&src, &s.edge_aux}, tgt, l, sc, shift);
         }
-        scale(tgt, sc);
     }
     void divergence(const VF& src, const VF& tgt)
     {
@@ -673,12 +671,13 @@ void ns_clean_leaf_correction_boundary(Ctx& c, const int* fields, int n, int lev
     for (int k = 0; k < n; ++k)
         if (fields[k] < 0 || fields[k] >= (int)c.fields.size()) throw Error(IBLGF_EINVAL, "bad field id");
     NsState& s = ns_state(c);
+    double* p[3] = {};
+    for (int k = 0; k < n; ++k) p[k] = c.field(fields[k]);
     if (leaf_only_boundary && level < (int)s.corr.size())
-        for (int k = 0; k < n; ++k) launch_zero_blocks(c, c.field(fields[k]), s.corr[level].p, (int)s.corr[level].n);
+        launch_zero_blocks_vf(c, p, n, s.corr[level].p, (int)s.corr[level].n);
     if (level != c.tree.base_level) return;
     const int v = leaf_only_boundary ? 1 : 0;
-    for (int k = 0; k < n; ++k)
-        launch_smooth(c, c.field(fields[k]), s.sm_list[v].p, s.sm_ptr[v].p, s.sm_dirs[v].p, s.sm_n[v], n);
+    launch_smooth_vf(c, p, n, s.sm_list[v].p, s.sm_ptr[v].p, s.sm_dirs[v].p, s.sm_n[v], n);
 }
 
 void ns_options(Ctx& c, const double* frame_vel, double cg_threshold, int cg_max_iter)

@@ -1514,7 +1514,7 @@ void apply_op(Ctx& c, int op, const int* in, int n_in, const int* out, int n_out
         for (int j = 0; j < n_in; ++j)
             if (out[i] == in[j]) throw Error(IBLGF_EINVAL, "operator output aliases an input");
     }
-    launch_op(c, op, pin, n_in, pout, n_out, ol.list[li].p, ol.dx[li].p, (int)ol.list[li].n, scale);
+    launch_op(c, op, pin, n_in, pout, n_out, ol.list[li].p, ol.dx[li].p, (int)ol.list[li].n, op == 4 ? scale : 1.0);
 }
 
 // The block operators on a list of octants (Operator::laplace ... applied to
@@ -1547,7 +1547,7 @@ void apply_op_octants(Ctx& c, int op, const int* in, int n_in, const int* out, i
     DevBuf<double> d_dx;
     d_list.upload(list, c.stream);
     d_dx.upload(dx, c.stream);
-    launch_op(c, op, pin, n_in, pout, n_out, d_list.p, d_dx.p, n, scale);
+    launch_op(c, op, pin, n_in, pout, n_out, d_list.p, d_dx.p, n, op == 4 ? scale : 1.0);
     IBLGF_CUDA(cudaStreamSynchronize(c.stream));  // the lists are freed on return
 }
 

@@ -242,18 +242,35 @@ __global__ void __launch_bounds__(256) tp_band2_kernel(const int* __restrict__ g
 }
 
 // threads walk the buffer shell only: the two z = 0, NB-1 planes, then per
-// inner z plane its ring (rows y = 0, NB-1, columns x = 0, NB-1)
+// inner z plane its ring (rows y = 0, NB-1, columns x = 0, NB-1). The 27
+// neighbours and their offsets are read once into shared memory, so that a
+// node's copy is one load, all of a thread's nodes in flight.
 template<int NB>
-__global__ void halo_kernel(const __grid_constant__ TpFields fs, const int* __restrict__ list, const int* __restrict__ nbr,
-                            const int* __restrict__ bbase, int e)
+__global__ void __launch_bounds__(256) halo_kernel(const __grid_constant__ TpFields fs, const int* __restrict__ list,
+                                                   const int* __restrict__ nbr, const int* __restrict__ bbase, int e)
 {
     constexpr int N3 = NB * NB * NB;
     constexpr int P2 = NB * NB, RING = 4 * NB - 4, SHELL = 2 * P2 + (NB - 2) * RING;
+    constexpr int K = (SHELL + 255) / 256;
+    __shared__ int s_q[27], s_off[27][3];
     const int o = list[blockIdx.x];
     double* f = fs.dst[blockIdx.y];
     double* blk = f + (size_t)o * N3;
-    for (int t = threadIdx.x; t < SHELL; t += blockDim.x)
+    if (threadIdx.x < 27)
     {
+        const int q = nbr[27 * o + threadIdx.x];
+        s_q[threadIdx.x] = q;
+        for (int a = 0; a < 3; ++a) s_off[threadIdx.x][a] = q < 0 ? 0 : bbase[3 * o + a] - 1 - bbase[3 * q + a];
+    }
+    __syncthreads();
+    double v[K];
+    int at[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+    {
+        const int t = 256 * k + threadIdx.x;
+        at[k] = -1;
+        if (t >= SHELL) continue;
         int x, y, z;
         if (t < 2 * P2)
         {
@@ -277,19 +294,20 @@ __global__ void halo_kernel(const __grid_constant__ TpFields fs, const int* __re
                 y = 1 + w / 2;
             }
         }
-        const int i = x + NB * (y + NB * z);
-        const int dx = x == 0 ? -1 : (x == NB - 1 ? 1 : 0);
-        const int dy = y == 0 ? -1 : (y == NB - 1 ? 1 : 0);
-        const int dz = z == 0 ? -1 : (z == NB - 1 ? 1 : 0);
-        const int q = nbr[27 * o + (dx + 1) + 3 * (dy + 1) + 9 * (dz + 1)];
+        const int dx = x == 0 ? 0 : (x == NB - 1 ? 2 : 1);
+        const int dy = y == 0 ? 0 : (y == NB - 1 ? 2 : 1);
+        const int dz = z == 0 ? 0 : (z == NB - 1 ? 2 : 1);
+        const int d = dx + 3 * dy + 9 * dz, q = s_q[d];
         if (q < 0) continue;
         // global cell of this buffer node and its position in q's interior
-        const int lx = bbase[3 * o] - 1 + x - bbase[3 * q];
-        const int ly = bbase[3 * o + 1] - 1 + y - bbase[3 * q + 1];
-        const int lz = bbase[3 * o + 2] - 1 + z - bbase[3 * q + 2];
+        const int lx = s_off[d][0] + x, ly = s_off[d][1] + y, lz = s_off[d][2] + z;
         if (lx < 0 || ly < 0 || lz < 0 || lx >= e || ly >= e || lz >= e) continue;
-        blk[i] = f[(size_t)q * N3 + (lx + 1) + NB * ((ly + 1) + NB * (lz + 1))];
+        at[k] = x + NB * (y + NB * z);
+        v[k] = f[(size_t)q * N3 + (lx + 1) + NB * ((ly + 1) + NB * (lz + 1))];
     }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (at[k] >= 0) blk[at[k]] = v[k];
 }
 
 // Block copies and sums are split over blockIdx.y in pieces of kPiece 16-byte
