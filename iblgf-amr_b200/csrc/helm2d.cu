@@ -157,74 +157,103 @@ __global__ void helm2d_apply_kernel(int nx, int ny, const double* __restrict__ t
 // components of unselected modes are left as they were.
 // op: 0 laplace (cell -> cell), 1 gradient (cell -> face), 2 divergence
 // (face -> cell), 3 curl (face -> edge), 4 curl_transpose (edge -> face, x scale)
-template<int OP>
-__global__ void helm_op_kernel(int nb, int n_modes, int in_comp, int out_comp, double dx, double lz, double scale,
-                               UnitMask mask, const double* __restrict__ src, double* __restrict__ dst)
+// Memory-bound: one thread owns every output component of one (mode, node)
+// pair, keeps real and imaginary parts in registers (each output written
+// once) and blockIdx.y splits a block's pairs over CTAs of kHelmItems pairs
+// per thread. NBT: the block extent at compile time (0: nb at run time).
+// 1024 blocks of 18^2 nodes, 16 modes, us (before: one CTA per block, outputs
+// accumulated in memory, extents divided at run time): curl 184 -> 130,
+// curl_transpose 182 -> 130, gradient 116 -> 109, divergence 96 -> 63, laplace
+// 74 -> 36, nonlinear (48 planes) 277 -> 228, where one pass over the operands
+// takes 78, 78, 52, 52, 26 and 175.
+template<int OP, int NBT>
+__global__ void __launch_bounds__(256) helm_op_kernel(int nb_, int n_modes, int in_comp, int out_comp, double dx,
+                                                      double lz, double scale, UnitMask mask,
+                                                      const double* __restrict__ src, double* __restrict__ dst)
 {
+    const int nb = NBT ? NBT : nb_;
     const int sep = 2 * n_modes, N2 = nb * nb;
-    const double* s = src + (size_t)blockIdx.x * in_comp * N2;
-    double* d = dst + (size_t)blockIdx.x * out_comp * N2;
+    const double* __restrict__ s = src + (size_t)blockIdx.x * in_comp * N2;
+    double* __restrict__ d = dst + (size_t)blockIdx.x * out_comp * N2;
     const double fac = 1.0 / dx;
-    // one thread per (mode, node): it owns every output component of that
-    // mode at that node (consecutive threads take consecutive nodes)
-    for (int q = threadIdx.x; q < n_modes * N2; q += blockDim.x)
+    // one thread per (mode, node): consecutive threads take consecutive nodes
+    const int total = n_modes * N2;
+    for (int q0 = blockIdx.y * (kHelmItems * 256); q0 < total; q0 += gridDim.y * (kHelmItems * 256))
+#pragma unroll
+    for (int k = 0; k < kHelmItems; ++k)
     {
+        const int q = q0 + k * 256 + threadIdx.x;
+        if (q >= total) break;
         const int mode = q / N2, p = q - mode * N2;
-        const int x = p % nb, y = p / nb;
+        const int y = p / nb, x = p - y * nb;
         if (x == 0 || y == 0 || x == nb - 1 || y == nb - 1 || !mask.on(mode)) continue;
-        auto at = [&](int c, int ox, int oy) { return s[(size_t)c * N2 + p + ox + oy * nb]; };
-        auto out = [&](int c) -> double& { return d[(size_t)c * N2 + p]; };
-        const int re = 2 * mode, im = 2 * mode + 1;
-        for (int i = re; i <= im; ++i)
+        const int re = 2 * mode;
+        const double om = 2.0 * M_PI * mode / lz;
+        // value of component group g (0 x or scalar, 1 y, 2 z), part i (0 real,
+        // 1 imaginary) at offset o
+        auto at = [&](int g, int i, int o) { return __ldg(s + (size_t)(g * sep + re + i) * N2 + p + o); };
+        auto put = [&](int g, int i, double v) { d[(size_t)(g * sep + re + i) * N2 + p] = v; };
+        if (OP == 0)
         {
-            if (OP == 0)
-                out(i) = fac * fac * (-4.0 * at(i, 0, 0) + at(i, 0, -1) + at(i, 0, 1) + at(i, -1, 0) + at(i, 1, 0));
-            else if (OP == 1)
+            double v[2], c[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
             {
-                out(i) = fac * (at(i, 0, 0) - at(i, -1, 0));
-                out(sep + i) = fac * (at(i, 0, 0) - at(i, 0, -1));
+                c[i] = at(0, i, 0);
+                v[i] = fac * fac * (-4.0 * c[i] + at(0, i, -nb) + at(0, i, nb) + at(0, i, -1) + at(0, i, 1));
             }
-            else if (OP == 2)
-                out(i) = fac * (-at(i, 0, 0) - at(sep + i, 0, 0) + at(i, 1, 0) + at(sep + i, 0, 1));
-            else if (OP == 3)
-            {
-                out(i) = fac * (at(2 * sep + i, 0, 0) - at(2 * sep + i, 0, -1));
-                out(sep + i) = fac * (-at(2 * sep + i, 0, 0) + at(2 * sep + i, -1, 0));
-                out(2 * sep + i) = fac * (at(sep + i, 0, 0) - at(sep + i, -1, 0) - at(i, 0, 0) + at(i, 0, -1));
-            }
-            else
-            {
-                const double f = fac * scale;
-                out(i) = f * (-at(2 * sep + i, 0, 0) + at(2 * sep + i, 0, 1));
-                out(sep + i) = f * (at(2 * sep + i, 0, 0) - at(2 * sep + i, 1, 0));
-                out(2 * sep + i) = f * (-at(sep + i, 0, 0) + at(sep + i, 1, 0) + at(i, 0, 0) - at(i, 0, 1));
-            }
+            put(0, 0, v[0] - c[0] * om * om);
+            put(0, 1, v[1] - c[1] * om * om);
         }
+        else if (OP == 1)
         {
-            const double om = 2.0 * M_PI * mode / lz;
-            if (OP == 0)
+            double c[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
             {
-                out(re) -= at(re, 0, 0) * om * om;
-                out(im) -= at(im, 0, 0) * om * om;
+                c[i] = at(0, i, 0);
+                put(0, i, fac * (c[i] - at(0, i, -1)));
+                put(1, i, fac * (c[i] - at(0, i, -nb)));
             }
-            else if (OP == 1)
+            put(2, 0, -c[1] * om);
+            put(2, 1, c[0] * om);
+        }
+        else if (OP == 2)
+        {
+            double v[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) v[i] = fac * (-at(0, i, 0) - at(1, i, 0) + at(0, i, 1) + at(1, i, nb));
+            put(0, 0, v[0] - at(2, 1, 0) * om);
+            put(0, 1, v[1] + at(2, 0, 0) * om);
+        }
+        else
+        {
+            // curl (differences backward) and curl_transpose (forward)
+            const double f = OP == 3 ? fac : fac * scale, w = OP == 3 ? om : om * scale;
+            double X[2], Y[2], vx[2], vy[2];
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
             {
-                out(2 * sep + re) = -at(im, 0, 0) * om;
-                out(2 * sep + im) = at(re, 0, 0) * om;
+                X[i] = at(0, i, 0);
+                Y[i] = at(1, i, 0);
+                const double z = at(2, i, 0);
+                if (OP == 3)
+                {
+                    vx[i] = f * (z - at(2, i, -nb));
+                    vy[i] = f * (-z + at(2, i, -1));
+                    put(2, i, f * (Y[i] - at(1, i, -1) - X[i] + at(0, i, -nb)));
+                }
+                else
+                {
+                    vx[i] = f * (-z + at(2, i, nb));
+                    vy[i] = f * (z - at(2, i, 1));
+                    put(2, i, f * (-Y[i] + at(1, i, 1) + X[i] - at(0, i, nb)));
+                }
             }
-            else if (OP == 2)
-            {
-                out(re) -= at(2 * sep + im, 0, 0) * om;
-                out(im) += at(2 * sep + re, 0, 0) * om;
-            }
-            else
-            {
-                const double w = OP == 3 ? om : om * scale;
-                out(re) += at(sep + im, 0, 0) * w;
-                out(im) -= at(sep + re, 0, 0) * w;
-                out(sep + re) -= at(im, 0, 0) * w;
-                out(sep + im) += at(re, 0, 0) * w;
-            }
+            put(0, 0, vx[0] + Y[1] * w);
+            put(0, 1, vx[1] - Y[0] * w);
+            put(1, 0, vy[0] - X[1] * w);
+            put(1, 1, vy[1] + X[0] * w);
         }
     }
 }
@@ -239,30 +268,38 @@ __global__ void helm_op_kernel(int nb, int n_modes, int in_comp, int out_comp, d
 //   dst_z = 1/2 (w_x u_y + w_x[+y] u_y[+y] - w_y u_x - w_y[+x] u_x[+x]).
 // The mask selects planes: every plane; planes mode P .. mode P + P - 1 for
 // the _oneMode form (P planes per mode); every 2^r-th for the _refined form.
-__global__ void helm_nonlinear_kernel(int nb, int n_planes, UnitMask mask, const double* __restrict__ face,
-                                      const double* __restrict__ edge, double* __restrict__ dst)
+// One thread per (plane, node), kHelmItems of them, as helm_op_kernel.
+template<int NBT>
+__global__ void __launch_bounds__(256) helm_nonlinear_kernel(int nb_, int n_planes, UnitMask mask,
+                                                             const double* __restrict__ face,
+                                                             const double* __restrict__ edge,
+                                                             double* __restrict__ dst)
 {
+    const int nb = NBT ? NBT : nb_;
     const int N2 = nb * nb;
     const size_t blk = (size_t)blockIdx.x * 3 * n_planes * N2;
-    const double* u = face + blk;
-    const double* w = edge + blk;
-    double* d = dst + blk;
-    for (int q = threadIdx.x; q < n_planes * N2; q += blockDim.x)
+    const double* __restrict__ u = face + blk;
+    const double* __restrict__ w = edge + blk;
+    double* __restrict__ d = dst + blk;
+    const int total = n_planes * N2;
+    for (int q0 = blockIdx.y * (kHelmItems * 256); q0 < total; q0 += gridDim.y * (kHelmItems * 256))
+#pragma unroll
+    for (int k = 0; k < kHelmItems; ++k)
     {
+        const int q = q0 + k * 256 + threadIdx.x;
+        if (q >= total) break;
         const int i = q / N2, p = q - i * N2;
-        const int x = p % nb, y = p / nb;
+        const int y = p / nb, x = p - y * nb;
         if (x == 0 || y == 0 || x == nb - 1 || y == nb - 1 || !mask.on(i)) continue;
-        const int cx = i, cy = n_planes + i, cz = 2 * n_planes + i;
-        auto U = [&](int c, int ox, int oy) { return u[(size_t)c * N2 + p + ox + oy * nb]; };
-        auto W = [&](int c, int ox, int oy) { return w[(size_t)c * N2 + p + ox + oy * nb]; };
-        d[(size_t)cx * N2 + p] = 0.5 * W(cy, 0, 0) * (U(cz, 0, 0) + U(cz, -1, 0)) -
-                                 0.25 * (W(cz, 0, 0) * (U(cy, 0, 0) + U(cy, -1, 0)) +
-                                         W(cz, 0, 1) * (U(cy, 0, 1) + U(cy, -1, 1)));
-        d[(size_t)cy * N2 + p] = 0.25 * (W(cz, 0, 0) * (U(cx, 0, 0) + U(cx, 0, -1)) +
-                                         W(cz, 1, 0) * (U(cx, 1, 0) + U(cx, 1, -1))) -
-                                 0.5 * W(cx, 0, 0) * (U(cz, 0, 0) + U(cz, 0, -1));
-        d[(size_t)cz * N2 + p] = 0.5 * (W(cx, 0, 0) * U(cy, 0, 0) + W(cx, 0, 1) * U(cy, 0, 1) -
-                                        W(cy, 0, 0) * U(cx, 0, 0) - W(cy, 1, 0) * U(cx, 1, 0));
+        const size_t cx = (size_t)i * N2 + p, cy = cx + (size_t)n_planes * N2, cz = cy + (size_t)n_planes * N2;
+        auto U = [&](size_t c, int ox, int oy) { return __ldg(u + c + ox + oy * nb); };
+        auto W = [&](size_t c, int ox, int oy) { return __ldg(w + c + ox + oy * nb); };
+        d[cx] = 0.5 * W(cy, 0, 0) * (U(cz, 0, 0) + U(cz, -1, 0)) -
+                0.25 * (W(cz, 0, 0) * (U(cy, 0, 0) + U(cy, -1, 0)) + W(cz, 0, 1) * (U(cy, 0, 1) + U(cy, -1, 1)));
+        d[cy] = 0.25 * (W(cz, 0, 0) * (U(cx, 0, 0) + U(cx, 0, -1)) + W(cz, 1, 0) * (U(cx, 1, 0) + U(cx, 1, -1))) -
+                0.5 * W(cx, 0, 0) * (U(cz, 0, 0) + U(cz, 0, -1));
+        d[cz] = 0.5 * (W(cx, 0, 0) * U(cy, 0, 0) + W(cx, 0, 1) * U(cy, 0, 1) - W(cy, 0, 0) * U(cx, 0, 0) -
+                       W(cy, 1, 0) * U(cx, 1, 0));
     }
 }
 
@@ -484,6 +521,32 @@ UnitMask unit_mask(int n_units, const unsigned char* host_mask)
     return m;
 }
 
+namespace
+{
+// the block extents of the solver's blocks at compile time, others at run time
+template<class F>
+void helm_extent(int nb, F&& f)
+{
+    switch (nb)
+    {
+        case 6: f(std::integral_constant<int, 6>{}); return;
+        case 8: f(std::integral_constant<int, 8>{}); return;
+        case 10: f(std::integral_constant<int, 10>{}); return;
+        case 12: f(std::integral_constant<int, 12>{}); return;
+        case 16: f(std::integral_constant<int, 16>{}); return;
+        case 18: f(std::integral_constant<int, 18>{}); return;
+        default: f(std::integral_constant<int, 0>{}); return;
+    }
+}
+
+// CTAs along y for `items` (unit, node) pairs of a block (the kernels stride
+// over what is beyond the grid's limit)
+unsigned helm_chunks(long long items)
+{
+    return (unsigned)std::min<long long>((items + 256 * kHelmItems - 1) / (256 * kHelmItems), 65535);
+}
+}  // namespace
+
 void helm2d_op(Ctx& c, int op, int nb, int n_blocks, int n_modes, double dx, double lz, double scale,
                const unsigned char* host_mode_mask, const double* dev_src, double* dev_dst)
 {
@@ -495,17 +558,21 @@ void helm2d_op(Ctx& c, int op, int nb, int n_blocks, int n_modes, double dx, dou
     const int sep = 2 * n_modes;
     const int in_comp = (op == 0 || op == 1) ? sep : 3 * sep;
     const int out_comp = (op == 0 || op == 2) ? sep : 3 * sep;
-    auto go = [&](auto kfn) {
-        kfn<<<n_blocks, 256, 0, c.stream>>>(nb, n_modes, in_comp, out_comp, dx, lz, scale, mask, dev_src, dev_dst);
-    };
-    switch (op)
-    {
-        case 0: go(helm_op_kernel<0>); break;
-        case 1: go(helm_op_kernel<1>); break;
-        case 2: go(helm_op_kernel<2>); break;
-        case 3: go(helm_op_kernel<3>); break;
-        default: go(helm_op_kernel<4>); break;
-    }
+    helm_extent(nb, [&](auto nbc) {
+        constexpr int N = decltype(nbc)::value;
+        auto go = [&](auto kfn) {
+            kfn<<<dim3(n_blocks, helm_chunks((long long)n_modes * nb * nb)), 256, 0, c.stream>>>(
+                nb, n_modes, in_comp, out_comp, dx, lz, scale, mask, dev_src, dev_dst);
+        };
+        switch (op)
+        {
+            case 0: go(helm_op_kernel<0, N>); break;
+            case 1: go(helm_op_kernel<1, N>); break;
+            case 2: go(helm_op_kernel<2, N>); break;
+            case 3: go(helm_op_kernel<3, N>); break;
+            default: go(helm_op_kernel<4, N>); break;
+        }
+    });
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }
@@ -517,7 +584,11 @@ void helm2d_nonlinear(Ctx& c, int nb, int n_blocks, int n_planes, const unsigned
     check_block_extent(nb, 3ll * n_planes);
     const UnitMask mask = unit_mask(n_planes, host_plane_mask);
     if (!n_blocks) return;
-    helm_nonlinear_kernel<<<n_blocks, 256, 0, c.stream>>>(nb, n_planes, mask, dev_face, dev_edge, dev_dst);
+    helm_extent(nb, [&](auto nbc) {
+        helm_nonlinear_kernel<decltype(nbc)::value>
+            <<<dim3(n_blocks, helm_chunks((long long)n_planes * nb * nb)), 256, 0, c.stream>>>(
+                nb, n_planes, mask, dev_face, dev_edge, dev_dst);
+    });
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }

@@ -1,10 +1,18 @@
 """Block kernels over the block extents and the edges of their work splits,
-against the oracle."""
+against the oracle: sweeps with partly present sibling groups, the integrating
+factor's truncation radii, the single-block convolution, and the Fourier-in-z
+operators at extents without a compile-time form."""
+import os
+import sys
+
 import numpy as np
 import pytest
 
 import iblgf_b200 as B
 import oracle_lib as O
+
+sys.path.insert(0, os.path.join(os.path.dirname(__file__), "..", "oracle"))
+import helm2d as H  # noqa: E402
 
 pytestmark = pytest.mark.gpu
 
@@ -74,3 +82,22 @@ def test_conv_block_extents(e, precision, tol):
         g.conv_block(ts.data_ptr(), tk.data_ptr(), out.data_ptr(), 0.5)
         ref = O.block_conv(src, ker, 0.5).ravel(order="F")
         assert rel_linf(out.cpu().numpy() - base, ref) < tol
+
+
+@pytest.mark.parametrize("nb,nm", [(3, 1), (7, 5), (18, 7), (40, 3)])
+@pytest.mark.parametrize("op", ["laplace", "gradient", "divergence", "curl", "curl_transpose"])
+def test_fourier_operators_extents(op, nb, nm):
+    """Extents with and without a compile-time form, from less than a CTA's work to several CTAs per block."""
+    import torch
+    g = B.Solver((-12,) * 3, (24,) * 3, 6, 1.0, [((-6,) * 3, (12,) * 3)])
+    rng = np.random.default_rng(nb)
+    sep = 2 * nm
+    cin = sep if op in ("laplace", "gradient") else 3 * sep
+    cout = sep if op in ("laplace", "divergence") else 3 * sep
+    src, dst = rng.standard_normal((2, cin, nb, nb)), rng.standard_normal((2, cout, nb, nb))
+    ref = H.helm_op(op, src, dst.copy(), nm, 0.25, 1.5, 0.6)
+    s, d = torch.tensor(src, device="cuda"), torch.tensor(dst, device="cuda")
+    torch.cuda.synchronize()
+    g.helm2d_op(op, s, d, nm, 0.25, 1.5, 0.6)
+    g.synchronize()
+    assert np.abs(d.cpu().numpy() - ref).max() < 1e-13 * np.abs(ref).max()
