@@ -166,6 +166,8 @@ __global__ void helm2d_apply_kernel(int nx, int ny, const double* __restrict__ t
 // curl_transpose 182 -> 130, gradient 116 -> 109, divergence 96 -> 63, laplace
 // 74 -> 36, nonlinear (48 planes) 277 -> 228, where one pass over the operands
 // takes 78, 78, 52, 52, 26 and 175.
+constexpr int kHelmItems = 4;
+
 template<int OP, int NBT>
 __global__ void __launch_bounds__(256) helm_op_kernel(int nb_, int n_modes, int in_comp, int out_comp, double dx,
                                                       double lz, double scale, UnitMask mask,
