@@ -624,17 +624,16 @@ void build_tc_tiles(const std::vector<int>& tgptr, const std::vector<int>& ttab,
 void check_status(Ctx& c);
 // inverse transforms assigned to the plan's target blocks
 void launch_inverse_targets(Ctx& c, const FmmPlan& p, const void* acc, double* fmm_t, double scale);
-// prime-factor inverse (inverse.cu); false when the block size has no
-// prime-factor split (the direct inverse runs instead)
-bool inverse_pfa(Ctx& c, const void* acc, const int* d_tgt_oct, int n, double scale, double* target,
-                 bool fp32_passes, bool assign);
+// prime-factor transforms (inverse.cu) of the block extents whose P splits;
+// the direct transforms run for the others
+constexpr bool pfa_extent(int nb) { return nb == 8 || nb == 18; }
+void inverse_pfa(Ctx& c, const void* acc, const int* d_tgt_oct, int n, double scale, double* target, bool assign);
+void forward_pfa(Ctx& c, const double* field, const int* d_item_oct, int n, void* spec);
 void init_pfa_constants(int device);
 // sharding (solver.cpp): the reference server's load-balanced partition and
 // this context's share of it
 std::vector<int> domain_partition(const Ctx& c, int n);
 void domain_set_owner(Ctx& c, const int* owner, int rank, iblgf_exchange_fn fn, void* user);
-// whether the prime-factor inverse runs its z and y passes in FP32
-bool inverse_fp32_passes(const Ctx& c);
 void launch_zero_blocks(Ctx& c, double* f, const int* list, int n);
 void launch_fill_zero(Ctx& c, double* p, size_t n);
 void launch_remap_blocks(Ctx& c, const double* old, double* nw, const int* d_src, int n_new);

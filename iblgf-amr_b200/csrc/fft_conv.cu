@@ -6,12 +6,13 @@
 // block, scaled by dx^2 / P^3.
 //
 // B200 structure (one sweep = all blocks of all tree levels at once):
-//   fwd_xy_rows  one CTA per source block: thread (z, y) transforms row y
-//                along x (real, Nb -> Nb half frequencies), thread (z, kx)
-//                then column kx along y (Nb -> P)
-//   fwd_z        one thread per (ky,kx) pencil: z transform (Nb -> P)
-//                Each source block is transformed once per sweep; the
-//                reference transforms it once per (source, target) pair.
+//   forward      each source block once per sweep (the reference transforms it
+//                once per (source, target) pair): one kernel for the extents
+//                with a prime-factor split (inverse.cu), two for the others:
+//     fwd_xy_rows  one CTA per source block: thread (z, y) transforms row y
+//                  along x (real, Nb -> Nb half frequencies), thread (z, kx)
+//                  then column kx along y (Nb -> P)
+//     fwd_z        one thread per (ky,kx) pencil: z transform (Nb -> P)
 //   group_mac    sibling-group spectral multiply-accumulate (mac_kernel:
 //                general pair-list fallback)
 //   inv_fused    one CTA per (target, half of the output planes): z inverse,
@@ -749,6 +750,11 @@ __global__ void __launch_bounds__(NB * NB, 2) inv_fused_kernel(const cx<RA>* __r
     for (int i = 0; i < ZH; ++i) out[i] = assign ? scale * (y0 + 2.0 * sx[i]) : out[i] + scale * (y0 + 2.0 * sx[i]);
 }
 
+void ensure(DevBuf<char>& b, size_t bytes)
+{
+    if (b.n < bytes) b.alloc(bytes);
+}
+
 template<class R, int NB>
 struct Conv
 {
@@ -777,10 +783,15 @@ struct Conv
     static void forward_field(Ctx& c, const double* field, const int* d_item_oct, int n, void* spec)
     {
         if (!n) return;
-        cx<R>* W = (cx<R>*)c.d_w.p;
-        launch_fwd_xy_rows(c, field, d_item_oct, n, W);
-        fwd_z_kernel<R, R, NB, NB><<<dim3(n, (NP + 127) / 128), 128, 0, c.stream>>>(W, nullptr, (cx<R>*)spec);
-        c.launches += 2;
+        if constexpr (pfa_extent(NB)) forward_pfa(c, field, d_item_oct, n, spec);
+        else
+        {
+            ensure(c.d_w, (size_t)n * NB * NP * sizeof(cx<R>));
+            cx<R>* W = (cx<R>*)c.d_w.p;
+            launch_fwd_xy_rows(c, field, d_item_oct, n, W);
+            fwd_z_kernel<R, R, NB, NB><<<dim3(n, (NP + 127) / 128), 128, 0, c.stream>>>(W, nullptr, (cx<R>*)spec);
+            c.launches += 2;
+        }
     }
 
     // LGF blocks are transformed in FP64 and stored in R
@@ -857,9 +868,12 @@ struct Conv
                         bool assign)
     {
         if (!n_tgt) return;
-        if (inverse_pfa(c, acc, d_tgt_oct, n_tgt, scale, target, inverse_fp32_passes(c), assign)) return;
-        launch_inverse(c, (const cx<R>*)acc, d_tgt_oct, n_tgt, scale, target, assign);
-        c.launches += 1;
+        if constexpr (pfa_extent(NB)) inverse_pfa(c, acc, d_tgt_oct, n_tgt, scale, target, assign);
+        else
+        {
+            launch_inverse(c, (const cx<R>*)acc, d_tgt_oct, n_tgt, scale, target, assign);
+            c.launches += 1;
+        }
     }
 };
 
@@ -885,10 +899,6 @@ void dispatch(Ctx& c, F&& f)
 #undef IBLGF_CASE
 }
 
-void ensure(DevBuf<char>& b, size_t bytes)
-{
-    if (b.n < bytes) b.alloc(bytes);
-}
 }  // namespace
 
 bool nb_supported(int Nb) { return Nb == 6 || Nb == 8 || Nb == 10 || Nb == 12 || Nb == 16 || Nb == 18; }
@@ -949,7 +959,6 @@ void launch_spectra(Ctx& c, const std::vector<std::array<int, 5>>& new_slots)
 
 void launch_forward_sources(Ctx& c, const double* fmm_s, const int* d_src_oct, int n_src, void* src_spec)
 {
-    ensure(c.d_w, (size_t)n_src * c.Nb * c.P * c.Nb * c.cplx_bytes());
     dispatch(c, [&](auto cv) {
         using CV = decltype(cv);
         CV::forward_field(c, fmm_s, d_src_oct, n_src, src_spec);

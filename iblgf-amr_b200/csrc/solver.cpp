@@ -268,8 +268,6 @@ void domain_set_owner(Ctx& c, const int* owner, int rank, iblgf_exchange_fn fn, 
     c.plans.clear();
 }
 
-bool inverse_fp32_passes(const Ctx& c) { return c.cfg.precision == IBLGF_FP32; }
-
 void check_status(Ctx& c)
 {
     if (!c.d_status.p) return;
