@@ -7,17 +7,24 @@
 //                 coarsification (interpolation/cell_center_nli_intrp.hpp:
 //                 310-420, 557-674). One CTA per receiving block; the sending
 //                 blocks of a group are applied in child order, so sums are
-//                 deterministic without atomics.
+//                 deterministic without atomics. tp_antrp_kernel: anterpolation
+//                 to few blocks, a cluster of eight CTAs each; tp_band2_kernel:
+//                 coarsification by width-2 bands, a thread per node
 //   halo_kernel   same-level buffer exchange (domain/mpi/haloCommunicator.hpp:
 //                 63-107): each buffer cell takes the value of the neighbour
 //                 interior cell that overlaps it
 //   correction    add_source_correction (cell_center_nli_intrp.hpp:171-238)
 //   zero / copy_interior / axpy over block lists (fmm.hpp:1029-1106,
-//                 poisson.hpp:921-1013)
+//                 poisson.hpp:921-1013); solve_begin, sweep_begin: those that
+//                 start a solve and a sweep, in one launch each
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstring>
 
 #include "ctx.hpp"
+
+namespace cg = cooperative_groups;
 
 namespace iblgf_b200
 {
@@ -28,16 +35,39 @@ namespace
 // unrolled every matrix entry is an FMA operand at a fixed offset (no
 // shared-memory loads). Face and edge components use one of two sets per axis
 // (their relative positions 0 and 1); set[c][a] is that of component c and
-// axis a. Dense transfers have one set.
+// axis a.
 // lo: for the banded passes (W > 0), first column of row m's band of width W
-// in summation order (the row's nonzeros all lie in [lo, lo + W))
+// in summation order (the row's nonzeros all lie in [lo, lo + W)); w5: the
+// entries of the bands of width 5
 template<int NB, class T>
 struct TpMats
 {
     T m[2][2][NB * NB];
+    T w5[2][2][NB][5];
     unsigned char lo[2][2][NB];
     unsigned char set[3][3];
 };
+
+// Pencils in shared memory: NB values at an odd row stride, so that the lanes
+// of a warp, each in its own pencil, read without bank conflicts.
+template<int NB>
+constexpr int tp_stride()
+{
+    return NB | 1;
+}
+// bytes of one block there
+template<int NB, class T>
+constexpr size_t tp_bytes()
+{
+    return (size_t)NB * NB * tp_stride<NB>() * sizeof(T);
+}
+// place of entry m of the pass's output for pencil p = (z, y): with the axes
+// rotated ([z][y][x] -> [x][z][y]) it is entry y of pencil (m, z)
+template<int NB>
+__device__ __forceinline__ int tp_out(int m, int p)
+{
+    return (m * NB + p / NB) * tp_stride<NB>() + p % NB;
+}
 
 // the component fields of one transfer (blockIdx.y = component)
 struct TpFields
@@ -52,19 +82,21 @@ constexpr int tp_threads()
     return (NB * NB + 31) / 32 * 32;
 }
 
-// One pass along the fastest axis of `in`: thread p owns the pencil
-// in[p*NB + n] and writes out[m*NB^2 + p] = sum_n T(m,n) in[p*NB + n] with
-// T(m,n) = M_K(m,n) (anterpolation) or M_K(n,m) (interpolation). Writing the
-// result with the axes rotated ([z][y][x] -> [x][z][y]) makes the next axis
-// the fastest one, so all three passes read contiguous pencils; after three
-// passes the layout is back to [z][y][x]. The last pass adds into the
+// One pass along the fastest axis of `in`: thread p owns pencil p and forms
+// sum_n T(m,n) in[p][n] with T(m,n) = M_K(m,n) (anterpolation) or M_K(n,m)
+// (interpolation). Writing the result with the axes rotated makes the next
+// axis the fastest one, so all three passes read contiguous pencils; after
+// three passes the layout is back to [z][y][x]. The last pass adds into the
 // thread's accumulators instead of writing shared memory.
 // W > 0: only the W entries of row m's band [lo, lo + W) are summed, in
 // the same order; the skipped entries are zeros, whose FMAs leave the running
-// sum unchanged, so the result equals the full row's
+// sum unchanged, so the result equals the full row's. At W = 5 the bands move
+// on by at most one column per row, so a window of five values in registers
+// takes one shared-memory load per move instead of five per row (the
+// cell-centred interpolation of three levels at extent 16: 760 -> 497 us).
 // T: arithmetic and shared-memory type of the passes (the accumulators acc,
 // which start from and end in the FP64 target block, stay FP64)
-template<int NB, int K, bool TR, bool LAST, int W, class T>
+template<int NB, int K, bool TR, bool LAST, int W, class T, bool MULTI>
 __device__ __forceinline__ void tp_pass(const T* __restrict__ in, T* __restrict__ out,
                                         const TpMats<NB, T>& mt, int set, int p, double* acc)
 {
@@ -72,20 +104,49 @@ __device__ __forceinline__ void tp_pass(const T* __restrict__ in, T* __restrict_
     {
         T v[NB];
 #pragma unroll
-        for (int n = 0; n < NB; ++n) v[n] = in[p * NB + n];
+        for (int n = 0; n < NB; ++n) v[n] = in[p * tp_stride<NB>() + n];
 #pragma unroll
         for (int m = 0; m < NB; ++m)
         {
             T s = 0;
 #pragma unroll
-            for (int n = 0; n < NB; ++n) s = fma(TR ? mt.m[0][K][n * NB + m] : mt.m[0][K][m * NB + n], v[n], s);
+            for (int n = 0; n < NB; ++n)
+            {
+                // one set: entries at fixed places of the constant bank
+                const T* mat = mt.m[MULTI ? set : 0][K];
+                s = fma(TR ? mat[n * NB + m] : mat[m * NB + n], v[n], s);
+            }
             if (LAST) acc[m] += s;
-            else out[m * NB * NB + p] = s;
+            else out[tp_out<NB>(m, p)] = s;
+        }
+    }
+    else if constexpr (W == 5)
+    {
+        const T* row = in + p * tp_stride<NB>();
+        int cur = mt.lo[set][K][0];
+        T v[5];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) v[j] = row[cur + j];
+#pragma unroll
+        for (int m = 0; m < NB; ++m)
+        {
+            if (m && mt.lo[set][K][m] != cur)
+            {
+                ++cur;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] = v[j + 1];
+                v[4] = row[cur + 4];
+            }
+            T s = 0;
+#pragma unroll
+            for (int j = 0; j < 5; ++j) s = fma(mt.w5[set][K][m][j], v[j], s);
+            if (LAST) acc[m] += s;
+            else out[tp_out<NB>(m, p)] = s;
         }
     }
     else
     {
-        const T* row = in + p * NB;
+        const T* row = in + p * tp_stride<NB>();
         const T* mat = mt.m[set][K];
 #pragma unroll
         for (int m = 0; m < NB; ++m)
@@ -99,17 +160,31 @@ __device__ __forceinline__ void tp_pass(const T* __restrict__ in, T* __restrict_
                 s = fma(TR ? mat[n * NB + m] : mat[m * NB + n], row[n], s);
             }
             if (LAST) acc[m] += s;
-            else out[m * NB * NB + p] = s;
+            else out[tp_out<NB>(m, p)] = s;
         }
     }
 }
 
-template<int NB, bool TR, bool LAST, int W, class T>
+// a block into shared-memory pencils
+template<int NB, class T>
+__device__ __forceinline__ void tp_stage(const double* __restrict__ block, T* __restrict__ a)
+{
+    const double2* s2 = reinterpret_cast<const double2*>(block);
+    for (int i = threadIdx.x; i < NB * NB * NB / 2; i += blockDim.x)
+    {
+        const double2 v = s2[i];
+        const int at = 2 * i / NB * tp_stride<NB>() + 2 * i % NB;  // NB is even: both in one pencil
+        a[at] = (T)v.x;
+        a[at + 1] = (T)v.y;
+    }
+}
+
+template<int NB, bool TR, bool LAST, int W, class T, bool MULTI = false>
 __device__ __forceinline__ void tp_pass_bit(int bit, const T* in, T* out, const TpMats<NB, T>& mt, int set, int p,
                                             double* acc)
 {
-    if (bit) tp_pass<NB, 1, TR, LAST, W, T>(in, out, mt, set, p, acc);
-    else tp_pass<NB, 0, TR, LAST, W, T>(in, out, mt, set, p, acc);
+    if (bit) tp_pass<NB, 1, TR, LAST, W, T, MULTI>(in, out, mt, set, p, acc);
+    else tp_pass<NB, 0, TR, LAST, W, T, MULTI>(in, out, mt, set, p, acc);
 }
 
 // mode 0: dst[group] += sum_tasks A(src)        (anterpolation / coarsify)
@@ -117,7 +192,7 @@ __device__ __forceinline__ void tp_pass_bit(int bit, const T* in, T* out, const 
 // mode 2: dst[group]  = I(src)                  (cell-centred interpolation)
 // One CTA per receiving block, one thread per pencil; the sending blocks of
 // a group are applied in child order into per-thread accumulators.
-template<int NB, bool TR, int W, class T>
+template<int NB, bool TR, int W, class T, bool MULTI = false>
 __global__ void __launch_bounds__(tp_threads<NB>(), 2) tp_kernel(
     const int* __restrict__ gptr, const int* __restrict__ gdst, const int* __restrict__ tsrc,
     const int* __restrict__ tcid, const __grid_constant__ TpFields f, const __grid_constant__ TpMats<NB, T> mt, int mode)
@@ -128,7 +203,7 @@ __global__ void __launch_bounds__(tp_threads<NB>(), 2) tp_kernel(
     const unsigned char* set = mt.set[blockIdx.y];
     extern __shared__ __align__(16) unsigned char tp_smem[];
     T* a = reinterpret_cast<T*>(tp_smem);
-    T* b = a + N3;
+    T* b = a + NB * NB * tp_stride<NB>();
     const int g = blockIdx.x;
     const int p = threadIdx.x;
     const bool active = p < NB * NB;
@@ -139,25 +214,73 @@ __global__ void __launch_bounds__(tp_threads<NB>(), 2) tp_kernel(
     for (int m = 0; m < NB; ++m) acc[m] = (active && mode != 2) ? d[m * NB * NB] : 0.0;
     for (int t = gptr[g]; t < gptr[g + 1]; ++t)
     {
-        const double2* s2 = reinterpret_cast<const double2*>(src + (size_t)tsrc[t] * N3);
         const int cid = tcid[t];
-        for (int i = threadIdx.x; i < N3 / 2; i += blockDim.x)
-        {
-            const double2 v = s2[i];
-            a[2 * i] = (T)v.x;
-            a[2 * i + 1] = (T)v.y;
-        }
+        tp_stage<NB, T>(src + (size_t)tsrc[t] * N3, a);
         __syncthreads();
-        if (active) tp_pass_bit<NB, TR, false, W, T>(cid & 1, a, b, mt, set[0], p, acc);
+        if (active) tp_pass_bit<NB, TR, false, W, T, MULTI>(cid & 1, a, b, mt, set[0], p, acc);
         __syncthreads();
-        if (active) tp_pass_bit<NB, TR, false, W, T>((cid >> 1) & 1, b, a, mt, set[1], p, acc);
+        if (active) tp_pass_bit<NB, TR, false, W, T, MULTI>((cid >> 1) & 1, b, a, mt, set[1], p, acc);
         __syncthreads();
-        if (active) tp_pass_bit<NB, TR, true, W, T>((cid >> 2) & 1, a, (T*)nullptr, mt, set[2], p, acc);
+        if (active) tp_pass_bit<NB, TR, true, W, T, MULTI>((cid >> 2) & 1, a, (T*)nullptr, mt, set[2], p, acc);
         __syncthreads();
     }
     if (!active) return;
 #pragma unroll
     for (int m = 0; m < NB; ++m) d[m * NB * NB] = acc[m];
+}
+
+// Dense anterpolation (mode 0): dst[group] += sum_tasks A(src). A cluster of
+// eight CTAs per receiving block, one per sending child: each runs its three
+// passes into its own shared memory, then takes an eighth of the receiving
+// block and adds the children's results, read through distributed shared
+// memory, in child order (the order and the roundings of one CTA that walks
+// the children). For the coarse levels with few receiving blocks, where eight
+// children in sequence are 24 barrier-separated passes on a few SMs: 22 against
+// 45 us at 44 blocks of 18^3 in FP32, 16 against 28 at 8; with more blocks than
+// kAntrpClusters the chip is full either way and the barriers of the cluster
+// cost more (106 blocks: 44 / 46 us, 184: 73 / 67, 1161: 382 / 202).
+constexpr int kAntrpClusters = 120;
+
+template<int NB, class T>
+__global__ void __cluster_dims__(8, 1, 1) __launch_bounds__(tp_threads<NB>(), 2) tp_antrp_kernel(
+    const int* __restrict__ gptr, const int* __restrict__ gdst, const int* __restrict__ tsrc,
+    const int* __restrict__ tcid, const __grid_constant__ TpFields f, const __grid_constant__ TpMats<NB, T> mt)
+{
+    constexpr int N3 = NB * NB * NB;
+    extern __shared__ __align__(16) unsigned char tp_smem[];
+    T* a = reinterpret_cast<T*>(tp_smem);
+    T* b = a + NB * NB * tp_stride<NB>();
+    cg::cluster_group cluster = cg::this_cluster();
+    const int g = blockIdx.x / 8, r = (int)cluster.block_rank();
+    const int t0 = gptr[g], n = gptr[g + 1] - t0;
+    const int p = threadIdx.x;
+    const bool active = p < NB * NB;
+    if (r < n)
+    {
+        const int cid = tcid[t0 + r];
+        tp_stage<NB, T>(f.src[blockIdx.y] + (size_t)tsrc[t0 + r] * N3, a);
+        __syncthreads();
+        if (active) tp_pass_bit<NB, false, false, 0, T>(cid & 1, a, b, mt, 0, p, nullptr);
+        __syncthreads();
+        if (active) tp_pass_bit<NB, false, false, 0, T>((cid >> 1) & 1, b, a, mt, 0, p, nullptr);
+        __syncthreads();
+        if (active) tp_pass_bit<NB, false, false, 0, T>((cid >> 2) & 1, a, b, mt, 0, p, nullptr);
+    }
+    cluster.sync();
+    double* d = f.dst[blockIdx.y] + (size_t)gdst[g] * N3;
+    const T* part[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) part[k] = cluster.map_shared_rank(b, k);
+    for (int i = N3 / 8 * r + threadIdx.x; i < N3 / 8 * (r + 1); i += blockDim.x)
+    {
+        double acc = d[i];
+        const int at = i / NB * tp_stride<NB>() + i % NB;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (k < n) acc += (double)part[k][at];
+        d[i] = acc;
+    }
+    cluster.sync();  // the others have read this CTA's result
 }
 
 // Width-2 band (mode 0, coarsening): each receiving node takes 2 x 2 x 2 nodes
@@ -542,13 +665,37 @@ void launch_tp_typed(Ctx& c, const TpTasks& t, const TpFields& f, int n, const i
                     width = std::max(width, lo < hi ? hi - lo : 0);
                 }
         }
-    const int W = width <= 2 ? 2 : (width <= 5 ? 5 : 0);
-    if (!W && base[1] >= 0) throw Error(IBLGF_EINTERNAL, "dense transfers have one matrix set");
-    if (W)
+    int W = width <= 2 ? 2 : (width <= 5 ? 5 : 0);
+    if (W == 5)
+    {
+        // the smallest starts that never move back and cover the rows; they move
+        // on by one column at most (checked, else the dense form)
+        unsigned char start[2][2][NB] = {};
+        for (int s = 0; s < 2 && base[s] >= 0; ++s)
+            for (int k = 0; k < 2; ++k)
+                for (int m = 0, st = 0; m < NB; ++m)
+                {
+                    int lo = NB, hi = 0;
+                    for (int i = 0; i < NB; ++i)
+                        if ((tr ? mt.m[s][k][i * NB + m] : mt.m[s][k][m * NB + i]) != (T)0)
+                        {
+                            lo = std::min(lo, i);
+                            hi = i + 1;
+                        }
+                    const int prev = st;
+                    st = std::max(st, hi - 5);
+                    if (st > lo || (m && st > prev + 1)) W = 0;
+                    start[s][k][m] = (unsigned char)st;
+                    for (int j = 0; j < 5; ++j)
+                        mt.w5[s][k][m][j] = tr ? mt.m[s][k][(st + j) * NB + m] : mt.m[s][k][m * NB + st + j];
+                }
+        if (W == 5) std::memcpy(mt.lo, start, sizeof(mt.lo));
+    }
+    if (W == 2)
         for (int s = 0; s < 2; ++s)
             for (int k = 0; k < 2; ++k)
                 for (int m = 0; m < NB; ++m) mt.lo[s][k][m] = (unsigned char)std::min<int>(mt.lo[s][k][m], NB - W);
-    const size_t smem = 2 * (size_t)NB * NB * NB * sizeof(T);
+    const size_t smem = 2 * tp_bytes<NB, T>();
     auto launch = [&](auto kfn) {
         IBLGF_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         kfn<<<dim3(t.n_groups, n), tp_threads<NB>(), smem, c.stream>>>(t.group_ptr.p, t.group_dst.p, t.task_src.p,
@@ -564,12 +711,22 @@ void launch_tp_typed(Ctx& c, const TpTasks& t, const TpFields& f, int n, const i
                 t.group_ptr.p, t.group_dst.p, t.task_src.p, t.task_cid.p, f, mt);
         }
         else if (W == 5) launch(tp_kernel<NB, false, 5, T>);
-        else launch(tp_kernel<NB, false, 0, T>);
+        else if (base[1] >= 0) throw Error(IBLGF_EINTERNAL, "anterpolation has one matrix set");
+        else if (t.n_groups * n > kAntrpClusters) launch(tp_kernel<NB, false, 0, T>);
+        else
+        {
+            static_assert((NB * NB * NB) % 8 == 0, "eight CTAs share a receiving block");
+            auto kfn = tp_antrp_kernel<NB, T>;
+            IBLGF_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            kfn<<<dim3(8 * t.n_groups, n), tp_threads<NB>(), smem, c.stream>>>(
+                t.group_ptr.p, t.group_dst.p, t.task_src.p, t.task_cid.p, f, mt);
+        }
     }
     else
     {
         if (W == 2) launch(tp_kernel<NB, true, 2, T>);
         else if (W == 5) launch(tp_kernel<NB, true, 5, T>);
+        else if (base[1] >= 0) launch(tp_kernel<NB, true, 0, T, true>);  // interpolation orders above 5
         else launch(tp_kernel<NB, true, 0, T>);
     }
 }
