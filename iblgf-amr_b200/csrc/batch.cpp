@@ -312,10 +312,8 @@ void batch_apply_lgf(Ctx& c, int src, int tgt)
         const double dx_level = c.cfg.dx_base / std::pow(2.0, r);
         if (!c.subtract_non_leaf)
         {
-            run_sweep(c, batch_plan(c, b, r, true), c.f_source_tmp, c.f_target_tmp, dx_level, 1.0, -1);
-            launch_tp(c, b.cc_intrp[r], tt, tt, 2, 2);
-            run_sweep(c, batch_plan(c, b, r, false), c.f_source_tmp, c.f_target_tmp, dx_level, 1.0, -1);
-            launch_axpy_blocks(c, tt, c.field(tgt), b.level_leaves[r].p, (int)b.level_leaves[r].n, 1.0, true);
+            run_level(c, batch_plan(c, b, r, true), batch_plan(c, b, r, false), dx_level, b.level_leaves[r],
+                      c.field(tgt), [&]() { launch_tp(c, b.cc_intrp[r], tt, tt, 2, 2); });
         }
         if (!c.use_correction || !b.corr_all[r].n) continue;
         launch_halo(c, st, b.corr_all[r].p, (int)b.corr_all[r].n);

@@ -179,6 +179,7 @@ struct FmmPlan
     // inverse transform assigns zeroed (2)
     DevBuf<int> begin;
     DevBuf<int> add_t;
+    size_t n_add_leaves = 0;  // leaf blocks in add_t
     std::vector<TpTasks> antrp;  // levels level-1 .. 0
     std::vector<TpTasks> intrp;  // levels 1 .. level-1
     int n_src = 0, n_tgt = 0;
@@ -456,7 +457,14 @@ int field_create(Ctx& c);
 void fmm_apply(Ctx& c, int src, int tgt, int level, bool nlas, double scale, int fmm_type, int ge = -1);
 // one FMM sweep of a ready plan: zero / copy / anterpolate, forward transforms,
 // MAC, inverse transforms + add, interpolate, add into tgt (fmm.hpp:729-870)
-void run_sweep(Ctx& c, FmmPlan& p, int src, int tgt, double dx_level, double add_with_scale, int ge);
+// leaf_out: takes the targets' values on leaf blocks as well
+void run_sweep(Ctx& c, FmmPlan& p, int src, int tgt, double dx_level, double add_with_scale, int ge,
+               double* leaf_out = nullptr);
+// the two sweeps of a level of apply_lgf (non-leaf as source, then not, with
+// `between` run between them) into target_tmp, whose leaves go to out; the
+// level's leaves are listed
+void run_level(Ctx& c, FmmPlan& all, FmmPlan& rest, double dx_level, const DevBuf<int>& leaves, double* out,
+               const std::function<void()>& between);
 // direct_only: a neighbour-only plan for the direct separable sweep (target
 // and neighbour lists only; no pair lists, groups or spectra)
 HostPlan build_host_plan(const Ctx& c, int level, int idx, int ge, bool direct_only = false);
@@ -650,8 +658,9 @@ void field_download_leaves_async(Ctx& c, int f, double* host, size_t count);
 void copy_stream_release(Ctx& c);
 void field_upload_leaves_async(Ctx& c, int f, const double* host, size_t count);
 void launch_copy_interior(Ctx& c, const double* src, double* dst, const int* list, int n);
+// leaf_out: a field that takes the results on leaf blocks as well
 void launch_axpy_blocks(Ctx& c, const double* src, double* dst, const int* list, int n, double a,
-                        bool assign);
+                        bool assign, double* leaf_out = nullptr);
 // fp32: the three passes in FP32, the sum into the FP64 receiving block in FP64
 void launch_tp(Ctx& c, const TpTasks& t, const double* src, double* dst, int mat_base,
                int mode /*0 antrp add, 1 intrp add, 2 intrp assign*/, bool fp32 = false);

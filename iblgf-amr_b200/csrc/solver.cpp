@@ -1030,6 +1030,7 @@ std::unique_ptr<FmmPlan> upload_plan(Ctx& c, const HostPlan& h)
         IBLGF_CUDA(cudaStreamSynchronize(c.stream));  // the host array goes out of scope
     }
     p.add_t.upload(h.at, c.stream);
+    for (int o : h.at) p.n_add_leaves += c.flags[o] & 1;
     for (auto& t : h.antrp)
     {
         p.antrp.emplace_back();
@@ -1320,7 +1321,7 @@ void fmm_apply(Ctx& c, int src, int tgt, int level, bool nlas, double add_with_s
     run_sweep(c, p, src, tgt, c.cfg.dx_base / std::pow(2.0, rl), add_with_scale, ge);
 }
 
-void run_sweep(Ctx& c, FmmPlan& p, int src, int tgt, double dx_level, double add_with_scale, int ge)
+void run_sweep(Ctx& c, FmmPlan& p, int src, int tgt, double dx_level, double add_with_scale, int ge, double* leaf_out)
 {
     c.stats[0] += 1;
     c.stats[1] += p.n_src;
@@ -1332,6 +1333,9 @@ void run_sweep(Ctx& c, FmmPlan& p, int src, int tgt, double dx_level, double add
     c.stats[7] += p.n_tgt - p.n_csr_tgt;
     c.stats[9] += p.mac_flops;
     c.stats[8] += p.n_exec;
+    // without a source the targets would take zeros (sharded: the exchange is
+    // called for every sweep)
+    if (!p.n_src && !leaf_out && c.owner.empty()) return;
     double* fs = c.field(c.f_fmm_s);
     double* ft = c.field(c.f_fmm_t);
     Timer tm(c);
@@ -1392,8 +1396,23 @@ void run_sweep(Ctx& c, FmmPlan& p, int src, int tgt, double dx_level, double add
             throw Error(IBLGF_EINTERNAL, "the exchange callback failed");
         launch_blocks_scatter(c, c.exchange_buf.p, ft, p.add_t.p, (int)p.add_t.n);
     }
-    launch_axpy_blocks(c, ft, c.field(tgt), p.add_t.p, (int)p.add_t.n, add_with_scale, false);
+    launch_axpy_blocks(c, ft, c.field(tgt), p.add_t.p, (int)p.add_t.n, add_with_scale, false, leaf_out);
     tm.mark(4);
+}
+
+void run_level(Ctx& c, FmmPlan& all, FmmPlan& rest, double dx_level, const DevBuf<int>& leaves, double* out,
+               const std::function<void()>& between)
+{
+    // the last sweep that has sources writes the leaves on its way where its
+    // targets hold them all
+    const int st = c.f_source_tmp, tt = c.f_target_tmp;
+    const bool second = rest.n_src || !c.owner.empty();
+    FmmPlan& last = second ? rest : all;
+    const bool fused = last.n_add_leaves == leaves.n && (last.n_src || !c.owner.empty());
+    run_sweep(c, all, st, tt, dx_level, 1.0, -1, fused && !second ? out : nullptr);
+    between();
+    run_sweep(c, rest, st, tt, dx_level, 1.0, -1, fused && second ? out : nullptr);
+    if (!fused) launch_axpy_blocks(c, c.field(tt), out, leaves.p, (int)leaves.n, 1.0, true);
 }
 
 // --------------------------------------------------------------- Poisson
@@ -1846,10 +1865,11 @@ void poisson_apply_lgf(Ctx& c, int src, int tgt, int fmm_type)
     {
         if (!c.subtract_non_leaf)
         {
-            fmm_apply(c, c.f_source_tmp, c.f_target_tmp, l, true, 1.0, IBLGF_AMR2AMR);
-            launch_tp(c, pl.cc_intrp[l], tt, tt, 2, 2);
-            fmm_apply(c, c.f_source_tmp, c.f_target_tmp, l, false, 1.0, IBLGF_AMR2AMR);
-            launch_axpy_blocks(c, tt, c.field(tgt), pl.level_leaves[l].p, (int)pl.level_leaves[l].n, 1.0, true);
+            const int rl = l - bl;
+            FmmPlan& all = get_plan(c, l, mask_idx_gen(IBLGF_AMR2AMR, rl, 1), -1);
+            FmmPlan& rest = get_plan(c, l, mask_idx_gen(IBLGF_AMR2AMR, rl, 0), -1);
+            run_level(c, all, rest, c.cfg.dx_base / std::pow(2.0, rl), pl.level_leaves[l], c.field(tgt),
+                      [&]() { launch_tp(c, pl.cc_intrp[l], tt, tt, 2, 2); });
         }
         if (!c.use_correction || l == depth - 1) continue;
         launch_halo(c, st, pl.level_all[l].p, (int)pl.level_all[l].n);

@@ -555,10 +555,14 @@ __global__ void __launch_bounds__(256) sweep_begin_kernel(const int* __restrict_
     }
 }
 
+// d = a s (assign) or d += a s on the listed blocks; leaf blocks' results also
+// to leaf_out (if given)
 __global__ void __launch_bounds__(256) axpy_kernel(const double2* __restrict__ s, double2* __restrict__ d,
-                                                   const int* __restrict__ list, int half, double a, int assign)
+                                                   const int* __restrict__ list, int half, double a, int assign,
+                                                   const int* __restrict__ flags, double2* __restrict__ leaf_out)
 {
     const size_t off = (size_t)list[blockIdx.x] * half;
+    const bool leaf = leaf_out && (flags[list[blockIdx.x]] & 1);
     double2 v[kPairs], w[kPairs];
 #pragma unroll
     for (int k = 0; k < kPairs; ++k)
@@ -572,8 +576,10 @@ __global__ void __launch_bounds__(256) axpy_kernel(const double2* __restrict__ s
     {
         const int i = blockIdx.y * kPiece + 256 * k + threadIdx.x;
         if (i >= half) break;
-        if (assign) d[off + i] = make_double2(a * v[k].x, a * v[k].y);
-        else d[off + i] = make_double2(w[k].x + v[k].x * a, w[k].y + v[k].y * a);
+        const double2 r = assign ? make_double2(a * v[k].x, a * v[k].y)
+                                 : make_double2(w[k].x + v[k].x * a, w[k].y + v[k].y * a);
+        d[off + i] = r;
+        if (leaf) leaf_out[off + i] = r;
     }
 }
 
@@ -1142,13 +1148,14 @@ void launch_copy_interior(Ctx& c, const double* src, double* dst, const int* lis
     launch_copy_interior_vf(c, &src, &dst, 1, list, n);
 }
 
-void launch_axpy_blocks(Ctx& c, const double* src, double* dst, const int* list, int n, double a, bool assign)
+void launch_axpy_blocks(Ctx& c, const double* src, double* dst, const int* list, int n, double a, bool assign,
+                        double* leaf_out)
 {
     if (!n) return;
     const int half = (int)(c.block_elems() / 2);
-    axpy_kernel<<<dim3(n, pieces(2 * half)), 256, 0, c.stream>>>(reinterpret_cast<const double2*>(src),
-                                                                 reinterpret_cast<double2*>(dst), list, half, a,
-                                                                 assign ? 1 : 0);
+    axpy_kernel<<<dim3(n, pieces(2 * half)), 256, 0, c.stream>>>(
+        reinterpret_cast<const double2*>(src), reinterpret_cast<double2*>(dst), list, half, a, assign ? 1 : 0,
+        c.d_flags.p, reinterpret_cast<double2*>(leaf_out));
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }
