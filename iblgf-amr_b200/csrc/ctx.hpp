@@ -158,8 +158,10 @@ struct TpTasks  // tensor-product transfer tasks of one tree level
 // sibling groups per group-MAC tile; the kernel's thread rows x groups per
 // row cover exactly this many
 constexpr int kGroupTileCap = 32;
-// bundles of two sibling groups per tile of the direct MAC
+// bundles of two sibling groups per tile of the direct MAC, at most
 constexpr int kMacTile = 96;
+// staging a tile's LGF table, in bundles' worth of an SM's time
+constexpr int kMacStage = 2;
 // bundles of a table up to which its tile is split over four warps per bundle
 // (the CTA has 20 warps in FP32, 12 in FP64): the tiles of the coarse levels'
 // tables, 1 to 4 bundles, then take 5 instead of 15 us of an SM. At 16 to 24

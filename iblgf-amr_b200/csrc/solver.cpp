@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -860,16 +861,17 @@ HostPlan build_host_plan(const Ctx& c, int level, int idx, int ge, bool direct_o
     std::vector<int>& gtgt = p.gtgt;
     std::vector<unsigned short>& gsrc = p.gsrc;
     std::vector<unsigned>& gpm = p.gpm;
-    std::map<int, int> local;
-    int cur_ld = -1, ngrp = 0, max_src = 0;
+    std::vector<int> local;  // row in the tile by source, -1: none
+    int cur_ld = -1, ngrp = 0, n_local = 0, max_src = 0;
     auto close_tile = [&]() {
         if (!ngrp) return;
         tgptr.push_back((int)gtgt.size() / 8);
         tsptr.push_back((int)tsrc.size());
         ttab.push_back(tab_of_ld[cur_ld]);
         tcoarse.push_back(neighbor_only ? 2 : (cur_ld > 0 ? 1 : 0));
-        max_src = std::max(max_src, (int)local.size());
-        local.clear();
+        max_src = std::max(max_src, n_local);
+        for (size_t k = tsrc.size() - n_local; k < tsrc.size(); ++k) local[tsrc[k]] = -1;
+        n_local = 0;
         ngrp = 0;
     };
     for (int g : gorder)
@@ -877,8 +879,12 @@ HostPlan build_host_plan(const Ctx& c, int level, int idx, int ge, bool direct_o
         const Grp& gr = groups[g];
         int extra = 0;
         for (int kk = 0; kk < 216; ++kk)
-            if (gr.used[kk] && !local.count(gr.cand[kk])) ++extra;
-        if (ngrp && (gr.ld != cur_ld || ngrp >= kGcap || (int)local.size() + extra > kScap)) close_tile();
+            if (gr.used[kk])
+            {
+                if ((size_t)gr.cand[kk] >= local.size()) local.resize(gr.cand[kk] + 1, -1);
+                if (local[gr.cand[kk]] < 0) ++extra;
+            }
+        if (ngrp && (gr.ld != cur_ld || ngrp >= kGcap || n_local + extra > kScap)) close_tile();
         cur_ld = gr.ld;
         for (int kk = 0; kk < 216; ++kk)
         {
@@ -887,16 +893,12 @@ HostPlan build_host_plan(const Ctx& c, int level, int idx, int ge, bool direct_o
                 gsrc.push_back(0xFFFF);
                 continue;
             }
-            auto it = local.find(gr.cand[kk]);
-            int j;
-            if (it == local.end())
+            int& j = local[gr.cand[kk]];
+            if (j < 0)
             {
-                j = (int)local.size();
-                local.emplace(gr.cand[kk], j);
+                j = n_local++;
                 tsrc.push_back(gr.cand[kk]);
             }
-            else
-                j = it->second;
             gsrc.push_back((unsigned short)j);
         }
         for (int cc = 0; cc < 8; ++cc) gtgt.push_back(gr.tgt[cc] >= 0 ? slot_of_tp[gr.tgt[cc]] : -1);
@@ -933,10 +935,37 @@ HostPlan build_host_plan(const Ctx& c, int level, int idx, int ge, bool direct_o
 
 namespace
 {
+// Bundles per tile of the direct MAC, for the bundle counts of a plan's tables.
+// A tile runs as one CTA per 32 frequencies, one CTA per SM. Plans of at least
+// two waves of the largest tiles take these: one staged table for 96 bundles
+// (amr_3level FP32 at tiles fitted to whole waves: 12.2 instead of 11.2 ms, as
+// more CTAs end with idle warps). Below that (short spectra: 23 chunks of 32
+// frequencies at extent 4, 58 at 6, 199 at 10) the size whose waves end first is
+// taken, a CTA counted as its bundles (half its warps at least), half its warps
+// for the end, where warps run out of bundles, and kMacStage. Whole solves on
+// three levels, FP64, tiles of 96 -> fitted: extent 4 1141 -> 623 us, extent 6
+// 1218 -> 1009 and 1332 -> 1243 us; batch of 29 problems, extent 10 200 -> 184 us.
+int mac_tile_size(const Ctx& c, const std::vector<int>& bundles)
+{
+    constexpr long long sms = 148;
+    const long long chunks = (c.NC + 31) / 32, warps = c.cfg.precision == IBLGF_FP32 ? 20 : 12;
+    int best = kMacTile;
+    long long best_cost = LLONG_MAX;
+    for (int t = kMacTile; t >= 4; --t)
+    {
+        long long tiles = 0;
+        for (int nb : bundles) tiles += (nb + t - 1) / t;
+        if (t == kMacTile && tiles * chunks >= 2 * sms) break;
+        const long long cost =
+            (tiles * chunks + sms - 1) / sms * (std::max<long long>(t, warps / 2) + warps / 2 + kMacStage);
+        if (cost < best_cost) best_cost = cost, best = t;
+    }
+    return best;
+}
+
 // Tiles and bundles of the direct MAC: the groups by (LGF table, pair mode) in
 // plan order (parent keys ascending), two to a bundle; equal tables of a
-// batch's problems share their tiles. A tile holds up to kMacTile bundles (the
-// staged table serves them all).
+// batch's problems share their tiles.
 void build_mac_bundles(Ctx& c, FmmPlan& p, const HostPlan& h, const std::vector<int>& gjr)
 {
     if (!p.n_tiles) return;
@@ -947,8 +976,25 @@ void build_mac_bundles(Ctx& c, FmmPlan& p, const HostPlan& h, const std::vector<
         const int tab = first_of.emplace(h.tab_keys[343 * (size_t)h.ttab[t]], h.ttab[t]).first->second;
         for (int g = h.tgptr[t]; g < h.tgptr[t + 1]; ++g) by_table[{tab, h.tcoarse[t]}].push_back(g);
     }
+    std::vector<int> bundles;
+    for (auto& kv : by_table) bundles.push_back(((int)kv.second.size() + 1) / 2);
+    const int per_tile = mac_tile_size(c, bundles);
+    // target rows (bits of a half parent's mask) that adjacent candidates reach
+    unsigned near_rows[27][2];
+    for (int n = 0; n < 27; ++n)
+        for (int cz = 0; cz < 2; ++cz)
+        {
+            const int ny = (n / 3) % 3 - 1, nz = n / 9 - 1;
+            near_rows[n][cz] = 0;
+            for (int q = 0; q < 4; ++q)
+                for (int r = 0; r < 4; ++r)
+                    if (std::abs((r & 1) - (q >> 1) - 2 * ny) <= 1 && std::abs((r >> 1) - cz - 2 * nz) <= 1)
+                        near_rows[n][cz] |= 1u << (4 * q + r);
+        }
     std::vector<int> tile, ptr{0}, grp, rows;
     std::vector<unsigned> head;
+    rows.reserve((size_t)p.n_groups * 54 * 4 + 32);
+    head.reserve((size_t)p.n_groups * 54 + 64);
     for (auto& kv : by_table)
     {
         const int mode = kv.first.second;
@@ -956,36 +1002,39 @@ void build_mac_bundles(Ctx& c, FmmPlan& p, const HostPlan& h, const std::vector<
         std::stable_sort(gs.begin(), gs.end(), [&](int a, int b) {
             return __builtin_popcount(h.gpm[a]) > __builtin_popcount(h.gpm[b]);
         });
-        const int nb = ((int)gs.size() + 1) / 2, nt = (nb + kMacTile - 1) / kMacTile, b0 = (int)ptr.size() - 1;
+        const int nb = ((int)gs.size() + 1) / 2, nt = (nb + per_tile - 1) / per_tile, b0 = (int)ptr.size() - 1;
         for (int i = 0; i < nt; ++i)
             tile.insert(tile.end(), {b0 + (int)((long long)nb * i / nt), b0 + (int)((long long)nb * (i + 1) / nt),
                                      kv.first.first, mode | (nb <= kMacSplit ? 4 : 0)});
         for (int b = 0; b < nb; ++b)
         {
             const int g[2] = {gs[2 * b], 2 * b + 1 < (int)gs.size() ? gs[2 * b + 1] : -1};
-            int row_bits[2] = {0, 0};
+            unsigned row_bits[2] = {0, 0}, parents = 0;
             for (int i = 0; i < 2 && g[i] >= 0; ++i)
+            {
+                parents |= h.gpm[g[i]];
                 for (int r = 0; r < 4; ++r)
                     if (h.gtgt[8 * (size_t)g[i] + 2 * r] >= 0 || h.gtgt[8 * (size_t)g[i] + 2 * r + 1] >= 0)
-                        row_bits[i] |= 1 << r;
+                        row_bits[i] |= 1u << r;
+            }
             grp.insert(grp.end(), {g[0], g[1]});
             for (int n = 0; n < 27; ++n)
+            {
+                if (!(parents >> n & 1)) continue;
                 for (int cz = 0; cz < 2; ++cz)
                 {
                     const int nx = n % 3 - 1, ny = (n / 3) % 3 - 1, nz = n / 9 - 1;
                     int src[8];
                     unsigned mask[2] = {0, 0};
                     for (int i = 0; i < 2; ++i)
+                    {
                         for (int q = 0; q < 4; ++q)
                         {
                             src[4 * i + q] = g[i] >= 0 ? gjr[(size_t)g[i] * 216 + 8 * n + 4 * cz + q] : p.n_src;
-                            if (src[4 * i + q] == p.n_src) continue;
-                            for (int r = 0; r < 4; ++r)
-                                if (row_bits[i] >> r & 1 &&
-                                    (mode != 2 || (std::abs((r & 1) - (q >> 1) - 2 * ny) <= 1 &&
-                                                   std::abs((r >> 1) - cz - 2 * nz) <= 1)))
-                                    mask[i] |= 1u << (4 * q + r);
+                            if (src[4 * i + q] != p.n_src) mask[i] |= row_bits[i] << (4 * q);
                         }
+                        if (mode == 2) mask[i] &= near_rows[n][cz];
+                    }
                     if (!(mask[0] | mask[1])) continue;
                     for (unsigned& m : mask)
                     {
@@ -993,10 +1042,11 @@ void build_mac_bundles(Ctx& c, FmmPlan& p, const HostPlan& h, const std::vector<
                         p.mac_flops += 8 * 2 * __builtin_popcount(m);
                     }
                     // offset d = (-1, -1, -c'z) of this half: u = d - 2n
-                    head.insert(head.end(), {(unsigned)((2 - 2 * nx) + 7 * (2 - 2 * ny) + 49 * (3 - cz - 2 * nz)),
-                                             mask[0] | mask[1] << 16});
+                    head.push_back((unsigned)((2 - 2 * nx) + 7 * (2 - 2 * ny) + 49 * (3 - cz - 2 * nz)));
+                    head.push_back(mask[0] | mask[1] << 16);
                     rows.insert(rows.end(), src, src + 8);
                 }
+            }
             ptr.push_back((int)head.size() / 2);
         }
     }
