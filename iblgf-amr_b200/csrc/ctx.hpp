@@ -163,7 +163,7 @@ constexpr int kMacTile = 96;
 // staging a tile's LGF table, in bundles' worth of an SM's time
 constexpr int kMacStage = 2;
 // bundles of a table up to which its tile is split over four warps per bundle
-// (the CTA has 20 warps in FP32, 12 in FP64): the tiles of the coarse levels'
+// (the CTA has 16 warps in FP32, 12 in FP64): the tiles of the coarse levels'
 // tables, 1 to 4 bundles, then take 5 instead of 15 us of an SM. At 16 to 24
 // bundles the split costs a third (vortex ring, 1.36 against 1.09 ms).
 constexpr int kMacSplit = 5;

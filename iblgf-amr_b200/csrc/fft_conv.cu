@@ -520,9 +520,14 @@ __device__ __forceinline__ void mac_load(cx<R> (&s)[4], const cx<R>* Sf, const u
 // of 32 groups, each of one problem of a batch: the MAC of a batch of 256
 // problems 6.06 -> 1.88 ms (one staged table for 192 groups of any problem
 // instead of one for the few groups of each), amr_3level FP32 7.53 -> 7.08 ms,
-// vortex ring FP32 1.12 -> 1.04 ms, amr_2level FP64 3.45 -> 3.41 ms. Not kept: all 27 LGF values of a
-// parent in registers without shared memory (10.0 ms on amr_3level: its loads
-// are not hidden at 16 warps), LGF rows read through L1 by small warps (25 ms).
+// vortex ring FP32 1.12 -> 1.04 ms, amr_2level FP64 3.45 -> 3.41 ms. In FP32
+// the source values are loaded one half parent ahead, at 16 warps (122
+// registers), instead of 20 warps without: solves of amr_3level 11.21 -> 11.05
+// ms, of 256 problems 2.86 -> 2.83 ms, vortex ring step 11.92 -> 11.64 ms. Not
+// kept: all 27 LGF values of a parent in registers without shared memory (10.0
+// ms on amr_3level), LGF rows read through L1 by small warps (25 ms), two CTAs
+// of 10 warps per SM (less L1 for the source rows: +0.7 ms), packed FP32 FMAs
+// with their accumulators doubled (+0.7 ms).
 // In a split tile (bit 2 of its mode) a warp takes one group of a bundle and one
 // half (cz) of its targets: tiles whose bundles are no more than a quarter of
 // the CTA's warps. ALL: every tile is split, and the kernel keeps the registers
@@ -633,26 +638,59 @@ __global__ void __launch_bounds__(NT, MINB) bundle_mac_kernel(
             const uint4* rp = rows + 2 * (size_t)e0;
             uint4 ra = rp[0], rb = rp[1];
             uint2 h = *hp;
-            for (int e = e0; e < e1; ++e)
+            if constexpr (sizeof(R) == 4)
             {
-                cx<R> s0[4], s1[4], gv[9];
+                // source values one half parent ahead, their rows two
+                cx<R> s0[4], s1[4];
                 mac_load<R, NB>(s0, Sf, ra);
                 mac_load<R, NB>(s1, Sf, rb);
-                const cx<R>* g = Gs + h.x * F + lane;
-                const unsigned m0 = h.y & 0xFFFFu, m1 = h.y >> 16;
-                rp += 2;
-                ra = rp[0];
-                rb = rp[1];
-                h = *++hp;
+                ra = rp[2];
+                rb = rp[3];
+#pragma unroll 2
+                for (int e = e0; e < e1; ++e)
+                {
+                    cx<R> n0[4], n1[4], gv[9];
+                    mac_load<R, NB>(n0, Sf, ra);
+                    mac_load<R, NB>(n1, Sf, rb);
+                    const cx<R>* g = Gs + h.x * F + lane;
+                    const unsigned m0 = h.y & 0xFFFFu, m1 = h.y >> 16;
+                    ra = rp[4];
+                    rb = rp[5];
+                    rp += 2;
+                    h = *++hp;
 #pragma unroll
-                for (int d = 0; d < 9; ++d) gv[d] = g[((d % 3) + 7 * (d / 3)) * F];
-                mac_half<R, 0>(gv, s0, acc0, m0);
-                mac_half<R, 0>(gv, s1, acc1, m1);
+                    for (int d = 0; d < 9; ++d) gv[d] = g[((d % 3) + 7 * (d / 3)) * F];
+                    mac_half<R, 0>(gv, s0, acc0, m0);
+                    mac_half<R, 0>(gv, s1, acc1, m1);
 #pragma unroll
-                for (int d = 0; d < 9; ++d) gv[d] = g[((d % 3) + 7 * (d / 3) + 49) * F];
-                mac_half<R, 1>(gv, s0, acc0, m0);
-                mac_half<R, 1>(gv, s1, acc1, m1);
+                    for (int d = 0; d < 9; ++d) gv[d] = g[((d % 3) + 7 * (d / 3) + 49) * F];
+                    mac_half<R, 1>(gv, s0, acc0, m0);
+                    mac_half<R, 1>(gv, s1, acc1, m1);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) s0[q] = n0[q], s1[q] = n1[q];
+                }
             }
+            else  // rows one half parent ahead; no registers for more
+                for (int e = e0; e < e1; ++e)
+                {
+                    cx<R> s0[4], s1[4], gv[9];
+                    mac_load<R, NB>(s0, Sf, ra);
+                    mac_load<R, NB>(s1, Sf, rb);
+                    const cx<R>* g = Gs + h.x * F + lane;
+                    const unsigned m0 = h.y & 0xFFFFu, m1 = h.y >> 16;
+                    rp += 2;
+                    ra = rp[0];
+                    rb = rp[1];
+                    h = *++hp;
+#pragma unroll
+                    for (int d = 0; d < 9; ++d) gv[d] = g[((d % 3) + 7 * (d / 3)) * F];
+                    mac_half<R, 0>(gv, s0, acc0, m0);
+                    mac_half<R, 0>(gv, s1, acc1, m1);
+#pragma unroll
+                    for (int d = 0; d < 9; ++d) gv[d] = g[((d % 3) + 7 * (d / 3) + 49) * F];
+                    mac_half<R, 1>(gv, s0, acc0, m0);
+                    mac_half<R, 1>(gv, s1, acc1, m1);
+                }
             if (f < NC)
 #pragma unroll
                 for (int c = 0; c < 8; ++c)
@@ -859,7 +897,7 @@ struct Conv
         }
         else
         {
-            if constexpr (kF32) group_mac_shape<640, 1, false>(c, p, S, acc);
+            if constexpr (kF32) group_mac_shape<512, 1, false>(c, p, S, acc);
             else group_mac_shape<384, 1, false>(c, p, S, acc);
         }
     }

@@ -941,14 +941,15 @@ namespace
 // (amr_3level FP32 at tiles fitted to whole waves: 12.2 instead of 11.2 ms, as
 // more CTAs end with idle warps). Below that (short spectra: 23 chunks of 32
 // frequencies at extent 4, 58 at 6, 199 at 10) the size whose waves end first is
-// taken, a CTA counted as its bundles (half its warps at least), half its warps
-// for the end, where warps run out of bundles, and kMacStage. Whole solves on
+// taken, a CTA counted as its bundles (at least `few`: fewer leave its warps'
+// latencies open), as many for the end, where warps run out of bundles, and
+// kMacStage. Whole solves on
 // three levels, FP64, tiles of 96 -> fitted: extent 4 1141 -> 623 us, extent 6
 // 1218 -> 1009 and 1332 -> 1243 us; batch of 29 problems, extent 10 200 -> 184 us.
 int mac_tile_size(const Ctx& c, const std::vector<int>& bundles)
 {
     constexpr long long sms = 148;
-    const long long chunks = (c.NC + 31) / 32, warps = c.cfg.precision == IBLGF_FP32 ? 20 : 12;
+    const long long chunks = (c.NC + 31) / 32, few = c.cfg.precision == IBLGF_FP32 ? 10 : 6;
     int best = kMacTile;
     long long best_cost = LLONG_MAX;
     for (int t = kMacTile; t >= 4; --t)
@@ -956,8 +957,7 @@ int mac_tile_size(const Ctx& c, const std::vector<int>& bundles)
         long long tiles = 0;
         for (int nb : bundles) tiles += (nb + t - 1) / t;
         if (t == kMacTile && tiles * chunks >= 2 * sms) break;
-        const long long cost =
-            (tiles * chunks + sms - 1) / sms * (std::max<long long>(t, warps / 2) + warps / 2 + kMacStage);
+        const long long cost = (tiles * chunks + sms - 1) / sms * (std::max<long long>(t, few) + few + kMacStage);
         if (cost < best_cost) best_cost = cost, best = t;
     }
     return best;
@@ -999,8 +999,13 @@ void build_mac_bundles(Ctx& c, FmmPlan& p, const HostPlan& h, const std::vector<
     {
         const int mode = kv.first.second;
         std::vector<int>& gs = kv.second;
+        // long walks first, so that a tile's warps end together. FP32 leaves 140
+        // KB of an SM's L1 to the source rows, which groups close in parent key
+        // share, so it sorts by thirds of the 27 parents only (batch of 256
+        // problems 2.86 -> 2.82 ms, FP64 on two levels the other way, 5.09 -> 5.12)
+        const int step = c.cfg.precision == IBLGF_FP32 ? 9 : 1;
         std::stable_sort(gs.begin(), gs.end(), [&](int a, int b) {
-            return __builtin_popcount(h.gpm[a]) > __builtin_popcount(h.gpm[b]);
+            return __builtin_popcount(h.gpm[a]) / step > __builtin_popcount(h.gpm[b]) / step;
         });
         const int nb = ((int)gs.size() + 1) / 2, nt = (nb + per_tile - 1) / per_tile, b0 = (int)ptr.size() - 1;
         for (int i = 0; i < nt; ++i)
