@@ -1,11 +1,11 @@
 // Immersed-boundary transfer kernels (FP64):
 //   ib_projection_kernel  Operator::ib_projection (operators.hpp:841-861):
-//                         one thread per (point, component) sums u_c(node) *
-//                         delta over the point's influence nodes in list order
+//                         one warp per point sums u_c(node) * delta over the
+//                         point's influence nodes
 //   ib_smearing_kernel    Operator::ib_smearing (operators.hpp:996-1013) as a
-//                         gather: one thread per (node, component) adds
-//                         f_c(point) * delta over the points that reach the
-//                         node, in point order (deterministic, no atomics)
+//                         gather: kSmearLanes lanes per node add f_c(point) *
+//                         delta over the points that reach the node
+//                         (fixed order, no atomics)
 //   face_planes_kernel    clean_ib_region_boundary / Operator::
 //                         clean_leaf_correction_boundary (operators.hpp:73-170,
 //                         329-517): zero the outer planes of listed faces
@@ -17,53 +17,102 @@ namespace iblgf_b200
 {
 namespace
 {
-// entries e in [ptr[i], ptr[i+1]) of point i: field offset at[e], weight w[3e + c]
-__global__ void ib_projection_kernel(const double* __restrict__ u0, const double* __restrict__ u1,
-                                     const double* __restrict__ u2, const int* __restrict__ ptr,
-                                     const long long* __restrict__ at, const double* __restrict__ w, int n,
-                                     double* __restrict__ f)
+// entries e in [ptr[i], ptr[i+1]) of point i: field offset at[e], weight w[3e + c].
+// A point's gathers are spread over a warp, all three components at once, and
+// summed across it in a fixed order: one thread per (point, component) followed
+// its entries one after another, 493 us for 2009 points.
+__global__ void __launch_bounds__(256) ib_projection_kernel(const double* __restrict__ u0,
+                                                            const double* __restrict__ u1,
+                                                            const double* __restrict__ u2,
+                                                            const int* __restrict__ ptr,
+                                                            const long long* __restrict__ at,
+                                                            const double* __restrict__ w, int n,
+                                                            double* __restrict__ f)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 3 * n) return;
-    const int i = t / 3, c = t % 3;
-    const double* u = c == 0 ? u0 : (c == 1 ? u1 : u2);
-    double s = 0.0;
-    for (int e = ptr[i]; e < ptr[i + 1]; ++e) s += u[at[e]] * w[3 * e + c];
-    f[3 * i + c] = s;
+    const int i = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
+    if (i >= n) return;
+    double s[3] = {0.0, 0.0, 0.0};
+    const int end = ptr[i + 1];
+#pragma unroll 4
+    for (int e = ptr[i] + lane; e < end; e += 32)
+    {
+        const long long a = at[e];
+        s[0] = fma(u0[a], w[3 * (size_t)e], s[0]);
+        s[1] = fma(u1[a], w[3 * (size_t)e + 1], s[1]);
+        s[2] = fma(u2[a], w[3 * (size_t)e + 2], s[2]);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+    {
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) s[c] += __shfl_xor_sync(0xffffffffu, s[c], m);
+        if (lane == c) f[3 * i + c] = s[c];
+    }
 }
 
 // nodes k: field offset node_at[k]; entries [nptr[k], nptr[k+1]) of node k
-// give (point nidx[j], entry weight row nw[j]) in increasing point order
-__global__ void ib_smearing_kernel(double* __restrict__ u0, double* __restrict__ u1, double* __restrict__ u2,
-                                   const long long* __restrict__ node_at, const int* __restrict__ nptr,
-                                   const int* __restrict__ npt, const int* __restrict__ nent,
-                                   const double* __restrict__ w, int n_nodes, const double* __restrict__ f)
+// give (point npt[j], entry weight row nent[j]) in increasing point order.
+// kSmearLanes lanes per node, summed in a fixed order (one thread per (node,
+// component): 42 us for 2009 points)
+constexpr int kSmearLanes = 8;
+
+__global__ void __launch_bounds__(128) ib_smearing_kernel(double* __restrict__ u0, double* __restrict__ u1,
+                                                          double* __restrict__ u2,
+                                                          const long long* __restrict__ node_at,
+                                                          const int* __restrict__ nptr, const int* __restrict__ npt,
+                                                          const int* __restrict__ nent, const double* __restrict__ w,
+                                                          int n_nodes, const double* __restrict__ f)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= 3 * n_nodes) return;
-    const int k = t / 3, c = t % 3;
-    double* u = c == 0 ? u0 : (c == 1 ? u1 : u2);
-    double v = u[node_at[k]];
-    for (int j = nptr[k]; j < nptr[k + 1]; ++j) v += f[3 * npt[j] + c] * w[3 * nent[j] + c];
-    u[node_at[k]] = v;
+    const int k = blockIdx.x * (128 / kSmearLanes) + threadIdx.x / kSmearLanes, lane = threadIdx.x % kSmearLanes;
+    double v[3] = {0.0, 0.0, 0.0};
+    if (k < n_nodes)
+    {
+        const int end = nptr[k + 1];
+#pragma unroll 2
+        for (int j = nptr[k] + lane; j < end; j += kSmearLanes)
+        {
+            const double* fp = f + 3 * (size_t)npt[j];
+            const double* wp = w + 3 * (size_t)nent[j];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[c] = fma(fp[c], wp[c], v[c]);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int m = kSmearLanes / 2; m > 0; m >>= 1) v[c] += __shfl_xor_sync(0xffffffffu, v[c], m);
+    if (k >= n_nodes || lane >= 3) return;
+    double* u = (lane == 0 ? u0 : lane == 1 ? u1 : u2) + node_at[k];
+    *u += lane == 0 ? v[0] : lane == 1 ? v[1] : v[2];
 }
 
-// list[b]: octant, faces[b]: bit q set = zero the planes towards face q
-// (q: 0 z-, 1 y-, 2 x-, 3 x+, 4 y+, 5 z+)
-template<int NB>
-__global__ void face_planes_kernel(double* __restrict__ f, const int* __restrict__ list,
-                                   const unsigned char* __restrict__ faces, int width)
+struct PlaneFields
 {
-    constexpr int N3 = NB * NB * NB;
-    double* b = f + (size_t)list[blockIdx.x] * N3;
+    double* f[3];
+};
+
+// list[b]: octant, faces[b]: bit q set = zero the planes towards face q
+// (q: 0 z-, 1 y-, 2 x-, 3 x+, 4 y+, 5 z+); one component field per blockIdx.y.
+// The threads walk the planes only (a walk over the whole block took 13 us for
+// each component of the sphere's blocks)
+template<int NB>
+__global__ void __launch_bounds__(256) face_planes_kernel(const __grid_constant__ PlaneFields fs,
+                                                          const int* __restrict__ list,
+                                                          const unsigned char* __restrict__ faces, int width)
+{
+    double* b = fs.f[blockIdx.y] + (size_t)list[blockIdx.x] * (NB * NB * NB);
     const unsigned m = faces[blockIdx.x];
-    for (int i = threadIdx.x; i < N3; i += blockDim.x)
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
     {
-        const int x = i % NB, y = (i / NB) % NB, z = i / (NB * NB);
-        const bool zero = ((m & 1) && z < width) || ((m & 2) && y < width) || ((m & 4) && x < width) ||
-                          ((m & 8) && x >= NB - width) || ((m & 16) && y >= NB - width) ||
-                          ((m & 32) && z >= NB - width);
-        if (zero) b[i] = 0.0;
+        if (!(m >> q & 1)) continue;
+        for (int i = threadIdx.x; i < width * NB * NB; i += 256)
+        {
+            const int d = i / (NB * NB), p = i % (NB * NB), l = q < 3 ? d : NB - 1 - d;
+            if (q == 0 || q == 5) b[l * NB * NB + p] = 0.0;
+            else if (q == 1 || q == 4) b[p / NB * NB * NB + l * NB + p % NB] = 0.0;
+            else b[p * NB + l] = 0.0;
+        }
     }
 }
 }  // namespace
@@ -72,7 +121,7 @@ void launch_ib_projection(Ctx& c, const double* const* u, const int* ptr, const 
                           int n, double* f)
 {
     if (!n) return;
-    ib_projection_kernel<<<(3 * n + 127) / 128, 128, 0, c.stream>>>(u[0], u[1], u[2], ptr, at, w, n, f);
+    ib_projection_kernel<<<(n + 7) / 8, 256, 0, c.stream>>>(u[0], u[1], u[2], ptr, at, w, n, f);
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }
@@ -81,23 +130,28 @@ void launch_ib_smearing(Ctx& c, double* const* u, const long long* node_at, cons
                         const int* nent, const double* w, int n_nodes, const double* f)
 {
     if (!n_nodes) return;
-    ib_smearing_kernel<<<(3 * n_nodes + 127) / 128, 128, 0, c.stream>>>(u[0], u[1], u[2], node_at, nptr, npt, nent,
-                                                                         w, n_nodes, f);
+    constexpr int per = 128 / kSmearLanes;
+    ib_smearing_kernel<<<(n_nodes + per - 1) / per, 128, 0, c.stream>>>(u[0], u[1], u[2], node_at, nptr, npt, nent, w,
+                                                                        n_nodes, f);
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }
 
-void launch_face_planes(Ctx& c, double* f, const int* list, const unsigned char* faces, int n, int width)
+void launch_face_planes(Ctx& c, double* const* f, int nf, const int* list, const unsigned char* faces, int n,
+                        int width)
 {
     if (!n) return;
+    PlaneFields fs{};
+    for (int k = 0; k < nf; ++k) fs.f[k] = f[k];
+    const dim3 grid(n, nf);
     switch (c.Nb)
     {
-        case 6: face_planes_kernel<6><<<n, 256, 0, c.stream>>>(f, list, faces, width); break;
-        case 8: face_planes_kernel<8><<<n, 256, 0, c.stream>>>(f, list, faces, width); break;
-        case 10: face_planes_kernel<10><<<n, 256, 0, c.stream>>>(f, list, faces, width); break;
-        case 12: face_planes_kernel<12><<<n, 256, 0, c.stream>>>(f, list, faces, width); break;
-        case 16: face_planes_kernel<16><<<n, 256, 0, c.stream>>>(f, list, faces, width); break;
-        case 18: face_planes_kernel<18><<<n, 256, 0, c.stream>>>(f, list, faces, width); break;
+        case 6: face_planes_kernel<6><<<grid, 256, 0, c.stream>>>(fs, list, faces, width); break;
+        case 8: face_planes_kernel<8><<<grid, 256, 0, c.stream>>>(fs, list, faces, width); break;
+        case 10: face_planes_kernel<10><<<grid, 256, 0, c.stream>>>(fs, list, faces, width); break;
+        case 12: face_planes_kernel<12><<<grid, 256, 0, c.stream>>>(fs, list, faces, width); break;
+        case 16: face_planes_kernel<16><<<grid, 256, 0, c.stream>>>(fs, list, faces, width); break;
+        case 18: face_planes_kernel<18><<<grid, 256, 0, c.stream>>>(fs, list, faces, width); break;
         default: throw Error(IBLGF_EINVAL, "unsupported block size");
     }
     c.launches += 1;

@@ -1,7 +1,8 @@
 """Block kernels over the block extents and the edges of their work splits,
 against the oracle: sweeps with partly present sibling groups, the integrating
-factor's truncation radii, the single-block convolution, and the Fourier-in-z
-operators at extents without a compile-time form."""
+factor's truncation radii, the single-block convolution, the Fourier-in-z
+operators at extents without a compile-time form, and few immersed-boundary
+points."""
 import os
 import sys
 
@@ -9,6 +10,7 @@ import numpy as np
 import pytest
 
 import iblgf_b200 as B
+import iblgf_setups as S
 import oracle_lib as O
 
 sys.path.insert(0, os.path.join(os.path.dirname(__file__), "..", "oracle"))
@@ -101,3 +103,18 @@ def test_fourier_operators_extents(op, nb, nm):
     g.helm2d_op(op, s, d, nm, 0.25, 1.5, 0.6)
     g.synchronize()
     assert np.abs(d.cpu().numpy() - ref).max() < 1e-13 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 33])
+def test_ib_few_points(n):
+    """Point counts around a CTA's eight points of the projection; 1e-9 as for the whole sphere's force solve."""
+    case = S.SphereIB("small")
+    args = (case.bd_base, case.bd_extent, case.block_extent, case.dx_base, case.blocks)
+    o = O.Domain(*args, n_levels=case.n_levels, predicate=case.predicate)
+    g = B.Solver(*args, n_levels=case.n_levels, predicate=case.predicate)
+    X = O.sphere_points(case.dx_base, o.depth - 1 - o.base_level, case.ibph)[:n]
+    u = case.velocity(o)
+    f_ref, _, _ = o.ib_solve(X, case.Re, u, 7e-4, 1e-3, 40)
+    g.ib_set_points(X, case.Re)
+    f, _ = g.ib_solve([g.field(u[k]) for k in range(3)], 7e-4, 1e-3, 40)
+    assert rel_linf(f, f_ref) < 1e-9
