@@ -504,9 +504,7 @@ void launch_ib_projection(Ctx& c, const double* const* u, const int* ptr, const 
                           int n, double* f);
 void launch_ib_smearing(Ctx& c, double* const* u, const long long* node_at, const int* nptr, const int* npt,
                         const int* nent, const double* w, int n_nodes, const double* f);
-// outer planes of nf (1 .. 3) component fields
-void launch_face_planes(Ctx& c, double* const* f, int nf, const int* list, const unsigned char* faces, int n,
-                        int width);
+void launch_face_planes(Ctx& c, double* f, const int* list, const unsigned char* faces, int n, int width);
 // device force CG (ib.cu): FP64 dot products by one CTA in a fixed order;
 // ctl = [done, iterations, not converged], sc = [rsold, p.Ap, rsnew, f.f]
 void launch_cg_dot(Ctx& c, const double* a, const double* b, const double* a2, const double* b2, int n,

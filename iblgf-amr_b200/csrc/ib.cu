@@ -20,7 +20,8 @@ namespace
 // entries e in [ptr[i], ptr[i+1]) of point i: field offset at[e], weight w[3e + c].
 // A point's gathers are spread over a warp, all three components at once, and
 // summed across it in a fixed order: one thread per (point, component) followed
-// its entries one after another, 493 us for 2009 points.
+// its entries one after another, 493 us for 2009 points, 47 us now (56 bytes per
+// entry, mostly from L2).
 __global__ void __launch_bounds__(256) ib_projection_kernel(const double* __restrict__ u0,
                                                             const double* __restrict__ u1,
                                                             const double* __restrict__ u2,
@@ -52,8 +53,8 @@ __global__ void __launch_bounds__(256) ib_projection_kernel(const double* __rest
 
 // nodes k: field offset node_at[k]; entries [nptr[k], nptr[k+1]) of node k
 // give (point npt[j], entry weight row nent[j]) in increasing point order.
-// kSmearLanes lanes per node, summed in a fixed order (one thread per (node,
-// component): 42 us for 2009 points)
+// kSmearLanes lanes per node, summed in a fixed order (33 us for 2009 points; one
+// thread per (node, component): 42 us)
 constexpr int kSmearLanes = 8;
 
 __global__ void __launch_bounds__(128) ib_smearing_kernel(double* __restrict__ u0, double* __restrict__ u1,
@@ -86,33 +87,22 @@ __global__ void __launch_bounds__(128) ib_smearing_kernel(double* __restrict__ u
     *u += lane == 0 ? v[0] : lane == 1 ? v[1] : v[2];
 }
 
-struct PlaneFields
-{
-    double* f[3];
-};
-
 // list[b]: octant, faces[b]: bit q set = zero the planes towards face q
-// (q: 0 z-, 1 y-, 2 x-, 3 x+, 4 y+, 5 z+); one component field per blockIdx.y.
-// The threads walk the planes only (a walk over the whole block took 13 us for
-// each component of the sphere's blocks)
+// (q: 0 z-, 1 y-, 2 x-, 3 x+, 4 y+, 5 z+)
 template<int NB>
-__global__ void __launch_bounds__(256) face_planes_kernel(const __grid_constant__ PlaneFields fs,
-                                                          const int* __restrict__ list,
-                                                          const unsigned char* __restrict__ faces, int width)
+__global__ void face_planes_kernel(double* __restrict__ f, const int* __restrict__ list,
+                                   const unsigned char* __restrict__ faces, int width)
 {
-    double* b = fs.f[blockIdx.y] + (size_t)list[blockIdx.x] * (NB * NB * NB);
+    constexpr int N3 = NB * NB * NB;
+    double* b = f + (size_t)list[blockIdx.x] * N3;
     const unsigned m = faces[blockIdx.x];
-#pragma unroll
-    for (int q = 0; q < 6; ++q)
+    for (int i = threadIdx.x; i < N3; i += blockDim.x)
     {
-        if (!(m >> q & 1)) continue;
-        for (int i = threadIdx.x; i < width * NB * NB; i += 256)
-        {
-            const int d = i / (NB * NB), p = i % (NB * NB), l = q < 3 ? d : NB - 1 - d;
-            if (q == 0 || q == 5) b[l * NB * NB + p] = 0.0;
-            else if (q == 1 || q == 4) b[p / NB * NB * NB + l * NB + p % NB] = 0.0;
-            else b[p * NB + l] = 0.0;
-        }
+        const int x = i % NB, y = (i / NB) % NB, z = i / (NB * NB);
+        const bool zero = ((m & 1) && z < width) || ((m & 2) && y < width) || ((m & 4) && x < width) ||
+                          ((m & 8) && x >= NB - width) || ((m & 16) && y >= NB - width) ||
+                          ((m & 32) && z >= NB - width);
+        if (zero) b[i] = 0.0;
     }
 }
 }  // namespace
@@ -137,21 +127,17 @@ void launch_ib_smearing(Ctx& c, double* const* u, const long long* node_at, cons
     IBLGF_CUDA(cudaGetLastError());
 }
 
-void launch_face_planes(Ctx& c, double* const* f, int nf, const int* list, const unsigned char* faces, int n,
-                        int width)
+void launch_face_planes(Ctx& c, double* f, const int* list, const unsigned char* faces, int n, int width)
 {
     if (!n) return;
-    PlaneFields fs{};
-    for (int k = 0; k < nf; ++k) fs.f[k] = f[k];
-    const dim3 grid(n, nf);
     switch (c.Nb)
     {
-        case 6: face_planes_kernel<6><<<grid, 256, 0, c.stream>>>(fs, list, faces, width); break;
-        case 8: face_planes_kernel<8><<<grid, 256, 0, c.stream>>>(fs, list, faces, width); break;
-        case 10: face_planes_kernel<10><<<grid, 256, 0, c.stream>>>(fs, list, faces, width); break;
-        case 12: face_planes_kernel<12><<<grid, 256, 0, c.stream>>>(fs, list, faces, width); break;
-        case 16: face_planes_kernel<16><<<grid, 256, 0, c.stream>>>(fs, list, faces, width); break;
-        case 18: face_planes_kernel<18><<<grid, 256, 0, c.stream>>>(fs, list, faces, width); break;
+        case 6: face_planes_kernel<6><<<n, 256, 0, c.stream>>>(f, list, faces, width); break;
+        case 8: face_planes_kernel<8><<<n, 256, 0, c.stream>>>(f, list, faces, width); break;
+        case 10: face_planes_kernel<10><<<n, 256, 0, c.stream>>>(f, list, faces, width); break;
+        case 12: face_planes_kernel<12><<<n, 256, 0, c.stream>>>(f, list, faces, width); break;
+        case 16: face_planes_kernel<16><<<n, 256, 0, c.stream>>>(f, list, faces, width); break;
+        case 18: face_planes_kernel<18><<<n, 256, 0, c.stream>>>(f, list, faces, width); break;
         default: throw Error(IBLGF_EINVAL, "unsupported block size");
     }
     c.launches += 1;

@@ -352,14 +352,14 @@ void apply_schur(Ctx& c, IbState& s, const int* src, const int* tgt)
     launch_op(c, 2, pin, 3, pc, 1, ol.list[l].p, ol.dx[l].p, (int)ol.list[l].n, 1.0);
     // Operator::clean_leaf_correction_boundary<cell_aux2>(l, true, 2)
     launch_zero_blocks(c, pc[0], s.corr_list.p, s.n_corr);
-    if (s.clean_base) launch_face_planes(c, pc, 1, s.cb_list.p, s.cb_faces.p, s.n_cb, 2);
-    launch_face_planes(c, pc, 1, s.ibc_list.p, s.ibc_faces.p, s.n_ibc, 2);
+    if (s.clean_base) launch_face_planes(c, pc[0], s.cb_list.p, s.cb_faces.p, s.n_cb, 2);
+    launch_face_planes(c, pc[0], s.ibc_list.p, s.ibc_faces.p, s.n_ibc, 2);
     poisson_apply_lgf(c, s.cell_aux2, s.cell_aux2, IBLGF_xIB2IB);
     const double* pg[1] = {c.field(s.cell_aux2)};
     double* pt[3] = {c.field(tgt[0]), c.field(tgt[1]), c.field(tgt[2])};
     launch_op(c, 1, pg, 1, pt, 3, ol.list[l].p, ol.dx[l].p, (int)ol.list[l].n, 1.0);
     launch_halo_vf(c, pt, 3, ol.list[l].p, (int)ol.list[l].n);
-    launch_face_planes(c, pt, 3, s.ibc_list.p, s.ibc_faces.p, s.n_ibc, 2);
+    for (int k = 0; k < 3; ++k) launch_face_planes(c, pt[k], s.ibc_list.p, s.ibc_faces.p, s.n_ibc, 2);
 }
 
 // LinSysSolver::ET_H_S_E (linsys.hpp:260-297): device forces in, device
@@ -750,7 +750,7 @@ void ns_ib_stage(Ctx& c, int stage, double alpha, double threshold, int max_iter
     double* pc[1] = {c.field(s.cell_aux2)};
     launch_op(c, 2, pin, 3, pc, 1, ol.list[l].p, ol.dx[l].p, (int)ol.list[l].n, 1.0);
     launch_zero_blocks(c, pc[0], s.corr_list.p, s.n_corr);
-    if (s.clean_base) launch_face_planes(c, pc, 1, s.cb_list.p, s.cb_faces.p, s.n_cb, 2);
+    if (s.clean_base) launch_face_planes(c, pc[0], s.cb_list.p, s.cb_faces.p, s.n_cb, 2);
     poisson_apply_lgf(c, s.cell_aux2, s.cell_aux2, IBLGF_IB2AMR);
     launch_axpby(c, c.field(d_field), c.field(s.cell_aux2), -1.0, 1);
     gradient_d();
