@@ -331,10 +331,6 @@ struct Ctx
     // device octant data
     DevBuf<int> d_bbase, d_nbr;
     DevBuf<int> d_flags;  // per octant: bit 0 leaf, bit 1 correction, bit 2 at or above the base level
-    // correction_tmp is zero everywhere: set by the solves that clean it, reset
-    // whenever its memory is handed out
-    bool correction_zero = false;
-    bool capturing_step = false;  // ns_step records a time step (its solves run in the recorded order only)
     // leaf blocks in canonical order and the device staging of their
     // interiors (leaf-interior field transfers); rebuilt with the domain
     DevBuf<int> d_leaf_blocks;
@@ -445,11 +441,7 @@ struct Ctx
     size_t block_elems() const { return (size_t)Nb * Nb * Nb; }
     size_t field_elems() const { return (size_t)n_oct * block_elems(); }
     size_t cplx_bytes() const { return cfg.precision == IBLGF_FP32 ? 8 : 16; }
-    double* field(int id)
-    {
-        if (id == f_correction_tmp) correction_zero = false;
-        return fields.at(id)->d.p;
-    }
+    double* field(int id) { return fields.at(id)->d.p; }
 };
 
 // -------------------------------------------------------------- library
@@ -596,7 +588,9 @@ void block_norms(Ctx& c, const int* fields, int n_comp, double* host_max, double
 OpLists& op_lists(Ctx& c);
 void apply_op_octants(Ctx& c, int op, const int* in, int n_in, const int* out, int n_out, const int* octants, int n,
                       double scale);
-void poisson_apply_lgf(Ctx& c, int src, int tgt, int fmm_type);
+// clean_correction: the solves without a source correction zero correction_tmp
+// first (false: the caller ran such a solve, and nothing since wrote the field)
+void poisson_apply_lgf(Ctx& c, int src, int tgt, int fmm_type, bool clean_correction = true);
 int mask_idx_gen(int type, int refinement_level, int nlas);
 
 // -------------------------------------------------------------- kernels (.cu)

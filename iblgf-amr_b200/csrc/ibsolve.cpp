@@ -341,7 +341,7 @@ void smearing(Ctx& c, IbState& s, const double* f, const int* u, bool cleaning =
 }
 
 // apply_Schur<Source, Target>(xIB2IB), linsys.hpp:299-330
-void apply_schur(Ctx& c, IbState& s, const int* src, const int* tgt)
+void apply_schur(Ctx& c, IbState& s, const int* src, const int* tgt, bool clean_correction)
 {
     OpLists& ol = op_lists(c);
     const int l = c.tree.depth - 1;
@@ -354,7 +354,7 @@ void apply_schur(Ctx& c, IbState& s, const int* src, const int* tgt)
     launch_zero_blocks(c, pc[0], s.corr_list.p, s.n_corr);
     if (s.clean_base) launch_face_planes(c, pc[0], s.cb_list.p, s.cb_faces.p, s.n_cb, 2);
     launch_face_planes(c, pc[0], s.ibc_list.p, s.ibc_faces.p, s.n_ibc, 2);
-    poisson_apply_lgf(c, s.cell_aux2, s.cell_aux2, IBLGF_xIB2IB);
+    poisson_apply_lgf(c, s.cell_aux2, s.cell_aux2, IBLGF_xIB2IB, clean_correction);
     const double* pg[1] = {c.field(s.cell_aux2)};
     double* pt[3] = {c.field(tgt[0]), c.field(tgt[1]), c.field(tgt[2])};
     launch_op(c, 1, pg, 1, pt, 3, ol.list[l].p, ol.dx[l].p, (int)ol.list[l].n, 1.0);
@@ -363,14 +363,15 @@ void apply_schur(Ctx& c, IbState& s, const int* src, const int* tgt)
 }
 
 // LinSysSolver::ET_H_S_E (linsys.hpp:260-297): device forces in, device
-// projection out
-void et_h_s_e(Ctx& c, IbState& s, const double* fin, double* fout, double alpha)
+// projection out. first: of a force solve; its Poisson solve cleans
+// correction_tmp, which the others of the force solve leave as it is.
+void et_h_s_e(Ctx& c, IbState& s, const double* fin, double* fout, double alpha, bool first)
 {
     zero_finest(c, s.face_aux);
     smearing(c, s, fin, s.face_aux2);
     static const int face[3][3] = {{0, 1, 1}, {1, 0, 1}, {1, 1, 0}};  // relative positions of face components
     if (std::fabs(alpha) > 1e-14) apply_if_vf(c, 3, s.face_aux2, s.face_aux2, alpha, IBLGF_IB2xIB, face);
-    apply_schur(c, s, s.face_aux2, s.face_aux);
+    apply_schur(c, s, s.face_aux2, s.face_aux, first);
     OpLists& ol = op_lists(c);
     const int l = c.tree.depth - 1;
     for (int k = 0; k < 3; ++k)
@@ -608,7 +609,7 @@ void cg_iteration(Ctx& c, IbState& s, double alpha, double threshold, int max_it
                   bool set_cond)
 {
     const int m = 3 * s.n;
-    et_h_s_e(c, s, s.cg_p.p, s.cg_Ap.p, alpha);
+    et_h_s_e(c, s, s.cg_p.p, s.cg_Ap.p, alpha, false);
     launch_cg_dot(c, s.cg_p.p, s.cg_Ap.p, nullptr, nullptr, m, s.cg_sc.p + 1, nullptr, s.cg_ctl.p);
     launch_cg_update(c, s.cg_f.p, s.cg_r.p, s.cg_p.p, s.cg_Ap.p, m, s.cg_sc.p, s.cg_ctl.p);
     launch_cg_dot(c, s.cg_r.p, s.cg_r.p, s.cg_f.p, s.cg_f.p, m, s.cg_sc.p + 2, s.cg_sc.p + 3, s.cg_ctl.p);
@@ -626,7 +627,7 @@ void cg_solve(Ctx& c, IbState& s, const int* u, double alpha, double threshold, 
     const int m = 3 * s.n;
     projection(c, s, u, s.cg_uc.p);
     zero_finest(c, s.face_aux2);
-    et_h_s_e(c, s, s.cg_f.p, s.cg_Ap.p, alpha);
+    et_h_s_e(c, s, s.cg_f.p, s.cg_Ap.p, alpha, true);
     launch_cg_init(c, s.cg_uc.p, s.cg_Ap.p, s.cg_r.p, s.cg_p.p, m, s.cg_ctl.p, max_iter);
     launch_cg_dot(c, s.cg_r.p, s.cg_r.p, nullptr, nullptr, m, s.cg_sc.p, nullptr, nullptr);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
@@ -751,7 +752,7 @@ void ns_ib_stage(Ctx& c, int stage, double alpha, double threshold, int max_iter
     launch_op(c, 2, pin, 3, pc, 1, ol.list[l].p, ol.dx[l].p, (int)ol.list[l].n, 1.0);
     launch_zero_blocks(c, pc[0], s.corr_list.p, s.n_corr);
     if (s.clean_base) launch_face_planes(c, pc[0], s.cb_list.p, s.cb_faces.p, s.n_cb, 2);
-    poisson_apply_lgf(c, s.cell_aux2, s.cell_aux2, IBLGF_IB2AMR);
+    poisson_apply_lgf(c, s.cell_aux2, s.cell_aux2, IBLGF_IB2AMR, false);  // clean since the force solve
     launch_axpby(c, c.field(d_field), c.field(s.cell_aux2), -1.0, 1);
     gradient_d();
     smearing(c, s, s.cg_f.p, face_aux, false);

@@ -302,7 +302,7 @@ class Step
             launch_op(c, 3, pin, 3, pout, 3, s.nc[l].p, s.nc_dx[l].p, (int)s.nc[l].n, 1.0);
         }
         clean_leaf_correction_boundary(s.edge_aux, bl, true);
-        for (int k = 0; k < 3; ++k) poisson_apply_lgf(c, s.edge_aux.id[k], s.stream_f.id[k], IBLGF_STREAM);
+        for (int k = 0; k < 3; ++k) poisson_apply_lgf(c, s.edge_aux.id[k], s.stream_f.id[k], IBLGF_STREAM, k == 0);
         // refresh_correction_only: curl_transpose on the base level only
         op(4, {&s.stream_f}, u, bl, -1.0);
         down_to_correction(u);
@@ -600,9 +600,6 @@ void ns_step(Ctx& c, const int* u, int p, double dt, double Re, double* T, int n
             cudaGraph_t g = nullptr;
             IBLGF_CUDA(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeRelaxed));
             bool ok = true;
-            // a step's first solve cleans correction_tmp by itself, so the
-            // recorded order holds whatever ran before a replay
-            c.capturing_step = true;
             try
             {
                 st.time_step(uf, pf, false);
@@ -611,7 +608,6 @@ void ns_step(Ctx& c, const int* u, int p, double dt, double Re, double* T, int n
             {
                 ok = false;
             }
-            c.capturing_step = false;
             const cudaError_t e = cudaStreamEndCapture(c.stream, &g);
             if (!ok || e != cudaSuccess || !g || cudaGraphInstantiate(&s.graph, g, 0) != cudaSuccess)
             {
@@ -619,7 +615,6 @@ void ns_step(Ctx& c, const int* u, int p, double dt, double Re, double* T, int n
                 if (g) cudaGraphDestroy(g);
                 s.graph = nullptr;
                 s.graph_failed = true;
-                c.correction_zero = false;
                 c.launches = l0;
                 st.time_step(uf, pf, false);  // nothing of the failed capture ran
             }

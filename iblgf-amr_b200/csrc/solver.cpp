@@ -1845,7 +1845,7 @@ void poisson_release(Ctx& c)
     c.ext[Ctx::kExtOpLists].reset();
 }
 
-void poisson_apply_lgf(Ctx& c, int src, int tgt, int fmm_type)
+void poisson_apply_lgf(Ctx& c, int src, int tgt, int fmm_type, bool clean_correction)
 {
     need_single(c);
     if (!c.finalized) throw Error(IBLGF_EINVAL, "domain not finalized");
@@ -1853,19 +1853,10 @@ void poisson_apply_lgf(Ctx& c, int src, int tgt, int fmm_type)
     PoissonLists& pl = poisson_lists(c);
     double* st = c.field(c.f_source_tmp);
     double* tt = c.field(c.f_target_tmp);
-    double* ct = c.fields[c.f_correction_tmp]->d.p;
+    double* ct = c.field(c.f_correction_tmp);
     const size_t elems = c.field_elems();
-    // the solves without a source correction leave correction_tmp zero; one
-    // recorded in a graph by the caller may be replayed after any other solve,
-    // so it cleans the field itself
-    if (fmm_type != IBLGF_AMR2AMR)
-    {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        if (!c.capturing_step) IBLGF_CUDA(cudaStreamIsCapturing(c.stream, &cs));
-        const bool caller = cs != cudaStreamCaptureStatusNone;
-        if (!c.correction_zero || caller) launch_fill_zero(c, ct, elems);
-        c.correction_zero = !caller;
-    }
+    // the solves without a source correction leave correction_tmp zero
+    if (fmm_type != IBLGF_AMR2AMR && clean_correction) launch_fill_zero(c, ct, elems);
     if (fmm_type == IBLGF_IB2AMR)
     {
         // finest-level interior copy, coarsified (cell mesh), one sweep per
@@ -1913,7 +1904,6 @@ void poisson_apply_lgf(Ctx& c, int src, int tgt, int fmm_type)
     // correction_tmp by the correction, so only the blocks at and above it are
     // zeroed, unless a switch leaves these out
     launch_solve_begin(c, c.field(src), st, tt, ct, c.subtract_non_leaf || !c.use_correction);
-    c.correction_zero = false;
     const int bl = c.tree.base_level, depth = c.tree.depth;
     for (int ls = depth - 2; ls >= bl; --ls) launch_tp(c, pl.coarsify[ls], st, st, 4, 0);
     for (int l = bl; l < depth; ++l)
