@@ -330,7 +330,7 @@ struct Ctx
 
     // device octant data
     DevBuf<int> d_bbase, d_nbr;
-    DevBuf<int> d_flags;  // per octant: bit 0 leaf, bit 1 correction, bit 2 at or above the base level
+    DevBuf<int> d_flags;  // per octant: bit 0 leaf, bit 1 correction, bit 2 not written by interpolation
     // leaf blocks in canonical order and the device staging of their
     // interiors (leaf-interior field transfers); rebuilt with the domain
     DevBuf<int> d_leaf_blocks;
@@ -674,7 +674,7 @@ void launch_leaf_copy_vf(Ctx& c, const double* const* src, double* const* dst, i
 void launch_zero_blocks_vf(Ctx& c, double* const* f, int m, const int* list, int n);
 void launch_copy_interior_vf(Ctx& c, const double* const* src, double* const* dst, int m, const int* list, int n);
 // start of an FMM sweep (FmmPlan::begin entries) and of a solve (st = leaves of
-// src, else 0; tt = ct = 0 at and above the base level, everywhere if zero)
+// src, else 0; tt = ct = 0 where no interpolation writes, everywhere if zero)
 void launch_sweep_begin(Ctx& c, const int* entries, int n, const double* src, double* fs, double* ft);
 void launch_solve_begin(Ctx& c, const double* src, double* st, double* tt, double* ct, bool zero);
 // correction_tmp of the listed child blocks from target_tmp (and, on correction

@@ -473,16 +473,19 @@ void domain_finalize(Ctx& c)
     c.f_fmm_t = field_create(c);
 }
 
-// the octants' flags on the device; bit 2: no parent level among the mesh levels
+// the octants' flags on the device; bit 2: no level loop's interpolation writes
+// the octant (at or above the base level, or its parent is not an octant:
+// imported lists may leave parents out)
 void upload_flags(Ctx& c)
 {
     std::vector<int> f(c.flags);
+    auto mark = [&f](const Ctx& s, int off) {
+        for (int o = 0; o < s.n_oct; ++o)
+            if (s.levels[o] <= s.tree.base_level || s.parent[o] < 0) f[off + o] |= 4;
+    };
     if (c.batch)
-        for (size_t i = 0; i < c.sub.size(); ++i)
-            for (int o = 0; o < c.sub[i]->n_oct; ++o)
-                f[c.sub_off[i] + o] |= c.sub[i]->levels[o] <= c.sub[i]->tree.base_level ? 4 : 0;
-    else
-        for (int o = 0; o < c.n_oct; ++o) f[o] |= c.levels[o] <= c.tree.base_level ? 4 : 0;
+        for (size_t i = 0; i < c.sub.size(); ++i) mark(*c.sub[i], c.sub_off[i]);
+    else mark(c, 0);
     c.d_flags.upload(f, c.stream);
     IBLGF_CUDA(cudaStreamSynchronize(c.stream));  // the host array goes out of scope
 }
@@ -1900,9 +1903,9 @@ void poisson_apply_lgf(Ctx& c, int src, int tgt, int fmm_type, bool clean_correc
         }
         return;
     }
-    // below the base level target_tmp is assigned by the interpolation and
-    // correction_tmp by the correction, so only the blocks at and above it are
-    // zeroed, unless a switch leaves these out
+    // children are assigned by the interpolation (target_tmp) and the correction
+    // (correction_tmp), so only the other blocks are zeroed, unless a switch
+    // leaves these out
     launch_solve_begin(c, c.field(src), st, tt, ct, c.subtract_non_leaf || !c.use_correction);
     const int bl = c.tree.base_level, depth = c.tree.depth;
     for (int ls = depth - 2; ls >= bl; --ls) launch_tp(c, pl.coarsify[ls], st, st, 4, 0);

@@ -54,3 +54,30 @@ def test_stream_solve_clears_correction(route):
     torch.cuda.synchronize()
     g.apply_lgf(fs, ft, B.STREAM)
     assert not g.download(corr).any()
+
+
+def test_octants_without_a_parent():
+    """An imported octant list may leave out an octant whose children it has: no interpolation writes these
+    children, and every solve starts them from zero."""
+    e = 6
+    args = ((-4 * e,) * 3, (8 * e,) * 3, e, 0.5, [((-2 * e,) * 3, (4 * e,) * 3)])
+    whole = B.Solver(*args, n_levels=1, predicate=lambda base, ext, rl, diff: rl == 0 and tuple(base) == (0, 0, 0))
+    refined = [o for o in range(whole.n) if whole.levels[o] == whole.base_level and not whole.flags[o] & 3]
+    assert refined
+    keep = np.array([o not in refined for o in range(whole.n)])
+    imp = (whole.keys[keep], whole.flags[keep])
+    rng = np.random.default_rng(4)
+    a, b = rng.standard_normal((2, int(keep.sum()), e + 2, e + 2, e + 2))
+    out = []
+    for first in (None, a):
+        g = B.Solver(*args, import_octants=imp)
+        assert np.any((g.levels == g.base_level + 1) & (g.flags & 1))
+        fs, ft = g.field(), g.field()
+        for x in (first, b):
+            if x is None:
+                continue
+            g.upload(fs, x)
+            g.apply_lgf(fs, ft)
+        out.append(g.download(ft))
+    assert out[0].any()
+    np.testing.assert_array_equal(out[1], out[0])
