@@ -1753,7 +1753,10 @@ bool if_level_direct(Ctx& c, PoissonLists& pl, int l, bool ib, int n, const int*
     c.stats[1] += n * lev.n_src;
     c.stats[2] += n * lev.n_tgt;
     c.stats[3] += n * lev.n_pairs;
+    Timer tm(c);
+    for (int i = 0; i < 4; ++i) tm.mark(i);
     launch_ge_direct(c, lev.tgt.p, lev.src.p, lev.n, from, to, n, ge, 1.0, true);
+    tm.mark(4);
     return true;
 }
 }  // namespace

@@ -1,5 +1,5 @@
 """Results that do not depend on what a context ran before: scratch fields
-that a solve leaves behind."""
+that a solve leaves behind or starts from, and phase times on every route."""
 import numpy as np
 import pytest
 
@@ -81,3 +81,16 @@ def test_octants_without_a_parent():
         out.append(g.download(ft))
     assert out[0].any()
     np.testing.assert_array_equal(out[1], out[0])
+
+
+@pytest.mark.parametrize("direct", [True, False])
+def test_integrating_factor_phase_times(direct):
+    """iblgf_profile_read covers the integrating factor's sums on both of its routes."""
+    case = S.VortexRingNS("small")
+    g = solver(case)
+    g.ge_direct(direct)
+    fs, ft = g.field(np.ones((g.n, g.Nb, g.Nb, g.Nb))), g.field()
+    g.apply_if(fs, ft, 1e-3)
+    g.profile(True)
+    g.apply_if(fs, ft, 1e-3)
+    assert g.profile_read()[2] > 0
