@@ -438,6 +438,17 @@ struct Ctx
         return static_cast<T*>(ext[i].get());
     }
 
+    // moves on whenever device memory that a recorded time step's launches may
+    // hold is replaced (work buffers, spectra and kernel tables, plans, points):
+    // a step recorded before is not replayed
+    long long step_epoch = 0;
+    void grow(DevBuf<char>& b, size_t bytes)
+    {
+        if (b.n >= bytes) return;
+        ++step_epoch;
+        b.alloc(bytes);
+    }
+
     size_t block_elems() const { return (size_t)Nb * Nb * Nb; }
     size_t field_elems() const { return (size_t)n_oct * block_elems(); }
     size_t cplx_bytes() const { return cfg.precision == IBLGF_FP32 ? 8 : 16; }

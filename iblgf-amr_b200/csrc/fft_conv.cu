@@ -788,11 +788,6 @@ __global__ void __launch_bounds__(NB * NB, 2) inv_fused_kernel(const cx<RA>* __r
     for (int i = 0; i < ZH; ++i) out[i] = assign ? scale * (y0 + 2.0 * sx[i]) : out[i] + scale * (y0 + 2.0 * sx[i]);
 }
 
-void ensure(DevBuf<char>& b, size_t bytes)
-{
-    if (b.n < bytes) b.alloc(bytes);
-}
-
 template<class R, int NB>
 struct Conv
 {
@@ -824,7 +819,7 @@ struct Conv
         if constexpr (pfa_extent(NB)) forward_pfa(c, field, d_item_oct, n, spec);
         else
         {
-            ensure(c.d_w, (size_t)n * NB * NP * sizeof(cx<R>));
+            c.grow(c.d_w, (size_t)n * NB * NP * sizeof(cx<R>));
             cx<R>* W = (cx<R>*)c.d_w.p;
             launch_fwd_xy_rows(c, field, d_item_oct, n, W);
             fwd_z_kernel<R, R, NB, NB><<<dim3(n, (NP + 127) / 128), 128, 0, c.stream>>>(W, nullptr, (cx<R>*)spec);
@@ -969,7 +964,7 @@ void launch_spectra(Ctx& c, const std::vector<std::array<int, 5>>& new_slots)
     // new_slots: {slot, ld, bx, by, bz}; processed in batches of 64
     const int P = c.P;
     const size_t wbytes = (size_t)64 * P * P * c.Nb * 16;
-    ensure(c.d_w, wbytes);
+    c.grow(c.d_w, wbytes);
     for (size_t b0 = 0; b0 < new_slots.size(); b0 += 64)
     {
         const size_t nb = std::min<size_t>(64, new_slots.size() - b0);
@@ -1097,7 +1092,7 @@ void launch_conv_block(Ctx& c, const double* src, const double* kernel, double* 
     const double s = scale / ((double)c.P * c.P * c.P);
     dispatch(c, [&](auto cv) {
         using CV = decltype(cv);
-        ensure(c.conv_work, CV::conv_bytes);
+        if (c.conv_work.n < CV::conv_bytes) c.conv_work.alloc(CV::conv_bytes);
         CV::conv_block(c, src, kernel, out, s, c.conv_work.p);
     });
     IBLGF_CUDA(cudaGetLastError());

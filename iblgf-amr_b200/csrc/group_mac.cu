@@ -442,6 +442,7 @@ int combo_table(Ctx& c, int ld, const std::vector<int>& slots)
         if (idx) IBLGF_CUDA(cudaMemcpyAsync(nb.p, c.d_combo.p, (size_t)idx * tbytes, cudaMemcpyDeviceToDevice, c.stream));
         IBLGF_CUDA(cudaStreamSynchronize(c.stream));
         c.d_combo = std::move(nb);
+        ++c.step_epoch;
         c.combo_cap = cap;
     }
     DevBuf<int> d_slots;

@@ -58,17 +58,20 @@ void relpos(int mesh, int comp, int rp[3])
 
 // What a captured time step depends on besides the device data: the field
 // ids, dt, Re, the frame velocity (a launch argument, and whether the
-// frame-velocity update launches at all) and the Poisson solver's switches
-// (which launches a solve makes)
+// frame-velocity update launches at all), the Poisson solver's switches
+// (which launches a solve makes) and the memory that the launches hold
+// (Ctx::step_epoch)
 struct StepKey
 {
     int u[3] = {-1, -1, -1}, p = -1;
     double dt = 0.0, Re = 0.0, fv[3] = {0.0, 0.0, 0.0};
     bool corr = true, snl = false;
+    long long epoch = -1;
     bool operator==(const StepKey& o) const
     {
         return u[0] == o.u[0] && u[1] == o.u[1] && u[2] == o.u[2] && p == o.p && dt == o.dt && Re == o.Re &&
-               fv[0] == o.fv[0] && fv[1] == o.fv[1] && fv[2] == o.fv[2] && corr == o.corr && snl == o.snl;
+               fv[0] == o.fv[0] && fv[1] == o.fv[1] && fv[2] == o.fv[2] && corr == o.corr && snl == o.snl &&
+               epoch == o.epoch;
     }
 };
 
@@ -88,8 +91,8 @@ struct NsState
     int sm_n[2] = {0, 0};
     double T_last_vel_refresh = 0.0;  // ifherk.hpp:1980
     bool force_refresh = false;       // base_mesh_update of the last adaptation
-    // one captured time step (steps without an immersed boundary): replayed
-    // while everything the capture baked in stays the same (g_key)
+    // one captured time step: replayed while everything the capture baked in
+    // stays the same (g_key)
     cudaGraphExec_t graph = nullptr;
     StepKey g_key;
     bool graph_failed = false;
@@ -581,6 +584,7 @@ void ns_step(Ctx& c, const int* u, int p, double dt, double Re, double* T, int n
         for (int k = 0; k < 3; ++k) key.fv[k] = opt.frame_vel[k];
         key.corr = c.use_correction;
         key.snl = c.subtract_non_leaf;
+        key.epoch = c.step_epoch;
         const bool same = s.graph && s.g_key == key;
         if (graphable && same)
         {
@@ -609,6 +613,7 @@ void ns_step(Ctx& c, const int* u, int p, double dt, double Re, double* T, int n
                 ok = false;
             }
             const cudaError_t e = cudaStreamEndCapture(c.stream, &g);
+            ok = ok && c.step_epoch == key.epoch;
             if (!ok || e != cudaSuccess || !g || cudaGraphInstantiate(&s.graph, g, 0) != cudaSuccess)
             {
                 cudaGetLastError();
@@ -629,6 +634,7 @@ void ns_step(Ctx& c, const int* u, int p, double dt, double Re, double* T, int n
         else
         {
             st.time_step(uf, pf, false);
+            key.epoch = c.step_epoch;  // what the step itself built is there now
             s.w_key = key;
         }
         ++s.steps_done;

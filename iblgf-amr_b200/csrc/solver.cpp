@@ -266,6 +266,7 @@ void domain_set_owner(Ctx& c, const int* owner, int rank, iblgf_exchange_fn fn, 
         c.owner.clear();
     c.exchange_fn = fn;
     c.exchange_user = user;
+    ++c.step_epoch;
     c.plans.clear();
 }
 
@@ -423,6 +424,7 @@ void build_ib_masks(Ctx& c, std::vector<int>& ib)
         upward_pass(c, lv, mv);
     }
     // plans and lists built from the previous masks are stale
+    ++c.step_epoch;
     if (auto* pl = c.ext_get<PoissonLists>(Ctx::kExtPLists))
         for (auto it = pl->if_levels.begin(); it != pl->if_levels.end();)
             it = it->first.second ? pl->if_levels.erase(it) : std::next(it);
@@ -1205,6 +1207,7 @@ std::unique_ptr<FmmPlan> upload_plan(Ctx& c, const HostPlan& h)
                                            cudaMemcpyDeviceToDevice, c.stream));
             IBLGF_CUDA(cudaStreamSynchronize(c.stream));
             c.d_spec = std::move(nb);
+            ++c.step_epoch;
             c.spec_cap = cap;
         }
         launch_spectra(c, new_slots);
@@ -1307,11 +1310,6 @@ void prebuild_plans(Ctx& c, const std::vector<std::tuple<int, int, int>>& keys)
 
 namespace
 {
-void ensure_bytes(DevBuf<char>& b, size_t bytes)
-{
-    if (b.n < bytes) b.alloc(bytes);
-}
-
 struct Timer
 {
     // phase events recorded on the context stream; read back (and summed) by
@@ -1422,10 +1420,10 @@ void run_sweep(Ctx& c, FmmPlan& p, int src, int tgt, double dx_level, double add
     if (!p.empty() && !direct)
     {
         // the source spectra and one zero row after them (absent MAC candidates read it)
-        ensure_bytes(c.d_src_spec, (size_t)(p.n_src + 1) * c.NC * cb);
+        c.grow(c.d_src_spec, (size_t)(p.n_src + 1) * c.NC * cb);
         launch_fill_zero(c, reinterpret_cast<double*>(c.d_src_spec.p + (size_t)p.n_src * c.NC * cb),
                          c.NC * cb / sizeof(double));
-        ensure_bytes(c.d_acc, (size_t)p.n_tgt * c.NC * cb);
+        c.grow(c.d_acc, (size_t)p.n_tgt * c.NC * cb);
         launch_forward_sources(c, fs, p.src_oct.p, p.n_src, c.d_src_spec.p);
     }
     tm.mark(2);
@@ -1626,6 +1624,30 @@ void apply_op_octants(Ctx& c, int op, const int* in, int n_in, const int* out, i
     IBLGF_CUDA(cudaStreamSynchronize(c.stream));  // the lists are freed on return
 }
 
+namespace
+{
+// one more integrating-factor table, on the host and on the device
+int add_ge(Ctx& c, double alpha, const std::vector<double>& f)
+{
+    size_t from = c.ge_host.size(), n = from + f.size();
+    DevBuf<double> nb;
+    if (c.d_ge.n < n) nb.alloc(2 * n);
+    c.ge_host.insert(c.ge_host.end(), f.begin(), f.end());
+    if (nb.n)
+    {
+        ++c.step_epoch;
+        c.d_ge = std::move(nb);
+        from = 0;
+    }
+    const int idx = (int)c.ge_index.size();
+    c.ge_index.emplace(alpha, idx);
+    IBLGF_CUDA(cudaMemcpyAsync(c.d_ge.p + from, c.ge_host.data() + from, (n - from) * sizeof(double),
+                               cudaMemcpyHostToDevice, c.stream));
+    IBLGF_CUDA(cudaStreamSynchronize(c.stream));
+    return idx;
+}
+}  // namespace
+
 // e^{-2 alpha} I_n(2 alpha), n = 0..stride-1, by Miller's backward recurrence
 // normalised with e^x = I_0 + 2 sum I_k (A&S 9.6.26, 9.6.37)
 int ge_table(Ctx& c, double alpha)
@@ -1641,12 +1663,7 @@ int ge_table(Ctx& c, double alpha)
     {
         // e^0 I_n(0) = [n == 0]: the identity (the recurrence divides by x)
         f[0] = 1.0;
-        const int idx = (int)c.ge_index.size();
-        c.ge_index.emplace(alpha, idx);
-        c.ge_host.insert(c.ge_host.end(), f.begin(), f.end());
-        c.d_ge.upload(c.ge_host, c.stream);
-        IBLGF_CUDA(cudaStreamSynchronize(c.stream));
-        return idx;
+        return add_ge(c, alpha, f);
     }
     const int m = nmax + 30 + (int)std::ceil(std::sqrt(90.0 * x));
     double a = 0.0, b = 1e-280, sum = 0.0;
@@ -1668,12 +1685,7 @@ int ge_table(Ctx& c, double alpha)
     f[0] = b;
     const double norm = b + 2.0 * sum;
     for (auto& v : f) v /= norm;
-    const int idx = (int)c.ge_index.size();
-    c.ge_index.emplace(alpha, idx);
-    c.ge_host.insert(c.ge_host.end(), f.begin(), f.end());
-    c.d_ge.upload(c.ge_host, c.stream);
-    IBLGF_CUDA(cudaStreamSynchronize(c.stream));
-    return idx;
+    return add_ge(c, alpha, f);
 }
 
 namespace

@@ -1,10 +1,12 @@
 """Results that do not depend on what a context ran before: scratch fields
-that a solve leaves behind or starts from, and phase times on every route."""
+that a solve leaves behind or starts from, time steps recorded before a call
+that replaces memory they hold, and phase times on every route."""
 import numpy as np
 import pytest
 
 import iblgf_b200 as B
 import iblgf_setups as S
+import oracle_lib as O
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +96,40 @@ def test_integrating_factor_phase_times(direct):
     g.profile(True)
     g.apply_if(fs, ft, 1e-3)
     assert g.profile_read()[2] > 0
+
+
+@pytest.mark.parametrize("call", ["apply_if", "stream", "refresh", "points"])
+def test_step_after_replaced_memory(call):
+    """A recorded step is not replayed over memory that a later call replaced: a kernel table, spectra and work
+    buffers of a sweep that was not there before, the immersed-boundary points. Against a context that launches every
+    step directly (it takes phase times), bit for bit with the same MAC variant."""
+    ib = call == "points"
+    case = S.SphereIB("small") if ib else S.VortexRingNS("small")
+    out = []
+    for direct in (False, True):
+        g = solver(case)
+        g.mac_variant(0)
+        if ib:
+            X = O.sphere_points(case.dx_base, g.depth - 1 - g.base_level, case.ibph)
+            g.ib_set_points(X, case.Re)
+            g.ns_options((-1.0, 0.0, 0.0))
+            u, dt = case.velocity(g), 0.01
+        else:
+            u, dt = case.initial_velocity(g), case.dt()
+        uf, pf = [g.field(u[k]) for k in range(3)], g.field()
+        g.profile(direct)
+        T = g.ns_step(uf, pf, dt, case.Re, 0.0, 3)  # direct, recorded, replayed
+        fs, ft = g.field(u[0]), g.field()
+        if call == "apply_if":
+            for k in range(20):
+                g.apply_if(fs, ft, 0.01 + 1e-3 * k)
+        elif call == "stream":
+            g.apply_lgf(fs, ft, B.STREAM)
+        elif call == "refresh":
+            T = g.ns_step(uf, pf, dt, case.Re, T + 1e6, 1)
+        else:
+            g.ib_set_points(X[: len(X) // 2], case.Re)
+        g.ns_step(uf, pf, dt, case.Re, T, 3)
+        out.append(np.stack([g.download(f) for f in uf + [pf]]))
+    assert out[0].any()
+    np.testing.assert_array_equal(out[0], out[1])
