@@ -644,6 +644,7 @@ int iblgf_mac_variant(iblgf_ctx* x, int variant)
         if (variant < -1 || variant > 3)
             throw iblgf_b200::Error(IBLGF_EINVAL, "MAC variant must be -1, 0, 1, 2 or 3");
         c.mac_variant_forced = variant;
+        ++c.step_epoch;
     });
 }
 
@@ -651,6 +652,7 @@ int iblgf_ge_direct(iblgf_ctx* x, int enable)
 {
     return guard(x, [&](iblgf_b200::Ctx& c) {
         c.ge_direct_enabled = enable != 0;
+        ++c.step_epoch;
     });
 }
 

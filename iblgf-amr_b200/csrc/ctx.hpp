@@ -439,8 +439,9 @@ struct Ctx
     }
 
     // moves on whenever device memory that a recorded time step's launches may
-    // hold is replaced (work buffers, spectra and kernel tables, plans, points):
-    // a step recorded before is not replayed
+    // hold is replaced (work buffers, spectra and kernel tables, plans, points)
+    // or a switch that selects its launches is set: a step recorded before is
+    // not replayed
     long long step_epoch = 0;
     void grow(DevBuf<char>& b, size_t bytes)
     {

@@ -526,6 +526,7 @@ void ib_warmstart(Ctx& c, int mode, int train_steps, int epochs, double lr, unsi
     if (mode == 1 && (train_steps <= 0 || epochs <= 0 || !(lr > 0)))
         throw Error(IBLGF_EINVAL, "learned warm start needs train_steps, epochs and lr > 0");
     WarmStart& w = s.ws;
+    ++c.step_epoch;
     w = WarmStart();
     w.mode = mode;
     w.train_steps = train_steps;

@@ -59,19 +59,21 @@ void relpos(int mesh, int comp, int rp[3])
 // What a captured time step depends on besides the device data: the field
 // ids, dt, Re, the frame velocity (a launch argument, and whether the
 // frame-velocity update launches at all), the Poisson solver's switches
-// (which launches a solve makes) and the memory that the launches hold
-// (Ctx::step_epoch)
+// (which launches a solve makes), the force CG's settings and the memory that
+// the launches hold (Ctx::step_epoch)
 struct StepKey
 {
     int u[3] = {-1, -1, -1}, p = -1;
     double dt = 0.0, Re = 0.0, fv[3] = {0.0, 0.0, 0.0};
     bool corr = true, snl = false;
+    double cg_threshold = 0.0;
+    int cg_max_iter = 0;
     long long epoch = -1;
     bool operator==(const StepKey& o) const
     {
         return u[0] == o.u[0] && u[1] == o.u[1] && u[2] == o.u[2] && p == o.p && dt == o.dt && Re == o.Re &&
                fv[0] == o.fv[0] && fv[1] == o.fv[1] && fv[2] == o.fv[2] && corr == o.corr && snl == o.snl &&
-               epoch == o.epoch;
+               cg_threshold == o.cg_threshold && cg_max_iter == o.cg_max_iter && epoch == o.epoch;
     }
 };
 
@@ -582,6 +584,8 @@ void ns_step(Ctx& c, const int* u, int p, double dt, double Re, double* T, int n
         key.Re = Re;
         const NsOptions& opt = ns_opt(c);
         for (int k = 0; k < 3; ++k) key.fv[k] = opt.frame_vel[k];
+        key.cg_threshold = opt.cg_threshold;
+        key.cg_max_iter = opt.cg_max_iter;
         key.corr = c.use_correction;
         key.snl = c.subtract_non_leaf;
         key.epoch = c.step_epoch;

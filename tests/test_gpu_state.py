@@ -1,6 +1,6 @@
 """Results that do not depend on what a context ran before: scratch fields
 that a solve leaves behind or starts from, time steps recorded before a call
-that replaces memory they hold, and phase times on every route."""
+that changes what they hold, and phase times on every route."""
 import numpy as np
 import pytest
 
@@ -98,12 +98,13 @@ def test_integrating_factor_phase_times(direct):
     assert g.profile_read()[2] > 0
 
 
-@pytest.mark.parametrize("call", ["apply_if", "stream", "refresh", "points"])
-def test_step_after_replaced_memory(call):
-    """A recorded step is not replayed over memory that a later call replaced: a kernel table, spectra and work
-    buffers of a sweep that was not there before, the immersed-boundary points. Against a context that launches every
-    step directly (it takes phase times), bit for bit with the same MAC variant."""
-    ib = call == "points"
+@pytest.mark.parametrize("call", ["apply_if", "stream", "refresh", "points", "ge_direct", "cg", "warmstart"])
+def test_step_after_another_call(call):
+    """A recorded step is not replayed over memory that a later call replaced (a kernel table, spectra and work
+    buffers of a sweep that was not there before, the immersed-boundary points), nor past a switch that a later call
+    set. Against a context that launches every step directly (it takes phase times), bit for bit with the same MAC
+    variant."""
+    ib = call in ("points", "cg", "warmstart")
     case = S.SphereIB("small") if ib else S.VortexRingNS("small")
     out = []
     for direct in (False, True):
@@ -127,8 +128,14 @@ def test_step_after_replaced_memory(call):
             g.apply_lgf(fs, ft, B.STREAM)
         elif call == "refresh":
             T = g.ns_step(uf, pf, dt, case.Re, T + 1e6, 1)
-        else:
+        elif call == "points":
             g.ib_set_points(X[: len(X) // 2], case.Re)
+        elif call == "ge_direct":
+            g.ge_direct(False)
+        elif call == "cg":
+            g.ns_options((-1.0, 0.0, 0.0), cg_threshold=1e-8)
+        else:
+            g.ib_warmstart(2)
         g.ns_step(uf, pf, dt, case.Re, T, 3)
         out.append(np.stack([g.download(f) for f in uf + [pf]]))
     assert out[0].any()
