@@ -86,6 +86,30 @@ def test_conv_block_extents(e, precision, tol):
         assert rel_linf(out.cpu().numpy() - base, ref) < tol
 
 
+# the 2-norm error is the mean over the block's 512 and 5832 nodes and six inputs, within 2 % from seed to seed; direct
+# sums of 15 and 35 terms in the inverse z and y passes give 8.3e-16 at both, the prime-factor sums 7.5e-16 and 7.2e-16
+@pytest.mark.parametrize("e,bound", [(6, 7.85e-16), (16, 7.75e-16)])
+def test_conv_block_rounding(e, bound):
+    """The FP64 convolution against extended precision where P = 2 Nb - 1 splits into coprime factors."""
+    torch = pytest.importorskip("torch")
+    N, P = e + 2, 2 * e + 3
+    g = B.Solver((-2 * e,) * 3, (4 * e,) * 3, e, 1.0, [((-e,) * 3, (2 * e,) * 3)])
+    err = []
+    for seed in range(6):
+        rng = np.random.default_rng(seed)
+        src, ker = rng.standard_normal((N, N, N)), rng.standard_normal((P, P, P))
+        ref, lk = np.zeros((N, N, N), np.longdouble), ker.astype(np.longdouble)
+        for z, y, x in np.ndindex(N, N, N):
+            ref += np.longdouble(src[z, y, x]) * lk[N - 1 - z:P - z, N - 1 - y:P - y, N - 1 - x:P - x]
+        out = torch.zeros(N ** 3, dtype=torch.float64, device="cuda")
+        ts, tk = torch.tensor(src.ravel(), device="cuda"), torch.tensor(ker.ravel(), device="cuda")
+        torch.cuda.synchronize()
+        g.conv_block(ts.data_ptr(), tk.data_ptr(), out.data_ptr(), 1.0)
+        d = out.cpu().numpy().reshape(N, N, N).astype(np.longdouble) - ref
+        err.append(float(np.sqrt((d ** 2).sum() / (ref ** 2).sum())))
+    assert np.mean(err) < bound, np.mean(err)
+
+
 @pytest.mark.parametrize("nb,nm", [(3, 1), (7, 5), (18, 7), (40, 3)])
 @pytest.mark.parametrize("op", ["laplace", "gradient", "divergence", "curl", "curl_transpose"])
 def test_fourier_operators_extents(op, nb, nm):
