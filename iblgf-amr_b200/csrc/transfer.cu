@@ -672,6 +672,17 @@ void launch_tp_typed(Ctx& c, const TpTasks& t, const TpFields& f, int n, const i
                 }
         }
     int W = width <= 2 ? 2 : (width <= 5 ? 5 : 0);
+    if (W == 2 && mode == 0)
+        // tp_band2_kernel takes one sending child per receiving node and axis and
+        // nothing on the buffer nodes; matrices that give more go another way
+        for (int s = 0; s < 2 && base[s] >= 0; ++s)
+            for (int m = 0; m < NB; ++m)
+            {
+                int children = 0;
+                for (int k = 0; k < 2; ++k)
+                    children += std::any_of(mt.m[s][k] + m * NB, mt.m[s][k] + (m + 1) * NB, [](T v) { return v != (T)0; });
+                if (children > (m > 0 && m < NB - 1 ? 1 : 0)) W = 5;
+            }
     if (W == 5)
     {
         // the smallest starts that never move back and cover the rows; they move
