@@ -120,7 +120,6 @@ HostPlan merge_plans(const std::vector<std::pair<HostPlan, int>>& parts)
         for (int x : h.gtgt)
             m.gtgt.push_back(x < 0 ? -1 : (x < h.n_csr_tgt ? csrb[i] + x : grpb[i] + x - h.n_csr_tgt));
         m.n_groups += h.n_groups;
-        m.max_tile_src = std::max(m.max_tile_src, h.max_tile_src);
     }
     std::vector<std::array<int, 4>> u = m.all_keys;
     std::sort(u.begin(), u.end());

@@ -155,8 +155,8 @@ struct TpTasks  // tensor-product transfer tasks of one tree level
     DevBuf<int> task_cid;       // child id (0..7)
 };
 
-// sibling groups per group-MAC tile; the kernel's thread rows x groups per
-// row cover exactly this many
+// sibling groups per tile of the plan's group lists, which the block-Toeplitz
+// MAC takes in up to three parts of kToeplitzPart
 constexpr int kGroupTileCap = 32;
 // bundles of two sibling groups per tile of the direct MAC, at most
 constexpr int kMacTile = 96;
@@ -164,8 +164,9 @@ constexpr int kMacTile = 96;
 constexpr int kMacStage = 2;
 // bundles of a table up to which its tile is split over four warps per bundle
 // (the CTA has 16 warps in FP32, 12 in FP64): the tiles of the coarse levels'
-// tables, 1 to 4 bundles, then take 5 instead of 15 us of an SM. At 16 to 24
-// bundles the split costs a third (vortex ring, 1.36 against 1.09 ms).
+// tables, 1 to 4 bundles, then take 5 instead of 15 us of an SM. Up to 3 only: the
+// vortex ring step and the amr_3level solve 0.6 % slower; 4, 5 and 8 are equal to
+// 0.2 %; at 16 to 24 bundles the split costs a third (ring, 1.36 against 1.09 ms).
 constexpr int kMacSplit = 5;
 // candidate x target rows (of 16) from which a half parent runs all of them:
 // 32 products without a branch cost about as much as 24 with
@@ -194,13 +195,12 @@ struct FmmPlan
     int n_spec_unique = 0;
     // targets handled by the general pair-list MAC come first in tgt_oct
     int n_csr_tgt = 0;
-    // sibling-group MAC: tiles of groups, staged source lists, per-group
-    // candidate sources (216, local index into the tile's staged list, 0xFFFF
-    // for none) and targets (8 child slots), LGF spectrum slot per offset
-    int n_tiles = 0, max_tile_src = 0, n_groups = 0;
+    // sibling-group MAC: tiles of groups, per-group targets (8 child slots),
+    // LGF spectrum slot per offset
+    int n_tiles = 0, n_groups = 0;
     // tile_jr: per tile kGroupTileCap x 216 source rows of its groups'
     // candidates (the zero row for absent ones)
-    DevBuf<int> tile_gptr, tile_jr, tile_tab, tile_coarse, spec_u, grp_tgt;
+    DevBuf<int> tile_gptr, tile_jr, spec_u, grp_tgt;
     DevBuf<unsigned> grp_pm;     // per group: bit n set = neighbour parent n has a candidate
     DevBuf<int> tile_combo;      // per tile: coefficient table of the block-Toeplitz MAC (its level difference)
     DevBuf<int> tile_parts;      // block-Toeplitz work: tile << 2 | part for the non-empty parts of 14 groups
@@ -223,7 +223,7 @@ struct FmmPlan
     // 27 neighbour sources (octants, -1: none)
     int n_ge = 0;
     DevBuf<int> ge_tgt, ge_src;
-    long long n_exec = 0;        // (target, source) products the MAC kernels execute
+    long long n_exec = 0;        // (target, source) products, all 64 of every present parent
     long long mac_flops = 0;     // floating-point operations of the MAC kernels per frequency
     bool adj_only = false;       // every tile takes adjacent pairs only (integrating factor)
     mutable int mac_variant = -1;  // group-MAC variant chosen by the autotuner (-1: not tuned yet)
@@ -255,7 +255,7 @@ struct HostPlan
     // source octants by neighbour offset, (ox+1) + 3 (oy+1) + 9 (oz+1), -1: none
     std::vector<int> ge_tgt, ge_src;
     std::vector<std::array<int, 4>> tab_keys;  // 343 per table
-    int n_groups = 0, max_tile_src = 0, n_spec_unique = 0;
+    int n_groups = 0, n_spec_unique = 0;
     long long n_pairs = 0, n_exec = 0;
 };
 
@@ -358,7 +358,6 @@ struct Ctx
     // Nb*Nb matrices (child bit 0 / 1): [0,1] FMM Nli, cell-centred transfers with
     // relative position 1: [2,3] interpolation, [4,5] coarsification; relative
     // position 0: [6,7] interpolation, [8,9] coarsification (injection)
-    DevBuf<double> d_mats;
     std::vector<double> h_mats;  // host copy (transfer kernels take them as launch parameters)
 
     // spectra cache: key (level_diff, bx, by, bz) -> slot; storage in the
@@ -556,7 +555,6 @@ struct IfLevel
 // device block lists of the Poisson level loop and of the level-wise operators
 struct PoissonLists
 {
-    DevBuf<int> all, leaves;
     std::vector<DevBuf<int>> level_all, level_leaves;
     // per (level, IB2xIB or not), built on first use
     std::map<std::pair<int, bool>, std::unique_ptr<IfLevel>> if_levels;
@@ -643,7 +641,7 @@ void launch_inverse_targets(Ctx& c, const FmmPlan& p, const void* acc, double* f
 // prime-factor transforms (inverse.cu) of the block extents whose P splits;
 // the direct transforms run for the others
 constexpr bool pfa_extent(int nb) { return nb == 8 || nb == 18; }
-void inverse_pfa(Ctx& c, const void* acc, const int* d_tgt_oct, int n, double scale, double* target, bool assign);
+void inverse_pfa(Ctx& c, const void* acc, const int* d_tgt_oct, int n, double scale, double* target);
 void forward_pfa(Ctx& c, const double* field, const int* d_item_oct, int n, void* spec);
 void init_pfa_constants(int device);
 // sharding (solver.cpp): the reference server's load-balanced partition and

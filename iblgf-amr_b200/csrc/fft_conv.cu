@@ -2,8 +2,8 @@
 // sm_100a (no cuFFT). Contract: include/iblgf/utilities/convolution.hpp:225-304
 // and src/utilities/convolution.cpp — a zero-padded Nb^3 source and a
 // (2Nb-1)^3 LGF block in a P^3 = (2Nb-1)^3 box, r2c, pointwise product
-// accumulated per target, c2r, window [Nb-1, 2Nb-2]^3 added into the target
-// block, scaled by dx^2 / P^3.
+// accumulated per target, c2r, window [Nb-1, 2Nb-2]^3 scaled by dx^2 / P^3 into
+// the target block.
 //
 // B200 structure (one sweep = all blocks of all tree levels at once):
 //   forward      each source block once per sweep (the reference transforms it
@@ -13,11 +13,13 @@
 //                  along x (real, Nb -> Nb half frequencies), thread (z, kx)
 //                  then column kx along y (Nb -> P)
 //     fwd_z        one thread per (ky,kx) pencil: z transform (Nb -> P)
-//   group_mac    sibling-group spectral multiply-accumulate (mac_kernel:
+//   bundle_mac   sibling-group spectral multiply-accumulate (mac_kernel:
 //                general pair-list fallback)
-//   inv_fused    one CTA per (target, half of the output planes): z inverse,
-//                y inverse and c2r along x of the extraction window, in
-//                shared memory, added into the FP64 target block
+//   inverse      assigned to the FP64 target block: one kernel for the extents
+//                with a prime-factor split (inverse.cu), for the others
+//                inv_fused, one CTA per (target, half of the output planes): z
+//                inverse, y inverse and c2r along x of the extraction window,
+//                in shared memory
 // The half spectrum is laid out [kz][ky][kx], kx < Nb (= P/2 + 1), as in the
 // reference's r2c output. Transforms are direct pruned DFTs (half of the
 // inputs zero, half of the outputs discarded). The forward loops are unrolled
@@ -66,13 +68,6 @@ __device__ __forceinline__ cx<R> ctw(int j)
         return mk<R>(c_tw32[2 * (tw_base(P) + j)], c_tw32[2 * (tw_base(P) + j) + 1]);
 }
 
-// Fully unrolled FP64 transforms at Nb = 18 exceed the register budget (the
-// scheduler hoists the loads of every term), so there the output loop stays
-// rolled and the twiddle index is carried in per-term counters; the twiddle
-// load is then one uniform constant-cache read.
-template<class R, int NB>
-constexpr bool kRollOutputs = std::is_same<R, double>::value && NB >= 18;
-
 // x and y transforms of a whole field block: thread (z, y) takes row y of
 // plane z along x (real NB -> NB half frequencies) into shared memory, then
 // thread (z, kx) takes column kx of plane z along y (NB -> P) and writes
@@ -94,34 +89,13 @@ __global__ void __launch_bounds__(NB * NB) fwd_xy_rows_kernel(const double* __re
 #pragma unroll
         for (int x = 0; x < NB; ++x) in[x] = (R)row[x];
         cx<R>* dst = s_x1 + (size_t)threadIdx.x * S;
-        if constexpr (kRollOutputs<R, NB>)
+#pragma unroll
+        for (int kx = 0; kx < NB; ++kx)
         {
-            int j[NB];  // j[x] = kx * x mod P
+            cx<R> s = mk<R>(0, 0);
 #pragma unroll
-            for (int x = 0; x < NB; ++x) j[x] = 0;
-#pragma unroll 1
-            for (int kx = 0; kx < NB; ++kx)
-            {
-                cx<R> s = mk<R>(0, 0);
-#pragma unroll
-                for (int x = 0; x < NB; ++x)
-                {
-                    rmac<R>(s, in[x], ctw<R, P>(j[x]));
-                    j[x] = j[x] + x >= P ? j[x] + x - P : j[x] + x;
-                }
-                dst[kx] = s;
-            }
-        }
-        else
-        {
-#pragma unroll
-            for (int kx = 0; kx < NB; ++kx)
-            {
-                cx<R> s = mk<R>(0, 0);
-#pragma unroll
-                for (int x = 0; x < NB; ++x) rmac<R>(s, in[x], ctw<R, P>((kx * x) % P));
-                dst[kx] = s;
-            }
+            for (int x = 0; x < NB; ++x) rmac<R>(s, in[x], ctw<R, P>((kx * x) % P));
+            dst[kx] = s;
         }
     }
     __syncthreads();
@@ -129,34 +103,13 @@ __global__ void __launch_bounds__(NB * NB) fwd_xy_rows_kernel(const double* __re
 #pragma unroll
     for (int y = 0; y < NB; ++y) v[y] = s_x1[(z * NB + y) * S + r];
     cx<R>* out = W + ((size_t)item * NB + z) * (P * NB) + r;
-    if constexpr (kRollOutputs<R, NB>)
+#pragma unroll
+    for (int ky = 0; ky < P; ++ky)
     {
-        int j[NB];  // j[y] = ky * y mod P
+        cx<R> s = mk<R>(0, 0);
 #pragma unroll
-        for (int y = 0; y < NB; ++y) j[y] = 0;
-#pragma unroll 1
-        for (int ky = 0; ky < P; ++ky)
-        {
-            cx<R> s = mk<R>(0, 0);
-#pragma unroll
-            for (int y = 0; y < NB; ++y)
-            {
-                cmac<R>(s, v[y], ctw<R, P>(j[y]));
-                j[y] = j[y] + y >= P ? j[y] + y - P : j[y] + y;
-            }
-            out[(size_t)ky * NB] = s;
-        }
-    }
-    else
-    {
-#pragma unroll
-        for (int ky = 0; ky < P; ++ky)
-        {
-            cx<R> s = mk<R>(0, 0);
-#pragma unroll
-            for (int y = 0; y < NB; ++y) cmac<R>(s, v[y], ctw<R, P>((ky * y) % P));
-            out[(size_t)ky * NB] = s;
-        }
+        for (int y = 0; y < NB; ++y) cmac<R>(s, v[y], ctw<R, P>((ky * y) % P));
+        out[(size_t)ky * NB] = s;
     }
 }
 
@@ -600,8 +553,7 @@ __device__ __forceinline__ void mac_load(cx<R> (&s)[4], const cx<R>* Sf, const u
 // of 10 warps per SM (less L1 for the source rows: +0.7 ms), packed FP32 FMAs
 // with their accumulators doubled (+0.7 ms).
 // In a split tile (bit 2 of its mode) a warp takes one group of a bundle and one
-// half (cz) of its targets: tiles whose bundles are no more than a quarter of
-// the CTA's warps. ALL: every tile is split, and the kernel keeps the registers
+// half (cz) of its targets: tables of at most kMacSplit bundles. ALL: every tile is split, and the kernel keeps the registers
 // of that path only (FP32: two CTAs per SM), for plans with few groups (8
 // groups of a uniform 64^3 solve: 52 against 73 us).
 template<class R, int NB, int NT, int MINB, bool ALL>
@@ -775,7 +727,7 @@ __global__ void __launch_bounds__(NT, MINB) bundle_mac_kernel(
 }
 
 // Fused inverse of one target block: z inverse, y inverse, c2r along x and
-// target[oct] += scale * window, with every intermediate in shared memory.
+// target[oct] = scale * window, with every intermediate in shared memory.
 // One CTA per (target, half of the NB output z-planes), NB^2 threads:
 //   z  thread per pencil (ky, kx): the P accumulators (working precision RA,
 //      widened to FP64) -> the NB/2 output planes of this half, into sV
@@ -790,7 +742,7 @@ __global__ void __launch_bounds__(NT, MINB) bundle_mac_kernel(
 template<class RA, int NB>
 __global__ void __launch_bounds__(NB * NB, 2) inv_fused_kernel(const cx<RA>* __restrict__ ACC,
                                                                const int* __restrict__ tgt_oct, double scale,
-                                                               double* __restrict__ target, int assign)
+                                                               double* __restrict__ target)
 {
     constexpr int P = 2 * NB - 1, NP = P * NB, ZH = NB / 2, S = NB + 1;
     static_assert(NB % 2 == 0, "the block splits into two halves of output planes");
@@ -856,7 +808,7 @@ __global__ void __launch_bounds__(NB * NB, 2) inv_fused_kernel(const cx<RA>* __r
     const double y0 = yrow[0].x;
     double* out = target + (size_t)tgt_oct[t] * NB * NB * NB + ((size_t)(h * ZH + zl2) * NB + yo) * NB + xh * ZH;
 #pragma unroll
-    for (int i = 0; i < ZH; ++i) out[i] = assign ? scale * (y0 + 2.0 * sx[i]) : out[i] + scale * (y0 + 2.0 * sx[i]);
+    for (int i = 0; i < ZH; ++i) out[i] = scale * (y0 + 2.0 * sx[i]);
 }
 
 template<class R, int NB>
@@ -875,13 +827,12 @@ struct Conv
         kfn<<<n, NB * NB, smem, c.stream>>>(field, d_item_oct, W);
     }
 
-    static void launch_inverse(Ctx& c, const cx<R>* acc, const int* d_tgt_oct, int n, double scale, double* target,
-                               bool assign)
+    static void launch_inverse(Ctx& c, const cx<R>* acc, const int* d_tgt_oct, int n, double scale, double* target)
     {
         const int smem = (P * NB + NB / 2 * NP) * (int)sizeof(double2);
         auto kfn = inv_fused_kernel<R, NB>;
         IBLGF_CUDA(cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        kfn<<<dim3(n, 2), NB * NB, smem, c.stream>>>(acc, d_tgt_oct, scale, target, assign ? 1 : 0);
+        kfn<<<dim3(n, 2), NB * NB, smem, c.stream>>>(acc, d_tgt_oct, scale, target);
     }
 
     static void forward_field(Ctx& c, const double* field, const int* d_item_oct, int n, void* spec)
@@ -968,14 +919,13 @@ struct Conv
         }
     }
 
-    static void inverse(Ctx& c, const void* acc, const int* d_tgt_oct, int n_tgt, double scale, double* target,
-                        bool assign)
+    static void inverse(Ctx& c, const void* acc, const int* d_tgt_oct, int n_tgt, double scale, double* target)
     {
         if (!n_tgt) return;
-        if constexpr (pfa_extent(NB)) inverse_pfa(c, acc, d_tgt_oct, n_tgt, scale, target, assign);
+        if constexpr (pfa_extent(NB)) inverse_pfa(c, acc, d_tgt_oct, n_tgt, scale, target);
         else
         {
-            launch_inverse(c, (const cx<R>*)acc, d_tgt_oct, n_tgt, scale, target, assign);
+            launch_inverse(c, (const cx<R>*)acc, d_tgt_oct, n_tgt, scale, target);
             c.launches += 1;
         }
     }
@@ -1071,7 +1021,7 @@ void launch_forward_sources(Ctx& c, const double* fmm_s, const int* d_src_oct, i
 }
 
 // one run of the sibling-group MAC in the given variant: 0, 1 the direct
-// kernel with two groups or one group per warp, 2 the block-Toeplitz kernel,
+// kernel with two groups or half a group per warp, 2 the block-Toeplitz kernel,
 // 3 the tensor-core kernel
 void group_mac_variant(Ctx& c, const FmmPlan& p, const void* src_spec, void* acc, int variant)
 {
@@ -1152,7 +1102,7 @@ void launch_inverse_targets(Ctx& c, const FmmPlan& p, const void* acc, double* f
 {
     dispatch(c, [&](auto cv) {
         using CV = decltype(cv);
-        CV::inverse(c, acc, p.tgt_oct.p, p.n_tgt, scale, fmm_t, true);
+        CV::inverse(c, acc, p.tgt_oct.p, p.n_tgt, scale, fmm_t);
     });
     IBLGF_CUDA(cudaGetLastError());
 }

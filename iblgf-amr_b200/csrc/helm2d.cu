@@ -149,12 +149,11 @@ __global__ void helm2d_apply_kernel(int nx, int ny, const double* __restrict__ t
 // x fastest; a scalar field has sep = 2 N_modes components (mode i: real 2i,
 // imaginary 2i+1), a vector field three groups of sep (x, y, z); the z
 // derivative of mode i is multiplication by i omega_i, omega_i = 2 pi i / lz.
-// One CTA per block, threads over (mode, interior node) pairs (nodes
-// 1 .. NB-2 per axis); buffers are read, not written. The mask selects the modes written: all of
-// them for the forms above, one for the _oneMode forms (:1548, :1620, :1801,
-// :2017, :2224), the first N_modes / 2^r for the _refined forms (:1653,
-// :1839, :2125), any set for the ModesBool forms (:1889, :1931); the
-// components of unselected modes are left as they were.
+// Interior nodes (1 .. NB-2 per axis) are written, buffers read only. The mask
+// selects the modes written: all of them for the forms above, one for the
+// _oneMode forms (:1548, :1620, :1801, :2017, :2224), the first N_modes / 2^r for
+// the _refined forms (:1653, :1839, :2125), any set for the ModesBool forms
+// (:1889, :1931); the components of unselected modes are left as they were.
 // op: 0 laplace (cell -> cell), 1 gradient (cell -> face), 2 divergence
 // (face -> cell), 3 curl (face -> edge), 4 curl_transpose (edge -> face, x scale)
 // Memory-bound: one thread owns every output component of one (mode, node)

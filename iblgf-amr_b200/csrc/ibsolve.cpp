@@ -22,7 +22,7 @@
 
 namespace iblgf_b200
 {
-void launch_axpby(Ctx& c, double* to, const double* from, double a, int mode);
+void launch_axpby_vf(Ctx& c, double* const* to, const double* const* from, int n, double a, int mode);
 
 namespace
 {
@@ -754,7 +754,8 @@ void ns_ib_stage(Ctx& c, int stage, double alpha, double threshold, int max_iter
     launch_zero_blocks(c, pc[0], s.corr_list.p, s.n_corr);
     if (s.clean_base) launch_face_planes(c, pc[0], s.cb_list.p, s.cb_faces.p, s.n_cb, 2);
     poisson_apply_lgf(c, s.cell_aux2, s.cell_aux2, IBLGF_IB2AMR, false);  // clean since the force solve
-    launch_axpby(c, c.field(d_field), c.field(s.cell_aux2), -1.0, 1);
+    double* pd[1] = {c.field(d_field)};
+    launch_axpby_vf(c, pd, pc, 1, -1.0, 1);
     gradient_d();
     smearing(c, s, s.cg_f.p, face_aux, false);
 }

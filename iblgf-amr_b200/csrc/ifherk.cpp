@@ -23,8 +23,6 @@
 
 namespace iblgf_b200
 {
-void launch_clean(Ctx& c, double* f, const int* d_leaf, bool non_leaf_only, int width = 1);
-void launch_axpby(Ctx& c, double* to, const double* from, double a, int mode);
 void launch_clean_vf(Ctx& c, double* const* f, int n, const int* d_leaf, bool non_leaf_only, int width = 1);
 void launch_axpby_vf(Ctx& c, double* const* to, const double* const* from, int n, double a, int mode);
 void launch_lincomb_vf(Ctx& c, double* const* to, const double* const* x, const double* const* y, int n, double a,
@@ -665,7 +663,8 @@ void ns_clean(Ctx& c, int field, bool non_leaf_only, int width)
     if (field < 0 || field >= (int)c.fields.size() || width < 1 || width > c.Nb / 2)
         throw Error(IBLGF_EINVAL, "bad clean arguments");
     NsState& s = ns_state(c);
-    launch_clean(c, c.field(field), s.leaf.p, non_leaf_only, width);
+    double* f = c.field(field);
+    launch_clean_vf(c, &f, 1, s.leaf.p, non_leaf_only, width);
 }
 
 void ns_clean_leaf_correction_boundary(Ctx& c, const int* fields, int n, int level, bool leaf_only_boundary)

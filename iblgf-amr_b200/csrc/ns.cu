@@ -1,8 +1,8 @@
 // Field kernels of the IF-HERK time step (FP64, whole component fields):
-//   clean_kernel     Ifherk::clean (ifherk.hpp:1309-1352): zero whole blocks,
+//   clean3_kernel    Ifherk::clean (ifherk.hpp:1309-1352): zero whole blocks,
 //                    or with non_leaf_only only the outer `width` planes of
 //                    leaves and all of every other block
-//   axpby_kernel     Ifherk::copy / add (ifherk.hpp:1878-1960), over every
+//   axpby3_kernel    Ifherk::copy / add (ifherk.hpp:1878-1960), over every
 //                    node including buffers
 //   lincomb_kernel   the sums of two fields that the stages form by a copy and
 //                    an add, in one pass (3 field passes instead of 5)
@@ -20,24 +20,6 @@ namespace iblgf_b200
 {
 namespace
 {
-template<int NB>
-__global__ void clean_kernel(double* __restrict__ f, const int* __restrict__ leaf, int non_leaf_only, int w)
-{
-    constexpr int N3 = NB * NB * NB;
-    const int o = blockIdx.x;
-    double* b = f + (size_t)o * N3;
-    const bool shell = non_leaf_only && leaf[o];
-    for (int i = threadIdx.x; i < N3; i += blockDim.x)
-    {
-        if (shell)
-        {
-            const int x = i % NB, y = (i / NB) % NB, z = i / (NB * NB);
-            if (x >= w && y >= w && z >= w && x < NB - w && y < NB - w && z < NB - w) continue;
-        }
-        b[i] = 0.0;
-    }
-}
-
 // up to three component fields per launch (blockIdx.y = component)
 struct Fields3
 {
@@ -99,18 +81,6 @@ __global__ void lincomb_kernel(const __grid_constant__ LinComb3 f, double a, siz
         const double2 u = x[i], v = y[i];
         if (mode == 0) to[i] = make_double2(u.x + v.x * a, u.y + v.y * a);
         else to[i] = make_double2((u.x - v.x) * a, (u.y - v.y) * a);
-    }
-}
-
-// mode 0: to = a * from; 1: to += a * from; 2: to *= a; 3: to += a
-__global__ void axpby_kernel(double* __restrict__ to, const double* __restrict__ from, double a, size_t n, int mode)
-{
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    {
-        if (mode == 0) to[i] = from[i] * a;
-        else if (mode == 1) to[i] += from[i] * a;
-        else if (mode == 2) to[i] *= a;
-        else to[i] += a;
     }
 }
 
@@ -194,18 +164,6 @@ void nb_switch(int Nb, F&& f)
 }
 }  // namespace
 
-void launch_clean(Ctx& c, double* f, const int* d_leaf, bool non_leaf_only, int width)
-{
-    if (!c.n_oct) return;
-    nb_switch(c.Nb, [&](auto nbc) {
-        constexpr int NB = decltype(nbc)::value;
-        clean_kernel<NB><<<c.n_oct, 256, 0, c.stream>>>(f, d_leaf, non_leaf_only ? 1 : 0, width);
-    });
-    c.launches += 1;
-    IBLGF_CUDA(cudaGetLastError());
-}
-
-// the component fields of one vector field in one launch
 void launch_clean_vf(Ctx& c, double* const* f, int n, const int* d_leaf, bool non_leaf_only, int width)
 {
     if (!c.n_oct || n < 1 || n > 3) return;
@@ -249,16 +207,6 @@ void launch_lincomb_vf(Ctx& c, double* const* to, const double* const* x, const 
     }
     const unsigned grid = (unsigned)std::min<size_t>((pairs + 255) / 256, 148 * 16 / n);
     lincomb_kernel<<<dim3(grid, n), 256, 0, c.stream>>>(p, a, pairs, mode);
-    c.launches += 1;
-    IBLGF_CUDA(cudaGetLastError());
-}
-
-void launch_axpby(Ctx& c, double* to, const double* from, double a, int mode)
-{
-    const size_t n = c.field_elems();
-    if (!n) return;
-    const unsigned grid = (unsigned)std::min<size_t>((n + 255) / 256, 148 * 16);
-    axpby_kernel<<<grid, 256, 0, c.stream>>>(to, from, a, n, mode);
     c.launches += 1;
     IBLGF_CUDA(cudaGetLastError());
 }

@@ -158,17 +158,11 @@ void ctx_init(Ctx& c)
             for (int j = 1; j < c.Nb - 1; ++j)
                 if (j + h * (c.Nb - 2) == 2 * p - 1) inject[(size_t)h * c.Nb * c.Nb + p * c.Nb + j] = 1.0;
     mats.insert(mats.end(), inject.begin(), inject.end());
-    c.d_mats.upload(mats, c.stream);
     c.h_mats = mats;
     c.tree.init(e, c.cfg.bd_base, c.cfg.bd_extent);
     launch_lgf_table(c);
 }
 
-// The FP32 path runs the prime-factor z and y inverse passes in FP32 (the
-// c2r stage, the sum over the two kx halves and the add into the target stay
-// FP64). Measured on the 3-level Gaussian workload: 4.8e-6 relative L-inf
-// against the FP64 oracle (FP64 passes: 1.4e-7; the direct 35-term FP32 sums
-// gave 1.16e-5), inverse phase 1.89 ms instead of 2.53 ms per solve.
 // Server::compute_distribution (decomposition/server.hpp:245-330) for this
 // process's octree: loads as FmmMaskBuilder::fmm_dry accumulates them
 // (fmm.hpp:597-626: neighbour + influence count per AMR2AMR sweep in which
@@ -853,10 +847,8 @@ HostPlan build_host_plan(const Ctx& c, int level, int idx, int ge, bool direct_o
                                   uz * e - (Nb - 1)});
         }
     }
-    // tiles: consecutive groups of one level distance while the union of their
-    // sources fits the staging budget
-    // a tile: up to 32 sibling groups (16 rows x 2 per row of the MAC CTA) whose
-    // union of candidate sources fits the 64-byte-row staging budget
+    // tiles: up to kGroupTileCap consecutive groups of one level distance whose
+    // union of candidate sources stays within 1024 rows
     const int kScap = 1024, kGcap = kGroupTileCap;
     std::vector<int>& tgptr = p.tgptr;
     std::vector<int>& tsptr = p.tsptr;
@@ -867,14 +859,13 @@ HostPlan build_host_plan(const Ctx& c, int level, int idx, int ge, bool direct_o
     std::vector<unsigned short>& gsrc = p.gsrc;
     std::vector<unsigned>& gpm = p.gpm;
     std::vector<int> local;  // row in the tile by source, -1: none
-    int cur_ld = -1, ngrp = 0, n_local = 0, max_src = 0;
+    int cur_ld = -1, ngrp = 0, n_local = 0;
     auto close_tile = [&]() {
         if (!ngrp) return;
         tgptr.push_back((int)gtgt.size() / 8);
         tsptr.push_back((int)tsrc.size());
         ttab.push_back(tab_of_ld[cur_ld]);
         tcoarse.push_back(neighbor_only ? 2 : (cur_ld > 0 ? 1 : 0));
-        max_src = std::max(max_src, n_local);
         for (size_t k = tsrc.size() - n_local; k < tsrc.size(); ++k) local[tsrc[k]] = -1;
         n_local = 0;
         ngrp = 0;
@@ -911,8 +902,8 @@ HostPlan build_host_plan(const Ctx& c, int level, int idx, int ge, bool direct_o
         for (int kk = 0; kk < 216; ++kk)
             if (gr.used[kk]) pm |= 1u << (kk / 8);
         gpm.push_back(pm);
-        // the kernel runs all 64 (c, c') products of a present parent, or
-        // only the adjacent ones when the plan is neighbour-only
+        // coverage counter: all 64 (c, c') products of a present parent, or only
+        // the adjacent ones when the plan is neighbour-only
         for (int n = 0; n < 27; ++n)
             if (pm >> n & 1u)
             {
@@ -925,7 +916,6 @@ HostPlan build_host_plan(const Ctx& c, int level, int idx, int ge, bool direct_o
     }
     close_tile();
     p.n_groups = (int)groups.size();
-    p.max_tile_src = max_src;
     for (auto& x : tp) p.all_keys.insert(p.all_keys.end(), x.key.begin(), x.key.end());
     for (auto& x : tp) p.n_pairs += (long long)x.src.size();
     p.n_exec += (long long)p.psrc.size();  // pair-list targets
@@ -947,8 +937,9 @@ namespace
 // more CTAs end with idle warps). Below that (short spectra: 23 chunks of 32
 // frequencies at extent 4, 58 at 6, 199 at 10) the size whose waves end first is
 // taken, a CTA counted as its bundles (at least `few`: fewer leave its warps'
-// latencies open), as many for the end, where warps run out of bundles, and
-// kMacStage. Whole solves on
+// latencies open; FP32's 10 was fitted at 20 warps per CTA, but 8, half of its 16,
+// takes a batch of 22 problems at extent 14 from 162 to 173 us), as many for the
+// end, where warps run out of bundles, and kMacStage. Whole solves on
 // three levels, FP64, tiles of 96 -> fitted: extent 4 1141 -> 623 us, extent 6
 // 1218 -> 1009 and 1332 -> 1243 us; batch of 29 problems, extent 10 200 -> 184 us.
 int mac_tile_size(const Ctx& c, const std::vector<int>& bundles)
@@ -1137,35 +1128,28 @@ std::unique_ptr<FmmPlan> upload_plan(Ctx& c, const HostPlan& h)
         p.ge_src.upload(h.ge_src, c.stream);
     }
     p.n_tiles = (int)h.ttab.size();
-    p.max_tile_src = h.max_tile_src;
-    p.tile_gptr.upload(h.tgptr, c.stream);
+    // per group its 216 candidates' source rows: candidate kk of group g of tile
+    // t reads row tsrc[tsptr[t] + gsrc[g][kk]], an absent one the zero row n_src
+    std::vector<int> gjr((size_t)h.n_groups * 216, p.n_src);
+    for (int t = 0; t < p.n_tiles; ++t)
+        for (size_t i = (size_t)h.tgptr[t] * 216; i < (size_t)h.tgptr[t + 1] * 216; ++i)
+            if (h.gsrc[i] != 0xFFFF) gjr[i] = h.tsrc[h.tsptr[t] + h.gsrc[i]];
+    p.mac_flops = (long long)h.psrc.size() * 8;  // per frequency: 8 per complex multiply-add
+    build_mac_bundles(c, p, h, gjr);
+    if (p.n_tiles && c.cfg.precision == IBLGF_FP32)
     {
-        // candidate source rows per tile: group g's candidate kk reads row
-        // tsrc[tsptr[t] + gsrc[g][kk]], absent ones (and unused group slots)
-        // the zero row n_src
-        // padded so that the block-Toeplitz MAC's copy of a tile's last part
-        // (3 parts of kToeplitzPart rows) stays inside the buffer
+        // the block-Toeplitz and tensor-core MACs (FP32 only)
+        p.tile_gptr.upload(h.tgptr, c.stream);
+        p.grp_pm.upload(h.gpm, c.stream);
+        p.grp_jr.upload(gjr, c.stream);
+        // the rows per tile, padded so that the block-Toeplitz MAC's copy of a
+        // tile's last part (3 parts of kToeplitzPart rows) stays inside the buffer
         const size_t pad = (size_t)(3 * kToeplitzPart - kGroupTileCap) * 216;
         std::vector<int> jr((size_t)p.n_tiles * kGroupTileCap * 216 + pad, p.n_src);
         for (int t = 0; t < p.n_tiles; ++t)
-            for (int g = h.tgptr[t]; g < h.tgptr[t + 1]; ++g)
-                for (int kk = 0; kk < 216; ++kk)
-                {
-                    const unsigned short j = h.gsrc[(size_t)g * 216 + kk];
-                    if (j != 0xFFFF)
-                        jr[((size_t)t * kGroupTileCap + (g - h.tgptr[t])) * 216 + kk] = h.tsrc[h.tsptr[t] + j];
-                }
+            std::copy(gjr.begin() + (size_t)h.tgptr[t] * 216, gjr.begin() + (size_t)h.tgptr[t + 1] * 216,
+                      jr.begin() + (size_t)t * kGroupTileCap * 216);
         p.tile_jr.upload(jr, c.stream);
-        // the same rows per group for the tensor-core MAC, whose tiles span
-        // up to 128 consecutive groups
-        std::vector<int> gjr((size_t)std::max(h.n_groups, 1) * 216, p.n_src);
-        for (int t = 0; t < p.n_tiles; ++t)
-            for (int g = h.tgptr[t]; g < h.tgptr[t + 1]; ++g)
-                std::copy_n(jr.begin() + ((size_t)t * kGroupTileCap + (g - h.tgptr[t])) * 216, 216,
-                            gjr.begin() + (size_t)g * 216);
-        if (p.n_tiles) p.grp_jr.upload(gjr, c.stream);
-        p.mac_flops = (long long)h.psrc.size() * 8;  // per frequency: 8 per complex multiply-add
-        build_mac_bundles(c, p, h, gjr);
         std::vector<int> tg, tt, tm;
         std::vector<unsigned> tp;
         build_tc_tiles(h.tgptr, h.ttab, h.tcoarse, h.gpm, tg, tt, tm, tp);
@@ -1178,10 +1162,7 @@ std::unique_ptr<FmmPlan> upload_plan(Ctx& c, const HostPlan& h)
             p.tc_pm.upload(tp, c.stream);
         }
     }
-    p.tile_tab.upload(h.ttab, c.stream);
-    p.tile_coarse.upload(h.tcoarse, c.stream);
     p.spec_u.upload(spec_u, c.stream);
-    p.grp_pm.upload(h.gpm, c.stream);
     p.grp_tgt.upload(h.gtgt, c.stream);
     p.n_exec = h.n_exec;
     p.adj_only = !h.tcoarse.empty();
@@ -1476,14 +1457,6 @@ PoissonLists& poisson_lists(Ctx& c)
 {
     if (auto* have = c.ext_get<PoissonLists>(Ctx::kExtPLists)) return *have;
     auto pl = std::make_unique<PoissonLists>();
-    std::vector<int> all, leaves;
-    for (int i = 0; i < c.n_oct; ++i)
-    {
-        all.push_back(i);
-        if (c.flags[i] & 1) leaves.push_back(i);
-    }
-    pl->all.upload(all, c.stream);
-    pl->leaves.upload(leaves, c.stream);
     const int L = kMaxLevel + 1;
     pl->level_all.resize(L);
     pl->level_leaves.resize(L);

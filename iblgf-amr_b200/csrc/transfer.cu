@@ -238,7 +238,10 @@ __global__ void __launch_bounds__(tp_threads<NB>(), 2) tp_kernel(
 // children in sequence are 24 barrier-separated passes on a few SMs: 22 against
 // 45 us at 44 blocks of 18^3 in FP32, 16 against 28 at 8; with more blocks than
 // kAntrpClusters the chip is full either way and the barriers of the cluster
-// cost more (106 blocks: 44 / 46 us, 184: 73 / 67, 1161: 382 / 202).
+// cost more (106 blocks: 44 / 46 us, 184: 73 / 67, 1161: 382 / 202; in FP64, 98 KB
+// per CTA, 64 blocks 31 / 67, 216: 96 / 86). The line is that of 18^3 blocks; the
+// clusters of smaller ones still win at 216 (extent 10, FP64 20 / 30 us, extent 4
+// 8.5 / 11 us).
 constexpr int kAntrpClusters = 120;
 
 template<int NB, class T>

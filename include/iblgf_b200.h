@@ -384,11 +384,11 @@ int iblgf_profile_read(iblgf_ctx* ctx, double* out4);
 int iblgf_stats(iblgf_ctx* ctx, long long* out8);
 
 /* The first n (1 <= n <= 10) counters: [0]-[7] as iblgf_stats, then [8] the
- * (target, source) spectral products the sibling-group MAC covers: a group
- * covers all 64 (child, candidate) products of every neighbour parent that
- * has a candidate, so [8] >= [3]; and [9] the floating-point operations the
- * direct MAC kernels execute per spectrum frequency (they skip absent
- * candidates and targets where that pays).
+ * (target, source) spectral products of a sibling-group MAC that forms all 64
+ * (child, candidate) products of every neighbour parent with a candidate, so
+ * [8] >= [3]; and [9] the floating-point operations per spectrum frequency that
+ * the direct MAC kernels execute (they skip absent candidates and targets where
+ * that pays, so they execute fewer products than [8]).
  * IBLGF_EINVAL for n outside [1, 10]. */
 int iblgf_stats_n(iblgf_ctx* ctx, long long* out, int n);
 
