@@ -1,8 +1,8 @@
 """Block kernels over the block extents and the edges of their work splits,
 against the oracle: sweeps with partly present sibling groups, the integrating
 factor's truncation radii, the single-block convolution, the Fourier-in-z
-operators at extents without a compile-time form, and few immersed-boundary
-points."""
+operators at extents without a compile-time form, interpolation orders, both
+forms of the anterpolation, and few immersed-boundary points."""
 import os
 import sys
 
@@ -127,6 +127,70 @@ def test_fourier_operators_extents(op, nb, nm):
     g.helm2d_op(op, s, d, nm, 0.25, 1.5, 0.6)
     g.synchronize()
     assert np.abs(d.cpu().numpy() - ref).max() < 1e-13 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("nb,npl", [(3, 1), (7, 5), (18, 7), (40, 3)])
+def test_fourier_nonlinear_extents(nb, npl):
+    """As test_fourier_operators_extents, the collocation-plane convective term; its bar in test_gpu_helm2d.py."""
+    import torch
+    g = B.Solver((-12,) * 3, (24,) * 3, 6, 1.0, [((-6,) * 3, (12,) * 3)])
+    face, edge, dst = np.random.default_rng(nb).standard_normal((3, 2, 3 * npl, nb, nb))
+    ref = H.nonlinear(face, edge, dst.copy(), npl, None)
+    d = torch.tensor(dst, device="cuda")
+    f, e = torch.tensor(face, device="cuda"), torch.tensor(edge, device="cuda")
+    torch.cuda.synchronize()
+    g.helm2d_nonlinear(f, e, d, npl)
+    g.synchronize()
+    assert np.abs(d.cpu().numpy() - ref).max() < 1e-14 * np.abs(ref).max()
+
+
+# band widths of the cell-centred transfers: 2 (orders 1, 2), the window of 5 (3 to 5), dense (above)
+@pytest.mark.parametrize("order", [1, 2, 3, 4, 6, 7, 11])
+@pytest.mark.parametrize("e", [4, 16])
+def test_interpolation_orders(e, order):
+    """apply_lgf across a level change; the FP64 parity bar."""
+    args = ((-4 * e,) * 3, (8 * e,) * 3, e, 0.5, [((-2 * e, -e, 0), (3 * e, 2 * e, e))])
+    kw = dict(n_levels=1, predicate=lambda base, ext, rl, diff: rl == 0 and tuple(base) == (0, 0, 0), intrp_order=order)
+    o, g = O.Domain(*args, **kw), B.Solver(*args, **kw)
+    src = np.random.default_rng(e).standard_normal((o.n, o.Nb, o.Nb, o.Nb))
+    fs, ft = g.field(src), g.field()
+    g.apply_lgf(fs, ft)
+    assert rel_linf(g.download(ft), o.apply_lgf(src)) < 1e-12
+
+
+@pytest.mark.parametrize("order", [2, 4, 7])
+def test_interpolation_orders_time_step(order):
+    """Face and edge fields take two matrix sets per transfer; the bar of the plain time steps (FP64)."""
+    case = S.VortexRingNS("small")
+    args = (case.bd_base, case.bd_extent, case.block_extent, case.dx_base, case.blocks)
+    kw = dict(n_levels=case.n_levels, predicate=case.predicate, intrp_order=order)
+    o, g = O.Domain(*args, **kw), B.Solver(*args, **kw)
+    u0 = case.initial_velocity(o)
+    ur, pr = o.ns_step(u0, case.dt(), case.Re, 0.0, 1)
+    uf, pf = [g.field(u0[k]) for k in range(3)], g.field()
+    g.ns_step(uf, pf, case.dt(), case.Re, 0.0, 1)
+    for f, ref in zip(uf + [pf], list(ur) + [pr]):
+        assert rel_linf(g.download(f), ref) < 1e-10
+
+
+@pytest.mark.parametrize("precision,tol", [(B.FP64, 1e-12), (B.FP32, 1e-5)])
+@pytest.mark.parametrize("e", [4, 6, 10, 16])
+def test_anterpolation_by_clusters_and_by_blocks(e, precision, tol):
+    """A problem of 4^3 blocks has 8 or 27 receiving blocks per coarse level, eight CTAs for each; sixteen of them in a
+    batch have more than 120, one CTA for each."""
+    prob = dict(bd_base=(-4 * e,) * 3, bd_extent=(8 * e,) * 3, blocks=[((-2 * e,) * 3, (4 * e,) * 3)])
+    one = B.Solver(prob["bd_base"], prob["bd_extent"], e, 0.5, prob["blocks"], precision=precision)
+    many = B.BatchSolver(e, 0.5, [prob] * 16, precision=precision)
+    one.mac_variant(0)
+    many.mac_variant(0)
+    src = np.random.default_rng(e).standard_normal((many.n, e + 2, e + 2, e + 2))
+    fs, ft = many.field(src), many.field()
+    many.apply_lgf(fs, ft)
+    out, a, b = many.split(many.download(ft)), one.field(), one.field()
+    for i in (0, 15):
+        one.upload(a, many.split(src)[i])
+        one.apply_lgf(a, b)
+        assert rel_linf(out[i], one.download(b)) < tol
 
 
 @pytest.mark.parametrize("n", [1, 7, 8, 33])
