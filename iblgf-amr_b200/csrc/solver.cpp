@@ -1097,6 +1097,16 @@ std::unique_ptr<FmmPlan> upload_plan(Ctx& c, const HostPlan& h)
     // LGF spectrum slots: every pair's key gets a slot (new ones are computed
     // below); the group tables reference registered keys only (-1: zero row)
     std::vector<std::array<int, 5>> new_slots;
+    // a failure before the new slots' spectra are there takes the slots back
+    struct SlotGuard
+    {
+        Ctx& c;
+        std::vector<std::array<int, 5>>& slots;
+        ~SlotGuard()
+        {
+            for (auto& s : slots) c.spec_slot.erase({s[1], s[2], s[3], s[4]});
+        }
+    } guard{c, new_slots};
     auto slot_of = [&](const std::array<int, 4>& k) {
         auto it = c.spec_slot.find(k);
         if (it != c.spec_slot.end()) return it->second;
@@ -1193,6 +1203,7 @@ std::unique_ptr<FmmPlan> upload_plan(Ctx& c, const HostPlan& h)
         }
         launch_spectra(c, new_slots);
         c.spec_used = need;
+        new_slots.clear();
     }
     if (toeplitz && !p.adj_only)
     {

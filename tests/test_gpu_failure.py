@@ -89,6 +89,31 @@ def test_allocation_failure_is_reported(after):
     g.close()
 
 
+@pytest.mark.parametrize("precision,variant,tol", [(B.FP64, -1, 1e-12)])
+def test_context_solves_after_failed_allocations(precision, variant, tol):
+    """One context whose first solve fails at its first allocation, the next at its second, and so on until a solve
+    finds all it needs: what the failed ones had begun (plans, spectra, kernel tables, buffers) is built anew."""
+    case = S.GaussianPoisson("amr_small")
+    g, o = make(case, precision), oracle(case)
+    g.mac_variant(variant)
+    src = case.fields(g)
+    fs, ft = g.field(src), g.field()
+    failed, solved = 0, False
+    while not solved and failed < 2000:
+        B.debug_fail_alloc(failed)
+        try:
+            g.apply_lgf(fs, ft)
+            solved = True
+        except B.IblgfError as e:
+            assert e.code == B.ENOMEM
+            failed += 1
+        finally:
+            B.debug_fail_alloc(-1)
+    assert solved and failed > 20
+    assert rel_linf(g.download(ft), o.apply_lgf(src)) < tol
+    g.close()
+
+
 def test_nonfinite_host_input_is_found():
     case = S.GaussianPoisson("amr_small")
     g = make(case)
