@@ -434,6 +434,11 @@ int combo_table(Ctx& c, int ld, const std::vector<int>& slots)
     if (it != c.combo_of_ld.end()) return it->second;
     const size_t tbytes = (size_t)729 * c.NC * c.cplx_bytes();
     const int idx = c.combo_tables;
+    if (c.cfg.precision != IBLGF_FP32) throw Error(IBLGF_EINTERNAL, "block-Toeplitz tables are FP32-path only");
+    // allocated first: once the tables have moved, nothing may fail before the
+    // tensor map follows them
+    DevBuf<int> d_slots;
+    d_slots.upload(slots, c.stream);
     if (idx + 1 > c.combo_cap)
     {
         const int cap = std::max(idx + 1, 2 * c.combo_cap);
@@ -445,11 +450,8 @@ int combo_table(Ctx& c, int ld, const std::vector<int>& slots)
         ++c.step_epoch;
         c.combo_cap = cap;
     }
-    DevBuf<int> d_slots;
-    d_slots.upload(slots, c.stream);
     dim3 grid((unsigned)((c.NC + 255) / 256), 729);
     char* out = c.d_combo.p + (size_t)idx * tbytes;
-    if (c.cfg.precision != IBLGF_FP32) throw Error(IBLGF_EINTERNAL, "block-Toeplitz tables are FP32-path only");
     combo_table_kernel<float><<<grid, 256, 0, c.stream>>>((const float2*)c.d_spec.p, d_slots.p, ld > 0 ? 1 : 0,
                                                           c.NC, (float2*)out);
     IBLGF_CUDA(cudaGetLastError());

@@ -89,7 +89,7 @@ def test_allocation_failure_is_reported(after):
     g.close()
 
 
-@pytest.mark.parametrize("precision,variant,tol", [(B.FP64, -1, 1e-12)])
+@pytest.mark.parametrize("precision,variant,tol", [(B.FP64, -1, 1e-12), (B.FP32, 2, 1e-5)])
 def test_context_solves_after_failed_allocations(precision, variant, tol):
     """One context whose first solve fails at its first allocation, the next at its second, and so on until a solve
     finds all it needs: what the failed ones had begun (plans, spectra, kernel tables, buffers) is built anew."""
